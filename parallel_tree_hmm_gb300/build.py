@@ -32,6 +32,8 @@ COMMON = [
 ]
 SOURCES = [
     # Slowest first: the build compiles them in parallel.
+    "engine_maximum_f64.cu",
+    "engine_maximum_f32.cu",
     "engine_linear_fd_rev_large.cu",
     "engine_linear_dd_rev_large.cu",
     "engine_linear_ff_rev_large.cu",
@@ -48,8 +50,6 @@ SOURCES = [
     "engine_linear_dd_fwd_small.cu",
     "engine_linear_ff_fwd_small.cu",
     "engine_linear_df_fwd_small.cu",
-    "engine_maximum_f64.cu",
-    "engine_maximum_f32.cu",
     "engine_sample_f64.cu",
     "engine_sample_f32.cu",
     "engine_wide.cu",
@@ -64,6 +64,10 @@ SOURCES = [
     "engine_phase_groups_16_f32.cu",
     "engine_phase_groups_8_f64.cu",
     "engine_phase_groups_8_f32.cu",
+    "engine_phase_sample_f64.cu",
+    "engine_phase_sample_f32.cu",
+    "engine_phase_max_f64.cu",
+    "engine_phase_max_f32.cu",
     "engine_linear_f32.cu",
     "engine_linear_f64.cu",
     "engine_maximum.cu",

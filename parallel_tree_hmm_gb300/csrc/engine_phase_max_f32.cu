@@ -1,0 +1,10 @@
+// MAP phase kernels (phase_log.cuh), float arithmetic.
+#include "phase_log.cuh"
+
+namespace thmm {
+
+cudaError_t LaunchPhaseMaximumF32(int kind, const PhaseArgs &args, cudaStream_t stream) {
+  return LaunchLog<float, false>(kind, args, stream);
+}
+
+} // namespace thmm

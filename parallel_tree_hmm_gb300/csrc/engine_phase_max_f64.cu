@@ -1,0 +1,10 @@
+// MAP phase kernels (phase_log.cuh), double arithmetic.
+#include "phase_log.cuh"
+
+namespace thmm {
+
+cudaError_t LaunchPhaseMaximumF64(int kind, const PhaseArgs &args, cudaStream_t stream) {
+  return LaunchLog<double, false>(kind, args, stream);
+}
+
+} // namespace thmm

@@ -1,0 +1,10 @@
+// Posterior sampling phase kernels (phase_log.cuh), float arithmetic.
+#include "phase_log.cuh"
+
+namespace thmm {
+
+cudaError_t LaunchPhaseSampleF32(int kind, const PhaseArgs &args, cudaStream_t stream) {
+  return LaunchLog<float, true>(kind, args, stream);
+}
+
+} // namespace thmm

@@ -1,0 +1,10 @@
+// Posterior sampling phase kernels (phase_log.cuh), double arithmetic.
+#include "phase_log.cuh"
+
+namespace thmm {
+
+cudaError_t LaunchPhaseSampleF64(int kind, const PhaseArgs &args, cudaStream_t stream) {
+  return LaunchLog<double, true>(kind, args, stream);
+}
+
+} // namespace thmm

@@ -72,7 +72,7 @@ PhasePlan::OpRange(int kind, std::uint32_t round, std::uint32_t a, std::uint32_t
   return {first, last};
 }
 
-PhasePlan::Tail PhasePlan::BuildTail(std::uint32_t tail_round) const {
+PhasePlan::Tail PhasePlan::BuildTail(std::uint32_t tail_round, bool every) const {
   Tail tail;
   const std::size_t n = instance_program.size();
   std::vector<std::uint64_t> gather_at(rounds, 0), rake_at(rounds, 0),
@@ -84,10 +84,10 @@ PhasePlan::Tail PhasePlan::BuildTail(std::uint32_t tail_round) const {
   }
   for (std::size_t i = 0; i < n; ++i) {
     const ProgramRounds &c = program_rounds[instance_program[i]];
-    if (c.rounds > tail_round) {
+    if (c.rounds > tail_round || every) {
       tail.items.push_back({static_cast<std::uint32_t>(i),
                             static_cast<std::uint32_t>(tail.rounds.size()),
-                            c.rounds - tail_round, 0u});
+                            c.rounds > tail_round ? c.rounds - tail_round : 0u, 0u});
       for (std::uint32_t r = tail_round; r < c.rounds; ++r) {
         tail.rounds.push_back({static_cast<std::uint32_t>(gather_at[r]), c.gathers[r],
                                static_cast<std::uint32_t>(compress_at[r]),
@@ -124,9 +124,10 @@ PhasePlan BuildPhasePlan(const ProgramSet &set, std::span<const PhaseInstance> i
   constexpr std::uint64_t kTreeLimit = (1ull << 31) / (2 * 3400);
   if (n == 0 || total_nodes >= kIndexLimit || total_edges_out >= kIndexLimit)
     return plan;
+  plan.exponents_fit = true;
   for (const DevProgram &program : set.programs)
     if (program.num_nodes > kTreeLimit)
-      return plan;
+      plan.exponents_fit = false;
 
   std::vector<ProgramLayout> layouts;
   layouts.reserve(set.programs.size());
@@ -172,6 +173,7 @@ PhasePlan BuildPhasePlan(const ProgramSet &set, std::span<const PhaseInstance> i
   plan.rakes.resize(plan.rake_base[rounds]);
   plan.gathers.resize(plan.gather_base[rounds]);
   plan.compress.resize(plan.compress_base[rounds]);
+  plan.ends.resize(plan.compress_base[rounds]);
   plan.roots.resize(n);
 
   const auto fill = [&](std::size_t first, std::size_t last) {
@@ -218,6 +220,9 @@ PhasePlan BuildPhasePlan(const ProgramSet &set, std::span<const PhaseInstance> i
         for (std::uint32_t c = 0; c < l.counts.compressions[r]; ++c) {
           const Uint4 &src = set.compress[l.compress_at[r] + c];
           plan.compress[comp0 + c] = {path(src.x), node(src.y), path(src.z), obs(src.w)};
+          const Uint2 &end = set.compress_ends[l.compress_at[r] + c];
+          plan.ends[comp0 + c] = {static_cast<std::uint32_t>(inst.node_base + end.x),
+                                  static_cast<std::uint32_t>(inst.node_base + end.y)};
         }
       }
       plan.roots[i] = {static_cast<std::uint32_t>(inst.node_base + root) |

@@ -101,7 +101,7 @@ struct PhaseArgs {
   const uint4 *tail_items;
   const uint4 *tail_rounds;
   const uint2 *tail_rakes;
-  // Shared-topology layout only (BatchPhaseKernel): items [first_item,
+  // Shared-topology layout only (batch set): items [first_item,
   // first_item + items) of a batch whose stored objects are `item_stride`
   // items apart, each with item_nodes nodes and item_edges edges.
   std::uint32_t batch;
@@ -110,8 +110,16 @@ struct PhaseArgs {
   std::uint64_t item_stride;
   std::uint64_t item_nodes;
   std::uint64_t item_edges;
-  // Wide-state kinds (32 < K <= 128) only: the error word (tensor-core wait
-  // time-outs) and the BF16 product tier.
+  // MAP and sampling kinds (phase_log.cuh) only; their values are in the
+  // input precision, their layout always the batch one (a forest: one item).
+  const uint2 *ends;         // [compression] parent and child node
+  void *branches;            // [rake][K] partial sums of wide gathers
+  std::uint8_t *rake_choices; // [rake][K]
+  std::uint8_t *comp_choices; // [compression][K][K]
+  std::uint32_t *states_out;  // [node]
+  const void *uniforms;       // [node]
+  // The error word (tensor-core wait time-outs, sampling errors), and the
+  // BF16 product tier of the wide-state kinds (32 < K <= 128).
   std::uint32_t *error;
   std::uint32_t bf16;
 };
@@ -131,6 +139,9 @@ struct PhasePlan {
   std::uint32_t rounds = 0;
   std::vector<Uint4> rakes, gathers, compress;
   std::vector<Uint2> roots;
+  std::vector<Uint2> ends; // [compression] parent and child node
+  // Whether every tree's exponent sum stays in int32 (the sum-product kinds).
+  bool exponents_fit = false;
   // First operation of each round in the global arrays ([rounds + 1]).
   std::vector<std::uint64_t> rake_base, gather_base, compress_base;
   // Per-program round counts and each instance's program, to locate the
@@ -152,7 +163,8 @@ struct PhasePlan {
     std::vector<Uint4> items, rounds;
     std::vector<Uint2> rakes;
   };
-  Tail BuildTail(std::uint32_t tail_round) const;
+  // With `every`, trees of fewer rounds get an item of zero rounds.
+  Tail BuildTail(std::uint32_t tail_round, bool every = false) const;
   // Default tail round: the first round with fewer than `ops` gathers and
   // compressions over all instances.
   std::uint32_t AutoTailRound(std::uint64_t ops) const;
@@ -164,8 +176,9 @@ struct PhaseInstance {
 };
 
 // Builds the phase schedule of `instances` over the compiled `set`. Returns
-// a disabled plan when an index would not fit the 31-bit record fields or a
-// tree is large enough for its exponent sum to leave int32 range.
+// a disabled plan when an index would not fit the 31-bit record fields;
+// `exponents_fit` is false when a tree is large enough for its exponent sum
+// to leave int32 range.
 struct ProgramSet;
 PhasePlan BuildPhasePlan(const ProgramSet &set, std::span<const PhaseInstance> instances,
                          std::uint64_t total_nodes, std::uint64_t total_edges_out,
@@ -196,6 +209,15 @@ THMM_GROUP_PHASE_LAUNCHER(LaunchGroupPhase20F32)
 THMM_GROUP_PHASE_LAUNCHER(LaunchGroupPhase24F32)
 THMM_GROUP_PHASE_LAUNCHER(LaunchGroupPhase28F32)
 #undef THMM_GROUP_PHASE_LAUNCHER
+
+// MAP and sampling (K <= 32, phase_log.cuh): the forward kinds, kPhaseFinish
+// (roots), the top-down kinds (kPhaseRakeReverse, kPhaseCompressReverse) and
+// kPhaseTailForward, which runs the last rounds, the root and the top-down
+// steps of those rounds in one CTA per tree (tail items of every tree).
+cudaError_t LaunchPhaseMaximumF32(int kind, const PhaseArgs &args, cudaStream_t stream);
+cudaError_t LaunchPhaseMaximumF64(int kind, const PhaseArgs &args, cudaStream_t stream);
+cudaError_t LaunchPhaseSampleF32(int kind, const PhaseArgs &args, cudaStream_t stream);
+cudaError_t LaunchPhaseSampleF64(int kind, const PhaseArgs &args, cudaStream_t stream);
 
 // The phase-ordered copy of the observations: ordered[j * items + b] =
 // observations[b * per_item + order[j]] for j < count, b < items (a forest:

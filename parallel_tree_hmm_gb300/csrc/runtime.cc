@@ -217,6 +217,11 @@ struct Workspace {
   std::uint32_t phase_rounds = 0;
   DeviceBuffer tail_items, tail_rounds, tail_rakes;
   std::vector<std::uint32_t> tail_instances;
+  // MAP and sampling (phase_log.cuh): rounds run grid-wide, then the tail of
+  // every tree; none of the tail records exist when every round is grid-wide.
+  std::uint32_t log_rounds = 0;
+  bool log_tail = false;
+  DeviceBuffer phase_ends, log_tail_items, log_tail_rounds, log_tail_rakes;
   // Phase-ordered copy of the observations (PhasePlan::observation_order),
   // rebuilt on the device whenever observations are uploaded.
   DeviceBuffer phase_observations, observation_order;
@@ -267,13 +272,16 @@ struct Workspace {
     schedule = THMM_SCHEDULE_TEAMS;
     phase_rounds = 0;
     tail_instances.clear();
+    log_rounds = 0;
+    log_tail = false;
     observation_reads = 0;
     phase_batch = false;
     for (DeviceBuffer *buffer :
          {&programs, &steps, &rakes, &combines, &absorbs, &compress, &instances,
           &compress_ends, &gathers, &team_order, &stripe_order, &control, &node_in,
           &phase_rakes, &phase_gathers, &phase_compress, &phase_roots, &node_exp,
-          &comp_exp, &tail_items, &tail_rounds, &tail_rakes, &phase_observations,
+          &comp_exp, &tail_items, &tail_rounds, &tail_rakes, &phase_ends,
+          &log_tail_items, &log_tail_rounds, &log_tail_rakes, &phase_observations,
           &observation_order, &edge_in,
           &observations, &root_potential, &emission, &uniforms, &values,
           &node_out, &edge_out, &states_out, &scratch, &bytes})
@@ -474,12 +482,12 @@ struct Workspace {
     gathers.Upload(set.gathers, stream);
     instances.Upload(table, stream);
     team_order.Upload(order, stream);
-    // Phase schedule of the sum-product calls. A forest gets records for
-    // every tree; the batch API (one plan shared by every item, shared edge
-    // input) gets, for up to 4 states, the records of one tree, which every
-    // item reads (the shared-topology layout of phase_engine.cuh); above 4
-    // states the batch API keeps the per-tree engine.
-    if (PaddedStates(states) == 4 || !shared_edges) {
+    // Phase schedule. A forest gets records for every tree; the batch API
+    // (one plan shared by every item, shared edge input) gets the records of
+    // one tree, which every item reads (the shared-topology layout of
+    // phase_engine.cuh). The batch API's sum-product calls use it up to 4
+    // states and keep the per-tree engine above (LinearPhases).
+    if (PaddedStates(states) == 4 || !shared_edges || maximum || sampling) {
       phase_batch = shared_edges;
       std::vector<PhaseInstance> phase_instances(phase_batch ? 1 : count);
       for (std::size_t i = 0; i < phase_instances.size(); ++i)
@@ -498,6 +506,10 @@ struct Workspace {
         phase_gathers.Upload(phase.gathers, stream);
         phase_compress.Upload(phase.compress, stream);
         phase_roots.Upload(phase.roots, stream);
+        if (maximum || sampling) {
+          phase_ends.Upload(phase.ends, stream);
+          SetLogRounds();
+        }
         node_exp.Allocate(total_nodes * sizeof(int));
         comp_exp.Allocate(phase.total_compressions * copies * sizeof(int));
         observation_reads = categorical ? phase.observation_order.size() : 0;
@@ -509,6 +521,7 @@ struct Workspace {
         phase.gathers = {};
         phase.compress = {};
         phase.roots = {};
+        phase.ends = {};
         schedule = THMM_SCHEDULE_PHASES;
         SetPhaseRounds(0);
       }
@@ -823,10 +836,38 @@ struct Workspace {
     return false;
   }
 
+  static bool IsLogDomain(int operation) {
+    return operation == THMM_OP_MAXIMUM || operation == THMM_OP_SAMPLE;
+  }
+  // Whether the sum-product calls have phase kernels in this workspace.
+  bool LinearPhases() const {
+    return phase.enabled && phase.exponents_fit && (!phase_batch || states <= 4);
+  }
   bool UsePhases(int operation) const {
-    return schedule == THMM_SCHEDULE_PHASES && phase.enabled &&
-           (operation == THMM_OP_PARTITION || operation == THMM_OP_LOG_PARTITION ||
-            operation == THMM_OP_MARGINALS);
+    return schedule == THMM_SCHEDULE_PHASES &&
+           (IsLogDomain(operation) ? phase.enabled : LinearPhases());
+  }
+
+  // Grid-wide rounds of MAP and sampling: up to the first round whose
+  // operations, shared out over the trees, are at most four passes of a CTA
+  // (512 threads' worth; 64 operations at 8 states). From there a grid-wide
+  // launch would do less than its own launch costs, and one CTA per tree runs
+  // the remaining rounds, the root and their top-down steps in one launch. A
+  // forest of more than 2^20 trees stays grid-wide (its tail records).
+  void SetLogRounds() {
+    const std::uint64_t lanes = states <= 4 ? 1 : states <= 8 ? 8 : states <= 16 ? 16 : 32;
+    const std::uint64_t trees = phase.instance_program.size(); // 1 in the batch layout
+    log_rounds = phase.AutoTailRound(trees * (512 / lanes) + 1);
+    log_tail = trees <= (1u << 20);
+    if (!log_tail) {
+      log_rounds = phase.rounds;
+      return;
+    }
+    const PhasePlan::Tail tail = phase.BuildTail(log_rounds, true);
+    log_tail_items.Upload(tail.items, stream);
+    log_tail_rounds.Upload(tail.rounds, stream);
+    log_tail_rakes.Upload(tail.rakes, stream);
+    Check(cudaStreamSynchronize(stream), "tail record upload");
   }
 
   const PhaseRanges &PhaseRangesFor(std::uint32_t a, std::uint32_t b) {
@@ -845,16 +886,9 @@ struct Workspace {
     return phase_ranges.back();
   }
 
-  // Launches the phase schedule of `operation` over instances [a, b):
-  // gather and compress phases round by round, the finish phase, then (for
-  // marginals) the adjoint phases in reverse round order. Returns the number
-  // of kernel launches.
-  int LaunchPhases(int operation, std::uint32_t a, std::uint32_t b) {
-    // Batch layout: every item runs the one tree's operations; items [a, b).
-    const PhaseRanges &ranges = phase_batch ? PhaseRangesFor(0, 1) : PhaseRangesFor(a, b);
-    const std::size_t K = states;
-    const std::size_t compute_bytes = compute_f64 ? 8 : 4;
-    unsigned char *work = scratch.as<unsigned char>();
+  // Kernel arguments common to every phase kind of `operation` over instances
+  // (batch layout: items) [a, b).
+  PhaseArgs MakePhaseArgs(int operation, std::uint32_t a, std::uint32_t b) const {
     PhaseArgs args{};
     args.rakes = phase_rakes.as<uint4>();
     args.gathers = phase_gathers.as<uint4>();
@@ -867,13 +901,7 @@ struct Workspace {
     args.categories = static_cast<std::uint32_t>(categories);
     args.categorical = categorical ? 1u : 0u;
     args.edge_in = edge_in.ptr;
-    args.edge_modulus = shared_edge_input ? static_cast<std::uint32_t>(edges_per_item) : 0u;
     args.states = static_cast<std::uint32_t>(states);
-    args.nodes = work;
-    args.comps = work + total_nodes * K * compute_bytes;
-    const std::uint64_t copies = phase_batch ? capacity : 1;
-    args.comp_mu =
-        work + (total_nodes * K + phase.total_compressions * copies * K * K) * compute_bytes;
     if (phase_batch) {
       args.batch = 1;
       args.first_item = a;
@@ -881,20 +909,94 @@ struct Workspace {
       args.item_stride = capacity;
       args.item_nodes = nodes_per_item;
       args.item_edges = edges_per_item;
-      args.edge_modulus = 0;
     }
-    args.node_exp = node_exp.as<int>();
-    args.comp_exp = comp_exp.as<int>();
     args.values = values.ptr;
-    args.node_out = node_out.ptr;
-    args.edge_out = edge_out.ptr;
     args.raw = operation == THMM_OP_PARTITION ? 1u : 0u;
     args.reverse = operation == THMM_OP_MARGINALS ? 1u : 0u;
+    args.error = control.as<std::uint32_t>() + 2;
+    args.bf16 = bf16 ? 1u : 0u;
+    return args;
+  }
+
+  // Launches MAP or sampling over instances [a, b): gather and compress
+  // phases of the grid-wide rounds, the tail (or the roots), then the
+  // top-down phases in reverse round order. Returns the number of launches.
+  int LaunchLogPhases(int operation, std::uint32_t a, std::uint32_t b) {
+    const PhaseRanges &ranges = phase_batch ? PhaseRangesFor(0, 1) : PhaseRangesFor(a, b);
+    PhaseArgs args = MakePhaseArgs(operation, a, b);
+    if (!phase_batch) { // one item
+      args.items = 1;
+      args.item_stride = 1;
+    }
+    const std::size_t K = states, S = ScalarBytes();
+    const std::uint64_t copies = phase_batch ? capacity : 1;
+    const std::uint64_t rake_total = phase.rake_base[phase.rounds] * copies;
+    unsigned char *work = scratch.as<unsigned char>();
+    args.nodes = work;
+    args.branches = work + total_nodes * K * S;
+    args.comps = work + (total_nodes + rake_total) * K * S;
+    args.ends = phase_ends.as<uint2>();
+    args.rake_choices = bytes.as<std::uint8_t>();
+    args.comp_choices = bytes.as<std::uint8_t>() + rake_total * K;
+    args.states_out = states_out.as<std::uint32_t>();
+    args.uniforms = uniforms.ptr;
+    args.tail_items = log_tail_items.as<uint4>();
+    args.tail_rounds = log_tail_rounds.as<uint4>();
+    args.tail_rakes = log_tail_rakes.as<uint2>();
+    int count = 0;
+    const auto launch = [&](int kind, std::pair<std::uint64_t, std::uint64_t> range) {
+      if (range.second <= range.first)
+        return;
+      args.offset = static_cast<std::uint32_t>(range.first);
+      args.count = static_cast<std::uint32_t>(range.second - range.first);
+      const auto launcher =
+          operation == THMM_OP_MAXIMUM
+              ? (scalar == 8 ? LaunchPhaseMaximumF64 : LaunchPhaseMaximumF32)
+              : (scalar == 8 ? LaunchPhaseSampleF64 : LaunchPhaseSampleF32);
+      Check(launcher(kind, args, stream), "tree-HMM accelerator kernel launch");
+      ++count;
+    };
+    for (std::uint32_t r = 0; r < log_rounds; ++r) {
+      launch(kPhaseGather, ranges.gather[r]);
+      launch(kPhaseCompress, ranges.compress[r]);
+    }
+    launch(log_tail ? kPhaseTailForward : kPhaseFinish,
+           phase_batch ? std::pair<std::uint64_t, std::uint64_t>{0, 1}
+                       : std::pair<std::uint64_t, std::uint64_t>{a, b});
+    for (std::uint32_t r = log_rounds; r-- > 0;) {
+      launch(kPhaseCompressReverse, ranges.compress[r]);
+      launch(kPhaseRakeReverse, ranges.rake[r]);
+    }
+    return count;
+  }
+
+  // Launches the phase schedule of `operation` over instances [a, b):
+  // gather and compress phases round by round, the finish phase, then (for
+  // marginals) the adjoint phases in reverse round order. Returns the number
+  // of kernel launches.
+  int LaunchPhases(int operation, std::uint32_t a, std::uint32_t b) {
+    if (IsLogDomain(operation))
+      return LaunchLogPhases(operation, a, b);
+    // Batch layout: every item runs the one tree's operations; items [a, b).
+    const PhaseRanges &ranges = phase_batch ? PhaseRangesFor(0, 1) : PhaseRangesFor(a, b);
+    const std::size_t K = states;
+    const std::size_t compute_bytes = compute_f64 ? 8 : 4;
+    unsigned char *work = scratch.as<unsigned char>();
+    PhaseArgs args = MakePhaseArgs(operation, a, b);
+    if (shared_edge_input && !phase_batch)
+      args.edge_modulus = static_cast<std::uint32_t>(edges_per_item);
+    args.nodes = work;
+    args.comps = work + total_nodes * K * compute_bytes;
+    const std::uint64_t copies = phase_batch ? capacity : 1;
+    args.comp_mu =
+        work + (total_nodes * K + phase.total_compressions * copies * K * K) * compute_bytes;
+    args.node_exp = node_exp.as<int>();
+    args.comp_exp = comp_exp.as<int>();
+    args.node_out = node_out.ptr;
+    args.edge_out = edge_out.ptr;
     args.tail_items = tail_items.as<uint4>();
     args.tail_rounds = tail_rounds.as<uint4>();
     args.tail_rakes = tail_rakes.as<uint2>();
-    args.error = control.as<std::uint32_t>() + 2;
-    args.bf16 = bf16 ? 1u : 0u;
     int count = 0;
     const auto launch = [&](int kind, std::pair<std::uint64_t, std::uint64_t> range) {
       if (range.second <= range.first)
@@ -1057,8 +1159,18 @@ struct Workspace {
         }
       }
     }
-    // The phase schedule's one setting: how many rounds run grid-wide.
-    if (phase.enabled && operation != THMM_OP_MAXIMUM && operation != THMM_OP_SAMPLE) {
+    if (phase.enabled && IsLogDomain(operation)) {
+      schedule = THMM_SCHEDULE_PHASES;
+      const float ms = TimeSteps(operation, repeats);
+      ++tried;
+      if (ms < best.kernel_ms) {
+        best.kernel_ms = ms;
+        best.schedule = THMM_SCHEDULE_PHASES;
+        best.phase_rounds = phase_rounds;
+      }
+    }
+    // The sum-product phases' one setting: how many rounds run grid-wide.
+    if (LinearPhases() && !IsLogDomain(operation)) {
       schedule = THMM_SCHEDULE_PHASES;
       std::vector<std::uint32_t> tried_rounds;
       const std::uint32_t automatic = phase.AutoTailRound(1u << 17);
