@@ -1,6 +1,6 @@
 // Phase kernels of the level-synchronous schedule (phase.h) for 32 < K <= 128
 // states: round r of EVERY tree in one grid-wide launch per kind, as for
-// K <= 4, but one operation per CTA (128 threads at K_P = 64, 256 at 128;
+// K <= 4, but one operation per CTA (256 threads at K_P = 64, 512 at 128;
 // rakes: warp-per-row K x K matrix-vector products; compressions and their
 // adjoints: tcgen05 products with TMEM accumulators, as the per-tree
 // tensor-core engine).
@@ -46,10 +46,18 @@ namespace wide {
 // state count KP: operand parts of KP rows x a depth chunk of 64 (hi, lo of
 // X, then of Y; BF16 uses the hi parts only), then the K-vectors.
 template <int KP> struct PhaseLayout {
-  // Threads per CTA: 128 at KP = 64 (three CTAs per SM), 256 at KP = 128
-  // (one CTA per SM, so twice the warps for staging and epilogues; warps w
-  // and w + 4 share TMEM lane quarter w and split the columns).
-  static constexpr unsigned kThreads = KP == 64 ? 128u : 256u;
+  // Threads per CTA: 256 at KP = 64 (three CTAs per SM), 512 at KP = 128 (one
+  // CTA per SM); warps w, w + 4, ... share TMEM lane quarter w and split the
+  // columns. The kernels wait on global loads and barriers, so warps in
+  // flight count for more than registers: against half the threads the dense
+  // K = 64 step (64 trees x 2000 nodes) went from 7.70 to 6.82 ms although
+  // 80 registers spill a little, the K = 128 one (64 x 500) from 12.9 to
+  // 9.1 ms. Two CTAs of 256 threads without spills took 9.4 ms at K = 64.
+  static constexpr unsigned kThreads = KP == 64 ? 256u : 512u;
+  // Quads of each operand whose loads a thread has in flight: with 24 warps
+  // per SM at KP = 64 one is faster than two (6.82 against 7.74 ms), for the
+  // registers; at KP = 128 two (9.13 against 9.44 ms).
+  static constexpr unsigned kBatch = KP == 64 ? 1 : 2;
   static constexpr unsigned kPart = KP * kChunk * 4;
   static constexpr unsigned kXh = 0, kXl = kPart, kYh = 2 * kPart, kYl = 3 * kPart;
   static constexpr unsigned kVectorsAt = 4 * kPart;
@@ -81,7 +89,7 @@ struct PhaseShared {
   double root_sum;
   std::uint32_t tmem;
   int root_finite;
-  float reduce[8]; // one per warp (at most 256 threads)
+  float reduce[16]; // one per warp (at most 512 threads)
 };
 
 template <unsigned T> __device__ __forceinline__ float CtaMax(float v, PhaseShared &sh) {
@@ -185,15 +193,13 @@ struct RatioColumns {
 // for a later, shorter chunk), padded rows are never read.
 //
 // K % 4 == 0: each thread moves quads (4 consecutive depths of one row) in
-// passes of kBatch: all loads of a pass for both operands are issued before
+// passes of kBatch (PhaseLayout): all loads of a pass for both operands are issued before
 // any store, so a thread has up to 2 kBatch global loads in flight.
 //   * Row sources: a warp takes 8 rows x 4 quads, so its global loads are
 //     64-byte runs of 8 rows and its 16-byte shared-memory stores fill whole
 //     128-byte core-matrix rows (4 wavefronts for 512 bytes);
 //   * column sources: a warp takes 32 consecutive rows of one quad of
 //     depths, four coalesced 128-byte loads and one 16-byte store per thread.
-constexpr unsigned kBatch = 4;
-
 // This thread's walk over the quad slots of an operand chunk: slot
 // threadIdx.x, then every T-th. The row and quad of each slot are
 // advanced incrementally (one division when the walk starts, none per slot).
@@ -297,7 +303,7 @@ __device__ __forceinline__ void StageScalar(const Src &src, unsigned K, unsigned
 }
 
 // Stages depth chunk d0 of both operands of a product.
-template <bool kBf16, unsigned T, class XS, class YS>
+template <bool kBf16, unsigned T, unsigned kBatch, class XS, class YS>
 __device__ __forceinline__ void StageChunk(const XS &x, const YS &y, unsigned K, unsigned d0,
                                            unsigned char *xh, unsigned char *xl,
                                            unsigned char *yh, unsigned char *yl) {
@@ -416,9 +422,9 @@ __device__ bool PhaseProduct(unsigned char *smem, PhaseShared &sh, std::uint32_t
     const unsigned d0 = chunk * kChunk;
     constexpr unsigned T = L::kThreads;
     if (bf16)
-      StageChunk<true, T>(x, y, K, d0, xh, nullptr, yh, nullptr);
+      StageChunk<true, T, L::kBatch>(x, y, K, d0, xh, nullptr, yh, nullptr);
     else
-      StageChunk<false, T>(x, y, K, d0, xh, xl, yh, yl);
+      StageChunk<false, T, L::kBatch>(x, y, K, d0, xh, xl, yh, yl);
     ok = MmaChunk<KP, kSplit>(smem, sh, phase, tmem, chunk, bf16) && ok;
   }
   return ok;
@@ -426,7 +432,7 @@ __device__ bool PhaseProduct(unsigned char *smem, PhaseShared &sh, std::uint32_t
 
 // Stages depth chunk d0 of one operand (K % 4 == 0), loads batched as in
 // StageChunk.
-template <bool kBf16, unsigned T, class Src>
+template <bool kBf16, unsigned T, unsigned kBatch, class Src>
 __device__ __forceinline__ void StageOne(const Src &src, unsigned K, unsigned d0,
                                          unsigned char *hi, unsigned char *lo) {
   const unsigned depth = K - d0 < kChunk ? K - d0 : kChunk;
@@ -483,11 +489,11 @@ __device__ __forceinline__ void TransposeStaged(unsigned K, const unsigned char 
 // One operation of a wide phase kind, executed by the whole CTA.
 template <int KP> struct WideOps {
   // Threads of the CTA; a thread's TMEM lane (accumulator row) is
-  // threadIdx.x % 128, and with 256 threads the two halves of the CTA take
-  // the two halves of the columns.
+  // threadIdx.x % 128, and each 128 threads of the CTA take their part of
+  // the columns.
   static constexpr unsigned kThreads = PhaseLayout<KP>::kThreads;
-  static constexpr unsigned kHalves = kThreads / 128;
-  static constexpr unsigned kHalfColumns = KP / kHalves;
+  static constexpr unsigned kParts = kThreads / 128;
+  static constexpr unsigned kPartColumns = KP / kParts;
   const PhaseArgs &a;
   PhaseShared &sh;
   unsigned char *smem;
@@ -517,8 +523,7 @@ template <int KP> struct WideOps {
   __device__ __forceinline__ const float *PathPtr(std::uint32_t ref) const {
     if (ref & kFlag)
       return Comps() + static_cast<std::size_t>(ref & kMask) * KK;
-    const std::size_t edge = a.edge_modulus != 0 ? ref % a.edge_modulus : ref;
-    return static_cast<const float *>(a.edge_in) + edge * KK;
+    return static_cast<const float *>(a.edge_in) + static_cast<std::size_t>(ref) * KK;
   }
   __device__ __forceinline__ int PathExp(std::uint32_t ref) const {
     return (ref & kFlag) ? a.comp_exp[ref & kMask] : 0;
@@ -701,12 +706,12 @@ template <int KP> struct WideOps {
     ok = PhaseProduct<KP, true>(smem, sh, phase, tmem, K, Rows{PathPtr(op.x), middle},
                                 Columns{PathPtr(op.z)}, a.bf16 != 0) &&
          ok;
-    // Accumulator row `row` (TMEM lane), columns [c0, c0 + kHalfColumns).
-    const unsigned row = threadIdx.x % 128, c0 = (threadIdx.x / 128) * kHalfColumns;
+    // Accumulator row `row` (TMEM lane), columns [c0, c0 + kPartColumns).
+    const unsigned row = threadIdx.x % 128, c0 = (threadIdx.x / 128) * kPartColumns;
     const std::uint32_t lane_base = tmem + ((row & ~31u) << 16);
     float m = 0.0f;
 #pragma unroll 1
-    for (unsigned c = c0; c < c0 + kHalfColumns; c += 32) {
+    for (unsigned c = c0; c < c0 + kPartColumns; c += 32) {
       float values[32];
       SplitSum32<KP>(lane_base, c, values, a.bf16 != 0);
 #pragma unroll
@@ -720,7 +725,7 @@ template <int KP> struct WideOps {
       // Rows through the (now idle) operand buffers, then coalesced stores.
       float *tile = reinterpret_cast<float *>(smem);
 #pragma unroll 1
-      for (unsigned c = c0; c < c0 + kHalfColumns; c += 32) {
+      for (unsigned c = c0; c < c0 + kPartColumns; c += 32) {
         float values[32];
         SplitSum32<KP>(lane_base, c, values, a.bf16 != 0);
         if (row < K) {
@@ -737,7 +742,7 @@ template <int KP> struct WideOps {
             *reinterpret_cast<const float4 *>(tile + w.row * TileStride() + w.column);
     } else {
 #pragma unroll 1
-      for (unsigned c = c0; c < c0 + kHalfColumns; c += 32) {
+      for (unsigned c = c0; c < c0 + kPartColumns; c += 32) {
         float values[32];
         SplitSum32<KP>(lane_base, c, values, a.bf16 != 0);
         if (row < K) {
@@ -880,11 +885,12 @@ template <int KP> struct WideOps {
       unsigned char *const yh = smem + L::kYh, *const yl = smem + L::kYl;
       const bool bf16 = a.bf16 != 0;
       if (bf16)
-        StageChunk<true, kThreads>(RatioRows{mu, stored, ratio_of}, Rows{right, nullptr}, K, 0,
-                                   xh, nullptr, yh, nullptr);
+        StageChunk<true, kThreads, L::kBatch>(RatioRows{mu, stored, ratio_of},
+                                              Rows{right, nullptr}, K, 0, xh, nullptr, yh,
+                                              nullptr);
       else
-        StageChunk<false, kThreads>(RatioRows{mu, stored, ratio_of}, Rows{right, nullptr}, K, 0,
-                                    xh, xl, yh, yl);
+        StageChunk<false, kThreads, L::kBatch>(RatioRows{mu, stored, ratio_of},
+                                               Rows{right, nullptr}, K, 0, xh, xl, yh, yl);
       ok = MmaChunk<KP, false>(smem, sh, phase, tmem, 0, bf16) && ok;
       if (bf16)
         TransposeStaged<true, kThreads>(K, xh, xl, yh, yl);
@@ -892,9 +898,9 @@ template <int KP> struct WideOps {
         TransposeStaged<false, kThreads>(K, xh, xl, yh, yl);
       __syncthreads();
       if (bf16)
-        StageOne<true, kThreads>(Columns{left}, K, 0, xh, nullptr);
+        StageOne<true, kThreads, L::kBatch>(Columns{left}, K, 0, xh, nullptr);
       else
-        StageOne<false, kThreads>(Columns{left}, K, 0, xh, xl);
+        StageOne<false, kThreads, L::kBatch>(Columns{left}, K, 0, xh, xl);
       ok = MmaChunk<KP, false>(smem, sh, phase, tmem + KP, 0, bf16) && ok;
     } else {
       ok = PhaseProduct<KP, false>(smem, sh, phase, tmem, K, RatioRows{mu, stored, ratio_of},
@@ -904,8 +910,8 @@ template <int KP> struct WideOps {
                                    RatioColumns{mu, stored, ratio_of}, a.bf16 != 0) &&
            ok;
     }
-    // Accumulator row `row` (TMEM lane), columns [c0, c0 + kHalfColumns).
-    const unsigned row = threadIdx.x % 128, c0 = (threadIdx.x / 128) * kHalfColumns;
+    // Accumulator row `row` (TMEM lane), columns [c0, c0 + kPartColumns).
+    const unsigned row = threadIdx.x % 128, c0 = (threadIdx.x / 128) * kPartColumns;
     const std::uint32_t lane_base = tmem + ((row & ~31u) << 16);
     float *left_out = AdjointOf(op.x);
     float *right_out = AdjointOf(op.z);
@@ -916,7 +922,7 @@ template <int KP> struct WideOps {
       float *tile = reinterpret_cast<float *>(smem);
       const auto stage_rows = [&](std::uint32_t column) {
 #pragma unroll 1
-        for (unsigned c = c0; c < c0 + kHalfColumns; c += 32) {
+        for (unsigned c = c0; c < c0 + kPartColumns; c += 32) {
           float values[32];
           umma::Load32(lane_base + column + c, values);
           if (row < K)
@@ -972,7 +978,7 @@ template <int KP> struct WideOps {
       const float *right_row = right + static_cast<std::size_t>(row) * K;
       const float middle_row = row < K ? middle[row] : 0.0f;
 #pragma unroll 1
-      for (unsigned c = c0; c < c0 + kHalfColumns; c += 32) {
+      for (unsigned c = c0; c < c0 + kPartColumns; c += 32) {
         float p1[32];
         umma::Load32(lane_base + c, p1);
         if (row < K) {
@@ -985,7 +991,7 @@ template <int KP> struct WideOps {
       }
       float partial = 0.0f;
 #pragma unroll 1
-      for (unsigned c = c0; c < c0 + kHalfColumns; c += 32) {
+      for (unsigned c = c0; c < c0 + kPartColumns; c += 32) {
         float p2[32];
         umma::Load32(lane_base + KP + c, p2);
         if (row < K) {
@@ -999,13 +1005,17 @@ template <int KP> struct WideOps {
           }
         }
       }
-      if (kHalves == 1) {
+      // v, leaf, msg and (past middle) ratio are free here: one vector per
+      // part of the columns.
+      float *const parts[4] = {msg, ratio, v, leaf};
+      if (kParts == 1) {
         total = partial;
       } else {
-        (threadIdx.x < 128 ? msg : ratio)[row] = partial;
+        parts[threadIdx.x / 128][row] = partial;
         __syncthreads();
         if (j < K)
-          total = msg[j] + ratio[j];
+          for (unsigned h = 0; h < kParts; ++h)
+            total += parts[h][j];
       }
     }
     if (j < K)
