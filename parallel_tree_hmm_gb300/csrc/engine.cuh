@@ -921,7 +921,7 @@ struct LinearEngine {
       const double log_z =
           (flag || !(sum > 0.0))
               ? -INFINITY
-              : static_cast<double>(total) * 0.6931471805599453094 + log(sum);
+              : fma(static_cast<double>(total), 0.6931471805599453094, log(sum));
       static_cast<Scalar *>(c.a.values)[item] =
           static_cast<Scalar>(c.a.raw ? exp(log_z) : log_z);
       if (c.a.reverse) {

@@ -97,8 +97,6 @@ cudaError_t LaunchPhase(int scalar_bytes, bool compute_f64, int kind, const Phas
                ? LaunchWidePhase(kind, args, stream, blocks_per_sm)
                : cudaErrorInvalidValue;
   if (args.states > 4) {
-    if (args.batch)
-      return cudaErrorInvalidValue;
     if (args.states <= 8)
       return compute_f64
                  ? LaunchGroupPhase8F64(scalar_bytes, kind, args, stream, blocks_per_sm)

@@ -86,7 +86,6 @@ struct PhaseArgs {
   std::uint32_t categories;
   std::uint32_t categorical;
   const void *edge_in;
-  std::uint32_t edge_modulus; // > 0: shared edge input, row = path % edge_modulus
   std::uint32_t states;
   void *nodes;        // [node][K] stored (normalised) node values, compute type
   int *node_exp;      // [node] their power-of-two exponents
@@ -101,9 +100,9 @@ struct PhaseArgs {
   const uint4 *tail_items;
   const uint4 *tail_rounds;
   const uint2 *tail_rakes;
-  // Shared-topology layout only (batch set): items [first_item,
-  // first_item + items) of a batch whose stored objects are `item_stride`
-  // items apart, each with item_nodes nodes and item_edges edges.
+  // Shared-topology layout (batch set): items [first_item, first_item + items)
+  // of a batch whose stored objects are `item_stride` items apart, each with
+  // item_nodes nodes and item_edges edges. A forest is one item at stride 1.
   std::uint32_t batch;
   std::uint32_t first_item;
   std::uint32_t items;
@@ -111,7 +110,7 @@ struct PhaseArgs {
   std::uint64_t item_nodes;
   std::uint64_t item_edges;
   // MAP and sampling kinds (phase_log.cuh) only; their values are in the
-  // input precision, their layout always the batch one (a forest: one item).
+  // input precision.
   const uint2 *ends;         // [compression] parent and child node
   void *branches;            // [rake][K] partial sums of wide gathers
   std::uint8_t *rake_choices; // [rake][K]
@@ -187,8 +186,8 @@ PhasePlan BuildPhasePlan(const ProgramSet &set, std::span<const PhaseInstance> i
 // Launches one phase (or reports its occupancy when blocks_per_sm is
 // non-null). scalar_bytes: 4 or 8 (input/output type); compute_f64: FP64
 // arithmetic. Padded state count 4 (K <= 4) runs one thread per operation
-// (phase_engine.cuh); 4 < K <= 32 (forest layout, no tail kinds) one lane
-// group per operation (phase_groups.cuh); 32 < K <= 128 (FP32 only, forest
+// (phase_engine.cuh); 4 < K <= 32 (no tail kinds) one lane group per
+// operation (phase_groups.cuh); 32 < K <= 128 (FP32 only, forest
 // layout, no tail kinds) one CTA per operation (wide_phase.cuh).
 cudaError_t LaunchPhase(int scalar_bytes, bool compute_f64, int kind, const PhaseArgs &args,
                         cudaStream_t stream, int *blocks_per_sm);

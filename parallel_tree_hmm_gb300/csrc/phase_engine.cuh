@@ -23,15 +23,13 @@ constexpr int kPhaseThreads = 128;
 
 // Where the operands of one operation live. Forest layout: the records hold
 // absolute indices of every tree's nodes, edges and compressions, so every
-// map is the identity (a shared edge input is read modulo its edge count).
+// map is the identity.
 struct ForestIndex {
   __device__ __forceinline__ std::size_t Store(std::uint32_t node) const { return node; }
   __device__ __forceinline__ std::size_t Io(std::uint32_t node) const { return node; }
   __device__ __forceinline__ std::size_t Comp(std::uint32_t tape) const { return tape; }
   __device__ __forceinline__ std::size_t Out(std::uint32_t edge) const { return edge; }
-  __device__ __forceinline__ std::size_t In(const PhaseArgs &a, std::uint32_t edge) const {
-    return a.edge_modulus != 0 ? edge % a.edge_modulus : edge;
-  }
+  __device__ __forceinline__ std::size_t In(std::uint32_t edge) const { return edge; }
   __device__ __forceinline__ std::size_t Obs(std::uint32_t slot) const { return slot; }
 };
 
@@ -60,9 +58,7 @@ struct BatchIndex {
   __device__ __forceinline__ std::size_t Out(std::uint32_t edge) const {
     return item * edges + edge;
   }
-  __device__ __forceinline__ std::size_t In(const PhaseArgs &, std::uint32_t edge) const {
-    return edge;
-  }
+  __device__ __forceinline__ std::size_t In(std::uint32_t edge) const { return edge; }
   __device__ __forceinline__ std::size_t Obs(std::uint32_t slot) const {
     return slot * stride + item;
   }
@@ -127,7 +123,7 @@ template <typename Scalar, typename Compute, class Index> struct PhaseOps {
   }
 
   __device__ __forceinline__ const Scalar *EdgeIn(std::uint32_t path) const {
-    return static_cast<const Scalar *>(a.edge_in) + ix.In(a, path) * KK;
+    return static_cast<const Scalar *>(a.edge_in) + ix.In(path) * KK;
   }
 
   // Row r of path `ref` (zero for padded rows).
@@ -271,7 +267,7 @@ template <typename Scalar, typename Compute, class Index> struct PhaseOps {
       sum += static_cast<double>(root[j]);
     const double log_z = !(sum > 0.0)
                              ? -INFINITY
-                             : static_cast<double>(total) * 0.6931471805599453094 + log(sum);
+                             : fma(static_cast<double>(total), 0.6931471805599453094, log(sum));
     static_cast<Scalar *>(a.values)[value] = static_cast<Scalar>(a.raw ? exp(log_z) : log_z);
     if (a.reverse) {
       Scalar *root_out = static_cast<Scalar *>(a.node_out) + ix.Io(node) * K;

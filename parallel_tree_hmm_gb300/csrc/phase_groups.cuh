@@ -1,18 +1,39 @@
 // Phase kernels of the level-synchronous schedule (phase.h) for 4 < K <= 32
-// states: one lane group of G = K_P lanes per operation (K_P = 8, 16 or 32,
-// the padded state count), lane r holding row r of the operation's K x K
-// matrices, as the lane-group (G > 1) branch of LinearEngine (engine.cuh).
-// Above 16 states the FP32 kernels size their register rows to K rounded
-// up to a multiple of 4 (20, 24, 28 or 32) rather than 32, which cuts the
-// padded arithmetic and the registers (at K = 20, 2.6x fewer multiply-adds
-// per compression) without changing a bit.
+// states: one lane group of G = 8, 16 or 32 lanes per operation, the
+// operation's K x K matrices in shared memory, products in register tiles.
 //
-// Each operation performs exactly that branch's floating-point operations
-// in the same order, so the phase and per-tree schedules agree bit for bit;
-// as in the K <= 4 phase kernels only the bookkeeping of the power-of-two
-// exponents differs (carried per stored object here, summed per team
-// there; both are exact integer sums). Forest layout only, and no tail
-// kinds: every round runs grid-wide.
+// Each operation performs exactly the floating-point operations of the
+// lane-group (G > 1) branch of LinearEngine (engine.cuh), every sum in the
+// same order, so the phase and per-tree schedules agree bit for bit; as in the
+// K <= 4 phase kernels only the bookkeeping of the power-of-two exponents
+// differs (carried per stored object here, summed per team there; both are
+// exact integer sums). Which lane forms which element is free, and that is
+// where the time went: with lane r holding row r, a K = 20 product took 100
+// broadcast loads and 20 rows of register traffic per lane, 20 of 32 lanes
+// worked, and the edge adjoints left by 4-byte stores 80 bytes apart.
+//
+// What bounds them now: shared-memory loads and multiply-adds, then DRAM.
+//   * A matrix arrives by asynchronous 16-byte copies (cp.async) in the
+//     caller's row-major order: coalesced, no registers held while in flight.
+//   * Lane (ti, tj) of the group owns TR x 4 elements of a product and reads
+//     16-byte quads: TR + 4 of them per TR x 4 x 4 multiply-adds. At K = 20,
+//     25 lanes own 4 x 4 tiles and a product takes 40 loads and 320
+//     multiply-adds per lane.
+//   * Row pitches P with P / 4 odd make the quads of consecutive rows fall on
+//     different banks; a lane's rows are RG apart for the same reason.
+//   * Adjoints are formed in place in shared memory and leave in 16-byte
+//     coalesced stores.
+// Measured on one GB300, rows per lane -> tiles: one reverse compression
+// launch list of 256 recursive trees x 5000 nodes at K = 20 3.24 -> 0.79 ms
+// (some 6,900 -> 1,500 warp instructions each), compressions 1.03 -> 0.28 ms,
+// rake adjoints 1.68 -> 0.71 ms (5.4 TB/s), gathers 0.91 -> 0.61 ms; that
+// marginal step 6.65 -> 2.23 ms. The batch API, 500 items on a 399-node tree
+// at K = 20, 1.62 -> 0.40 ms (the per-tree engine before).
+//
+// Both layouts of phase_engine.cuh: a forest (every tree's records, one item)
+// and the batch API's shared topology (one tree's records, stored objects
+// item-minor, the groups of a warp on consecutive items of one operation). No
+// tail kinds: every round runs grid-wide.
 #ifndef THMM_PHASE_GROUPS_CUH_
 #define THMM_PHASE_GROUPS_CUH_
 
@@ -26,421 +47,739 @@ namespace thmm {
 
 constexpr int kGroupPhaseThreads = 128;
 
-// Minimum resident blocks per SM (a register cap of 65536 / (128 n) per
-// thread), chosen so that no FP32 variant spills.
-template <int KMAX, bool kWide> constexpr int GroupPhaseMinBlocks() {
-  if constexpr (KMAX <= 16)
-    return kWide ? 3 : 4;
-  else if constexpr (KMAX <= 24)
-    return kWide ? 2 : 4;
+// Tile shape for padded state count KMAX (a multiple of 4): KMAX / 4 column
+// quads times RG row groups of TR rows fit the G lanes.
+template <int KMAX> struct GroupTile {
+  static constexpr int G = GroupLanes<KMAX>();
+  static constexpr int CQ = KMAX / 4;
+  static constexpr int TR = KMAX <= 8 ? 2 : KMAX <= 20 ? 4 : 8;
+  static constexpr int RG = (KMAX + TR - 1) / TR;
+  static constexpr int kRows = RG * TR;
+  static constexpr int P = (kRows / 4) % 2 == 1 ? kRows : kRows + 4;
+  static constexpr int kMatrix = kRows * P; // elements of one matrix buffer
+  static_assert(RG * CQ <= G && G >= KMAX, "tiles and rows fit the group");
+};
+
+// Elements of shared memory per lane group.
+template <int KMAX, int kKind>
+inline constexpr int kGroupPhaseElements =
+    kKind == kPhaseGather            ? 2 * (GroupTile<KMAX>::kMatrix + KMAX)
+    : kKind == kPhaseRakeReverse     ? GroupTile<KMAX>::kMatrix + 2 * KMAX
+    : kKind == kPhaseCompress        ? 2 * GroupTile<KMAX>::kMatrix + KMAX
+    : kKind == kPhaseCompressReverse ? 4 * GroupTile<KMAX>::kMatrix + KMAX
+                                     : 0;
+
+// Four consecutive values at a 16-byte boundary.
+template <typename T> __device__ __forceinline__ void Load4(const T *p, T (&out)[4]) {
+  if constexpr (sizeof(T) == 4) {
+    const float4 v = *reinterpret_cast<const float4 *>(p);
+    out[0] = v.x, out[1] = v.y, out[2] = v.z, out[3] = v.w;
+  } else {
+    const double2 v = reinterpret_cast<const double2 *>(p)[0];
+    const double2 w = reinterpret_cast<const double2 *>(p)[1];
+    out[0] = v.x, out[1] = v.y, out[2] = w.x, out[3] = w.y;
+  }
+}
+template <bool kStreaming = false, typename D, typename T>
+__device__ __forceinline__ void Store4(D *p, const T (&in)[4]) {
+  if constexpr (sizeof(D) == 4) {
+    const float4 v = make_float4(static_cast<float>(in[0]), static_cast<float>(in[1]),
+                                 static_cast<float>(in[2]), static_cast<float>(in[3]));
+    if constexpr (kStreaming)
+      __stcs(reinterpret_cast<float4 *>(p), v);
+    else
+      *reinterpret_cast<float4 *>(p) = v;
+  } else {
+    const double2 v = make_double2(static_cast<double>(in[0]), static_cast<double>(in[1]));
+    const double2 w = make_double2(static_cast<double>(in[2]), static_cast<double>(in[3]));
+    if constexpr (kStreaming) {
+      __stcs(reinterpret_cast<double2 *>(p), v);
+      __stcs(reinterpret_cast<double2 *>(p) + 1, w);
+    } else {
+      reinterpret_cast<double2 *>(p)[0] = v;
+      reinterpret_cast<double2 *>(p)[1] = w;
+    }
+  }
+}
+
+// Asynchronous global -> shared copies of 16 (4, 8) bytes.
+template <int kBytes> __device__ __forceinline__ void CopyAsync(void *dst, const void *src) {
+  const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+  if constexpr (kBytes == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at), "l"(src) : "memory");
   else
-    return kWide ? 2 : 3;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(at), "l"(src), "n"(kBytes)
+                 : "memory");
+}
+__device__ __forceinline__ void CopyCommit() {
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int kPending> __device__ __forceinline__ void CopyWait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
 }
 
 template <typename Scalar, typename Compute, int KMAX> struct GroupPhaseOps {
-  // KMAX: the register arrays' length (K rounded up to a multiple of 4
-  // above 16 states, else the padded state count); G >= KMAX lanes per
-  // group, lane r holding row r (lanes >= K hold zero rows). Terms past K
-  // are exact zeros, so every KMAX >= K gives the same bits.
-  static constexpr int G = GroupLanes<KMAX>();
-  static_assert(G >= KMAX, "one row per lane");
+  using Tile = GroupTile<KMAX>;
+  static constexpr int G = Tile::G, CQ = Tile::CQ, TR = Tile::TR, RG = Tile::RG, P = Tile::P;
   const PhaseArgs &a;
   unsigned K;
   unsigned KK;
+  std::size_t item;   // batch item (0 for a forest)
+  std::size_t stride; // items per stored object (1 for a forest)
+  unsigned lane;      // lane within the group
+  unsigned mask;      // the group's lanes of the warp
+  unsigned ti, tj;    // this lane's tile (ti < RG for lanes that own one)
+  Compute *smem;      // the group's shared memory
 
-  __device__ explicit GroupPhaseOps(const PhaseArgs &args)
-      : a(args), K(args.states), KK(args.states * args.states) {}
+  __device__ __forceinline__ GroupPhaseOps(const PhaseArgs &args, std::uint32_t batch_item,
+                                           Compute *group_smem)
+      : a(args), K(args.states), KK(args.states * args.states), item(batch_item),
+        stride(args.item_stride), lane(threadIdx.x % G),
+        mask(G == 32 ? kFull : ((1u << (G & 31)) - 1u) << (threadIdx.x % 32 / G * G)),
+        ti(lane / CQ), tj(lane % CQ), smem(group_smem) {}
 
-  __device__ __forceinline__ Compute *Nodes() const { return static_cast<Compute *>(a.nodes); }
-  __device__ __forceinline__ Compute *Comps() const { return static_cast<Compute *>(a.comps); }
-  __device__ __forceinline__ Compute *CompMu() const { return static_cast<Compute *>(a.comp_mu); }
-  __device__ __forceinline__ Scalar *NodeOut() const { return static_cast<Scalar *>(a.node_out); }
+  __device__ __forceinline__ std::size_t Store(std::uint32_t object) const {
+    return object * stride + item;
+  }
+  __device__ __forceinline__ std::size_t Io(std::uint32_t node) const {
+    return item * a.item_nodes + node;
+  }
+  __device__ __forceinline__ Compute *NodeAt(std::uint32_t node) const {
+    return static_cast<Compute *>(a.nodes) + Store(node) * K;
+  }
+  __device__ __forceinline__ Scalar *NodeOutAt(std::uint32_t node) const {
+    return static_cast<Scalar *>(a.node_out) + Io(node) * K;
+  }
+  __device__ __forceinline__ Compute *CompAt(std::uint32_t tape) const {
+    return static_cast<Compute *>(a.comps) + Store(tape) * KK;
+  }
+  __device__ __forceinline__ Compute *CompMuAt(std::uint32_t tape) const {
+    return static_cast<Compute *>(a.comp_mu) + Store(tape) * KK;
+  }
+  __device__ __forceinline__ const Scalar *EdgeAt(std::uint32_t edge) const {
+    return static_cast<const Scalar *>(a.edge_in) + static_cast<std::size_t>(edge) * KK;
+  }
 
-  // Input factor vector of `node`: dense row, or the reference's categorical
-  // (root ? root_potential : 1) * emission[observation]
+  // Element j < K of `node`'s input factor: dense row, or the reference's
+  // categorical (root ? root_potential : 1) * emission[observation]
   // (src/gpu_backend_impl.inc:326-382), as Context::InputNode.
-  __device__ __forceinline__ void Input(std::uint32_t node, std::uint32_t obs, bool root,
-                                        Compute (&out)[KMAX]) const {
-    Scalar raw[KMAX];
-    if (!a.categorical) {
-      LoadRow<KMAX>(static_cast<const Scalar *>(a.node_in) + static_cast<std::size_t>(node) * K,
-                    K, raw);
-    } else {
-      const Scalar *root_potential = static_cast<const Scalar *>(a.root_potential);
-      if (obs == kNone) {
-#pragma unroll
-        for (unsigned j = 0; j < KMAX; ++j)
-          raw[j] = j < K ? (root ? root_potential[j] : Scalar(1)) : Scalar(0);
-      } else {
-        const unsigned category = a.observations[obs];
-        if (category >= a.categories) {
-#pragma unroll
-          for (unsigned j = 0; j < KMAX; ++j)
-            raw[j] = Scalar(0);
-        } else {
-          LoadRow<KMAX>(static_cast<const Scalar *>(a.emission) + category * K, K, raw);
-          if (root) {
-#pragma unroll
-            for (unsigned j = 0; j < KMAX; ++j)
-              raw[j] = j < K ? root_potential[j] * raw[j] : Scalar(0);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (unsigned j = 0; j < KMAX; ++j)
-      out[j] = static_cast<Compute>(raw[j]);
+  __device__ __forceinline__ Scalar Input(std::uint32_t node, std::uint32_t obs, bool root,
+                                          unsigned j) const {
+    if (!a.categorical)
+      return static_cast<const Scalar *>(a.node_in)[Io(node) * K + j];
+    const Scalar *root_potential = static_cast<const Scalar *>(a.root_potential);
+    if (obs == kNone)
+      return root ? root_potential[j] : Scalar(1);
+    const unsigned category = a.observations[Store(obs)];
+    if (category >= a.categories)
+      return Scalar(0);
+    const Scalar emitted = static_cast<const Scalar *>(a.emission)[category * K + j];
+    return root ? root_potential[j] * emitted : emitted;
   }
-
-  // Value of a rake leaf or compression middle (every lane the whole
-  // vector): the stored value (adding its exponent to `e`) or the input.
-  __device__ __forceinline__ void Node(std::uint32_t ref, std::uint32_t obs,
-                                       Compute (&out)[KMAX], int &e) const {
+  // Element `lane` of a rake leaf or compression middle (0 past K): the
+  // stored value (adding its exponent to `e`) or the input factor.
+  __device__ __forceinline__ Compute Node(std::uint32_t ref, std::uint32_t obs, int &e) const {
     if (ref & kFlag) {
-      const std::uint32_t node = ref & kMask;
-      LoadRow<KMAX>(Nodes() + static_cast<std::size_t>(node) * K, K, out);
-      e += a.node_exp[node];
-    } else {
-      Input(ref, obs, false, out);
+      e += a.node_exp[Store(ref & kMask)];
+      return lane < K ? NodeAt(ref & kMask)[lane] : Compute(0);
     }
-  }
-
-  __device__ __forceinline__ const Scalar *EdgeIn(std::uint32_t path) const {
-    const std::size_t edge = a.edge_modulus != 0 ? path % a.edge_modulus : path;
-    return static_cast<const Scalar *>(a.edge_in) + edge * KK;
-  }
-  __device__ __forceinline__ void PathRow(std::uint32_t ref, unsigned r,
-                                          Compute (&out)[KMAX]) const {
-    if (r >= K) {
-#pragma unroll
-      for (unsigned j = 0; j < KMAX; ++j)
-        out[j] = Compute(0);
-    } else if (ref & kFlag) {
-      LoadRow<KMAX>(Comps() + static_cast<std::size_t>(ref & kMask) * KK + r * K, K, out);
-    } else {
-      LoadRow<KMAX>(EdgeIn(ref) + r * K, K, out);
-    }
-  }
-  __device__ __forceinline__ Compute PathElem(std::uint32_t ref, unsigned i, unsigned j) const {
-    return (ref & kFlag) ? Comps()[static_cast<std::size_t>(ref & kMask) * KK + i * K + j]
-                         : static_cast<Compute>(EdgeIn(ref)[i * K + j]);
+    return lane < K ? static_cast<Compute>(Input(ref, obs, false, lane)) : Compute(0);
   }
   __device__ __forceinline__ int PathExp(std::uint32_t ref) const {
-    return (ref & kFlag) ? a.comp_exp[ref & kMask] : 0;
+    return (ref & kFlag) ? a.comp_exp[Store(ref & kMask)] : 0;
   }
   __device__ __forceinline__ static int Exponent(Compute m) {
     return m > Compute(0) ? Pow2Exponent(m) : 0;
   }
-  __device__ __forceinline__ void StorePathAdjoint(std::uint32_t ref, unsigned r,
-                                                   const Compute (&row)[KMAX]) const {
+  __device__ __forceinline__ Compute Max(Compute v) const {
+#pragma unroll
+    for (int offset = G / 2; offset > 0; offset >>= 1) {
+      const Compute other = __shfl_xor_sync(mask, v, offset, G);
+      v = v < other ? other : v;
+    }
+    return v;
+  }
+
+  // ------------------------------------------------ matrices and shared memory
+  // Zero padding of a matrix buffer whose K is below KMAX (the copies write
+  // rows and columns below K only).
+  __device__ __forceinline__ void ClearPadding(Compute *m) const {
+    if (K != KMAX)
+      for (unsigned i = lane; i < Tile::kMatrix; i += G)
+        m[i] = Compute(0);
+  }
+  // Starts copying a K x K matrix into `m` (pitch P); complete after
+  // CopyCommit, CopyWait and a group barrier.
+  template <typename T> __device__ __forceinline__ void StageFrom(const T *src, Compute *m) const {
+    if (K == KMAX) { // rows of whole 16-byte quads
+      constexpr int kQuads = KMAX * CQ;
+#pragma unroll
+      for (int first = 0; first < kQuads; first += G) {
+        const unsigned q = first + lane;
+        if (kQuads % G == 0 || q < kQuads) {
+          Compute *dst = m + (q / CQ) * P + 4 * (q % CQ);
+          if constexpr (sizeof(T) == sizeof(Compute)) {
+#pragma unroll
+            for (unsigned part = 0; part < sizeof(T) / 4; ++part)
+              CopyAsync<16>(dst + part * 2, src + 4 * q + part * 2);
+          } else {
+            T in[4];
+            Load4(src + 4 * q, in);
+            const Compute out[4] = {static_cast<Compute>(in[0]), static_cast<Compute>(in[1]),
+                                    static_cast<Compute>(in[2]), static_cast<Compute>(in[3])};
+            Store4(dst, out);
+          }
+        }
+      }
+    } else {
+      unsigned r = lane / K, c = lane % K;
+      const unsigned step_r = G / K, step_c = G % K;
+      for (unsigned i = lane; i < KK; i += G) {
+        if constexpr (sizeof(T) == sizeof(Compute))
+          CopyAsync<sizeof(T)>(m + r * P + c, src + i);
+        else
+          m[r * P + c] = static_cast<Compute>(src[i]);
+        r += step_r;
+        c += step_c;
+        if (c >= K) {
+          c -= K;
+          ++r;
+        }
+      }
+    }
+  }
+  __device__ __forceinline__ void Stage(std::uint32_t ref, Compute *m) const {
     if (ref & kFlag)
-      StoreRow<KMAX>(CompMu() + static_cast<std::size_t>(ref & kMask) * KK + r * K, K, row);
+      StageFrom(static_cast<const Compute *>(CompAt(ref & kMask)), m);
     else
-      StoreRowStreaming<KMAX>(static_cast<Scalar *>(a.edge_out) +
-                                  static_cast<std::size_t>(ref) * KK + r * K,
-                              K, row);
+      StageFrom(EdgeAt(ref), m);
+  }
+  // Writes the K x K matrix in `m` out, transformed element by element
+  // (value, row, column).
+  template <bool kStreaming, typename T, class Map>
+  __device__ __forceinline__ void Drain(const Compute *m, T *dst, Map map) const {
+    if (K == KMAX) {
+      constexpr int kQuads = KMAX * CQ;
+#pragma unroll
+      for (int first = 0; first < kQuads; first += G) {
+        const unsigned q = first + lane;
+        if (kQuads % G == 0 || q < kQuads) {
+          const unsigned r = q / CQ, c = 4 * (q % CQ);
+          Compute v[4];
+          Load4(m + r * P + c, v);
+          map(v, r, c);
+          Store4<kStreaming>(dst + 4 * q, v);
+        }
+      }
+    } else {
+      unsigned r = lane / K, c = lane % K;
+      const unsigned step_r = G / K, step_c = G % K;
+      for (unsigned i = lane; i < KK; i += G) {
+        Compute v[1] = {m[r * P + c]};
+        map(v, r, c);
+        if constexpr (kStreaming)
+          __stcs(dst + i, static_cast<T>(v[0]));
+        else
+          dst[i] = static_cast<T>(v[0]);
+        r += step_r;
+        c += step_c;
+        if (c >= K) {
+          c -= K;
+          ++r;
+        }
+      }
+    }
+  }
+  // The adjoint of path `ref` (a compressed path's stays, an edge's is the
+  // caller's marginal).
+  template <class Map>
+  __device__ __forceinline__ void DrainAdjoint(std::uint32_t ref, const Compute *m,
+                                               Map map) const {
+    if (ref & kFlag)
+      Drain<false>(m, CompMuAt(ref & kMask), map);
+    else
+      Drain<true>(m,
+                  static_cast<Scalar *>(a.edge_out) +
+                      (item * a.item_edges + ref) * static_cast<std::size_t>(KK),
+                  map);
+  }
+
+  // Row `lane` of `m` times `x`, terms in order.
+  __device__ __forceinline__ Compute RowDot(const Compute *m, const Compute *x) const {
+    Compute dot = Compute(0);
+    const Compute *row = m + (lane < KMAX ? lane : 0u) * P;
+#pragma unroll
+    for (unsigned j = 0; j < KMAX; j += 4) {
+      if (j < K) {
+        Compute u[4], v[4];
+        Load4(row + j, u);
+        Load4(x + j, v);
+#pragma unroll
+        for (int d = 0; d < 4; ++d)
+          dot = fma(u[d], v[d], dot);
+      }
+    }
+    return dot;
   }
 
   // ---------------------------------------------------------- forward
   // Rakes of gather i absorbed into its parent (LinearEngine::AbsorbRake):
-  // lane r holds element r of the parent's value. Groups of a warp share
-  // the shuffles, so every group runs the warp's largest rake count and a
-  // group past its own rakes computes on a stand-in and keeps nothing.
-  __device__ __forceinline__ void Gather(std::uint32_t i, bool active, unsigned lane) const {
+  // lane r holds element r of the parent's value. The next rake's matrix and
+  // leaf are on their way while this one is worked on.
+  __device__ __forceinline__ void Gather(std::uint32_t i) const {
     const uint4 op = a.gathers[i];
     const std::uint32_t node = op.x & kMask;
-    Compute v;
+    const std::uint32_t count = op.w & kCountMask;
+    // Two buffers of a matrix and a leaf vector each.
+    const auto matrix = [&](unsigned at) { return smem + at * Tile::kMatrix; };
+    const auto leaf = [&](unsigned at) { return smem + 2 * Tile::kMatrix + at * KMAX; };
+    uint4 rake = a.rakes[op.z];
+    ClearPadding(matrix(0));
+    ClearPadding(matrix(1));
+    __syncwarp(mask);
+    int next_exp = PathExp(rake.x);
+    Stage(rake.x, matrix(0));
+    CopyCommit();
+    Compute next_leaf = Node(rake.y, rake.z, next_exp);
+    if (count > 1)
+      rake = a.rakes[op.z + 1];
+    Compute v = Compute(0);
     int e = 0;
     if (op.x & kFlag) {
-      Compute input[KMAX];
-      Input(node, op.y, (op.w & kRootBit) != 0, input);
-      v = lane < K ? Select(input, lane) : Compute(0);
+      if (lane < K)
+        v = static_cast<Compute>(Input(node, op.y, (op.w & kRootBit) != 0, lane));
     } else {
-      v = lane < K ? Nodes()[static_cast<std::size_t>(node) * K + lane] : Compute(0);
-      e = a.node_exp[node];
+      if (lane < K)
+        v = NodeAt(node)[lane];
+      e = a.node_exp[Store(node)];
     }
-    const std::uint32_t count = op.w & kCountMask;
-    const unsigned rounds = __reduce_max_sync(kFull, active ? count : 0u);
-    for (unsigned k = 0; k < rounds; ++k) {
-      const bool live = active && k < count;
-      // rounds > 0: some group has a rake, so rake 0 (and its path) exist.
-      const uint4 rake = a.rakes[live ? op.z + k : 0u];
-      int le = 0;
-      Compute leaf[KMAX];
-      Node(rake.y, rake.z, leaf, le);
-      le += PathExp(rake.x);
-      Compute row[KMAX];
-      PathRow(rake.x, lane, row);
-      Compute dot = Compute(0);
-#pragma unroll
-      for (unsigned j = 0; j < KMAX; ++j)
-        dot = fma(row[j], leaf[j], dot);
-      const int s1 = Exponent(GroupMax<G>(dot));
-      const Compute value = v * ScalePow2(dot, -s1);
-      const int s2 = Exponent(GroupMax<G>(value));
-      if (live) {
-        v = ScalePow2(value, -s2);
-        e += le + s1 + s2;
+    for (std::uint32_t k = 0; k < count; ++k) {
+      const unsigned at = k & 1u;
+      if (lane < KMAX)
+        leaf(at)[lane] = next_leaf;
+      e += next_exp;
+      if (k + 1 < count) {
+        next_exp = PathExp(rake.x);
+        Stage(rake.x, matrix(at ^ 1u));
+        CopyCommit();
+        next_leaf = Node(rake.y, rake.z, next_exp);
+        if (k + 2 < count)
+          rake = a.rakes[op.z + k + 2];
+        CopyWait<1>();
+      } else {
+        CopyWait<0>();
       }
+      __syncwarp(mask);
+      Compute dot = RowDot(matrix(at), leaf(at));
+      if (lane >= K)
+        dot = Compute(0);
+      const int s1 = Exponent(Max(dot));
+      const Compute value = v * ScalePow2(dot, -s1);
+      const int s2 = Exponent(Max(value)); // also: every lane is done with matrix(at)
+      v = ScalePow2(value, -s2);
+      e += s1 + s2;
     }
-    if (active && lane < K)
-      Nodes()[static_cast<std::size_t>(node) * K + lane] = v;
-    if (active && lane == 0)
-      a.node_exp[node] = e;
+    if (lane < K)
+      NodeAt(node)[lane] = v;
+    if (lane == 0)
+      a.node_exp[Store(node)] = e;
   }
 
-  // Compressed path i = left * diag(middle) * right; lane r computes row r.
-  __device__ __forceinline__ void Compress(std::uint32_t i, bool active, unsigned lane) const {
-    const uint4 op = a.compress[i];
-    int e = PathExp(op.x) + PathExp(op.z);
-    Compute middle[KMAX];
-    Node(op.y, op.w, middle, e);
-    Compute left[KMAX];
-    Compute out[KMAX];
-    PathRow(op.x, lane, left);
+  // acc[q][c] += sum over d of A[ti + RG q][d] * B[d][4 tj + c].
+  __device__ __forceinline__ void Product(const Compute *A, const Compute *B,
+                                          Compute (&acc)[TR][4]) const {
+    const Compute *rows = A + (ti < RG ? ti : 0u) * P;
+    const Compute *columns = B + 4 * tj;
 #pragma unroll
-    for (unsigned j = 0; j < KMAX; ++j)
-      out[j] = Compute(0);
+    for (unsigned d0 = 0; d0 < KMAX; d0 += 4) {
+      if (d0 < K) {
+        Compute u[TR][4];
 #pragma unroll
-    for (unsigned mid = 0; mid < KMAX; ++mid) {
-      if (mid < K) {
-        Compute right[KMAX];
-        PathRow(op.z, mid, right);
-        const Compute weight = left[mid] * middle[mid];
+        for (int q = 0; q < TR; ++q)
+          Load4(rows + q * RG * P + d0, u[q]);
 #pragma unroll
-        for (unsigned j = 0; j < KMAX; ++j)
-          out[j] = fma(weight, right[j], out[j]);
+        for (int d = 0; d < 4; ++d) {
+          Compute w[4];
+          Load4(columns + (d0 + d) * P, w);
+#pragma unroll
+          for (int q = 0; q < TR; ++q)
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              acc[q][c] = fma(u[q][d], w[c], acc[q][c]);
+        }
       }
     }
+  }
+
+  // The weights left[r][m] * middle[m] of a compression, from `left` into
+  // `out` (which may be `left`).
+  __device__ __forceinline__ void Weigh(const Compute *left, const Compute *middle,
+                                        Compute *out) const {
+    constexpr int kQuads = KMAX * CQ;
+#pragma unroll
+    for (int first = 0; first < kQuads; first += G) {
+      const unsigned q = first + lane;
+      if (kQuads % G == 0 || q < kQuads) {
+        const unsigned at = (q / CQ) * P + 4 * (q % CQ);
+        Compute v[4], w[4];
+        Load4(left + at, v);
+        Load4(middle + 4 * (q % CQ), w);
+#pragma unroll
+        for (int d = 0; d < 4; ++d)
+          v[d] = v[d] * w[d];
+        Store4(out + at, v);
+      }
+    }
+  }
+
+  // Compressed path i = left * diag(middle) * right.
+  __device__ __forceinline__ void Compress(std::uint32_t i) const {
+    const uint4 op = a.compress[i];
+    Compute *left = smem, *right = smem + Tile::kMatrix, *middle = smem + 2 * Tile::kMatrix;
+    ClearPadding(left);
+    ClearPadding(right);
+    __syncwarp(mask);
+    Stage(op.x, left);
+    Stage(op.z, right);
+    CopyCommit();
+    int e = PathExp(op.x) + PathExp(op.z);
+    const Compute own = Node(op.y, op.w, e);
+    if (lane < KMAX)
+      middle[lane] = own;
+    CopyWait<0>();
+    __syncwarp(mask);
+    Weigh(left, middle, left);
+    __syncwarp(mask);
+    Compute out[TR][4];
+#pragma unroll
+    for (int q = 0; q < TR; ++q)
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        out[q][c] = Compute(0);
+    Product(left, right, out);
     Compute m = Compute(0);
 #pragma unroll
-    for (unsigned j = 0; j < KMAX; ++j)
-      m = m < out[j] ? out[j] : m;
-    const int s = Exponent(GroupMax<G>(m));
-    if (active && lane < K) {
+    for (int q = 0; q < TR; ++q)
+      if (ti < RG && ti + q * RG < K)
 #pragma unroll
-      for (unsigned j = 0; j < KMAX; ++j)
-        out[j] = ScalePow2(out[j], -s);
-      StoreRow<KMAX>(Comps() + static_cast<std::size_t>(i) * KK + lane * K, K, out);
+        for (int c = 0; c < 4; ++c)
+          m = m < out[q][c] ? out[q][c] : m; // columns past K are zero
+    const int s = Exponent(Max(m));
+    Compute *dst = CompAt(i);
+    if (ti < RG) {
+#pragma unroll
+      for (int q = 0; q < TR; ++q) {
+        const unsigned r = ti + q * RG;
+        if (r < K) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            out[q][c] = ScalePow2(out[q][c], -s);
+          if (K == KMAX) {
+            Store4(dst + r * KMAX + 4 * tj, out[q]);
+          } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              if (4 * tj + c < K)
+                dst[r * K + 4 * tj + c] = out[q][c];
+          }
+        }
+      }
     }
-    if (active && lane == 0)
-      a.comp_exp[i] = e + s;
+    if (lane == 0)
+      a.comp_exp[Store(i)] = e + s;
   }
 
   // log Z = ln 2 * (root exponent) + log(sum(root)), as LinearEngine::Run
-  // (one thread per instance).
-  __device__ __forceinline__ void Finish(std::uint32_t i) const {
+  // (one thread): root record i, result of instance `value`.
+  __device__ __forceinline__ void Finish(std::uint32_t i, std::uint32_t value) const {
     const uint2 rec = a.roots[i];
     const std::uint32_t node = rec.x & kMask;
     Compute root[KMAX];
     long long total = 0;
     if (rec.x & kFlag) {
-      LoadRow<KMAX>(Nodes() + static_cast<std::size_t>(node) * K, K, root);
-      total = a.node_exp[node];
+#pragma unroll
+      for (unsigned j = 0; j < KMAX; ++j)
+        root[j] = j < K ? NodeAt(node)[j] : Compute(0);
+      total = a.node_exp[Store(node)];
     } else {
-      Input(node, rec.y, true, root);
+#pragma unroll
+      for (unsigned j = 0; j < KMAX; ++j)
+        root[j] = j < K ? static_cast<Compute>(Input(node, rec.y, true, j)) : Compute(0);
     }
     double sum = 0.0;
     for (unsigned j = 0; j < KMAX; ++j)
       sum += static_cast<double>(root[j]);
     const double log_z = !(sum > 0.0)
                              ? -INFINITY
-                             : static_cast<double>(total) * 0.6931471805599453094 + log(sum);
-    static_cast<Scalar *>(a.values)[i] = static_cast<Scalar>(a.raw ? exp(log_z) : log_z);
+                             : fma(static_cast<double>(total), 0.6931471805599453094, log(sum));
+    static_cast<Scalar *>(a.values)[value] = static_cast<Scalar>(a.raw ? exp(log_z) : log_z);
     if (a.reverse) {
-      Scalar *root_out = NodeOut() + static_cast<std::size_t>(node) * K;
+      Scalar *root_out = NodeOutAt(node);
       const bool finite = log_z > -INFINITY;
-      for (unsigned j = 0; j < K; ++j) {
-        double value = 0.0;
 #pragma unroll
-        for (unsigned k = 0; k < KMAX; ++k)
-          if (k == j)
-            value = static_cast<double>(root[k]);
-        root_out[j] = static_cast<Scalar>(finite ? value / sum : 0.0);
-      }
+      for (unsigned j = 0; j < KMAX; ++j)
+        if (j < K)
+          root_out[j] =
+              static_cast<Scalar>(finite ? static_cast<double>(root[j]) / sum : 0.0);
     }
   }
 
   // ---------------------------------------------------------- adjoint
-  __device__ __forceinline__ void RakeReverse(std::uint32_t i, bool active, unsigned lane) const {
+  __device__ __forceinline__ void RakeReverse(std::uint32_t i) const {
     const uint4 op = a.rakes[i];
-    Compute leaf[KMAX];
+    Compute *matrix = smem, *leaf = smem + Tile::kMatrix, *ratio = leaf + KMAX;
+    ClearPadding(matrix);
+    __syncwarp(mask);
+    Stage(op.x, matrix);
+    CopyCommit();
     int unused = 0;
-    Node(op.y, op.z, leaf, unused);
+    const Compute own = Node(op.y, op.z, unused);
     const Compute parent_adjoint =
-        lane < K ? static_cast<Compute>(NodeOut()[static_cast<std::size_t>(op.w) * K + lane])
-                 : Compute(0);
-    Compute row[KMAX];
-    PathRow(op.x, lane, row);
-    Compute unnormalised = Compute(0);
+        lane < K ? static_cast<Compute>(NodeOutAt(op.w)[lane]) : Compute(0);
+    if (lane < KMAX)
+      leaf[lane] = own;
+    CopyWait<0>();
+    __syncwarp(mask);
+    const Compute unnormalised = RowDot(matrix, leaf);
+    if (lane < KMAX)
+      ratio[lane] = lane < K && unnormalised > Compute(0) ? parent_adjoint / unnormalised
+                                                          : Compute(0);
+    __syncwarp(mask);
+    // Edge adjoint: ratio[r] * path[r][c] * leaf[c].
+    DrainAdjoint(op.x, matrix, [&](auto &v, unsigned r, unsigned c) {
+      const Compute ratio_r = ratio[r];
 #pragma unroll
-    for (unsigned j = 0; j < KMAX; ++j)
-      unnormalised = fma(row[j], leaf[j], unnormalised);
-    const Compute ratio = unnormalised > Compute(0) ? parent_adjoint / unnormalised : Compute(0);
-    if (active && lane < K) {
-      Compute w[KMAX];
-#pragma unroll
-      for (unsigned j = 0; j < KMAX; ++j)
-        w[j] = ratio * row[j] * leaf[j];
-      StorePathAdjoint(op.x, lane, w);
-    }
+      for (unsigned d = 0; d < sizeof(v) / sizeof(v[0]); ++d)
+        v[d] = ratio_r * v[d] * leaf[c + d];
+    });
     // Leaf adjoint: leaf[j] * sum_p ratio_p * path[p][j].
     Compute column = Compute(0);
-    for (unsigned p = 0; p < K; ++p) {
-      const Compute ratio_p = GroupBroadcast<G>(ratio, static_cast<int>(p));
-      if (lane < K)
-        column = fma(ratio_p, PathElem(op.x, p, lane), column);
+    const Compute *down = matrix + (lane < KMAX ? lane : 0u);
+#pragma unroll
+    for (unsigned p = 0; p < KMAX; p += 4) {
+      if (p < K) {
+        Compute u[4];
+        Load4(ratio + p, u);
+#pragma unroll
+        for (int d = 0; d < 4; ++d)
+          column = fma(u[d], down[(p + d) * P], column);
+      }
     }
-    if (active && lane < K)
-      NodeOut()[static_cast<std::size_t>(op.y & kMask) * K + lane] =
-          static_cast<Scalar>(Select(leaf, lane) * column);
+    if (lane < K)
+      NodeOutAt(op.y & kMask)[lane] = static_cast<Scalar>(own * column);
   }
 
-  // Adjoint of compression i; `tile` is this group's K x K shared-memory
-  // scratch for the ratio matrix.
-  __device__ __forceinline__ void CompressReverse(std::uint32_t i, bool active, unsigned lane,
-                                                  Compute *tile) const {
+  // Adjoint of compression i.
+  __device__ __forceinline__ void CompressReverse(std::uint32_t i) const {
     const uint4 op = a.compress[i];
-    const Compute *output_adjoint = CompMu() + static_cast<std::size_t>(i) * KK;
-    Compute middle[KMAX];
-    int unused = 0;
-    Node(op.y, op.w, middle, unused);
-    // Unnormalised output row `lane`, recomputed with the forward's
-    // operation order, and ratio = adjoint / output.
-    Compute left[KMAX];
-    Compute ratio[KMAX];
-    PathRow(op.x, lane, left);
+    Compute *left = smem, *right = left + Tile::kMatrix, *weight = right + Tile::kMatrix,
+            *ratio = weight + Tile::kMatrix, *middle = ratio + Tile::kMatrix;
+    ClearPadding(left);
+    ClearPadding(right);
+    ClearPadding(ratio);
+    __syncwarp(mask);
+    Stage(op.x, left);
+    Stage(op.z, right);
+    CopyCommit();
+    // The output's adjoint, in this lane's product tile.
+    const Compute *output_adjoint = CompMuAt(i);
+    Compute adjoint[TR][4];
 #pragma unroll
-    for (unsigned j = 0; j < KMAX; ++j)
-      ratio[j] = Compute(0);
-#pragma unroll
-    for (unsigned mid = 0; mid < KMAX; ++mid) {
-      if (mid < K) {
-        Compute right[KMAX];
-        PathRow(op.z, mid, right);
-        const Compute weight = left[mid] * middle[mid];
-#pragma unroll
-        for (unsigned j = 0; j < KMAX; ++j)
-          ratio[j] = fma(weight, right[j], ratio[j]);
-      }
-    }
-    {
-      Compute adjoint[KMAX];
-      if (lane < K) {
-        LoadRow<KMAX>(output_adjoint + lane * K, K, adjoint);
+    for (int q = 0; q < TR; ++q) {
+      const unsigned r = ti + q * RG;
+      if (K == KMAX && ti < RG && (RG * TR == KMAX || r < K)) {
+        Load4(output_adjoint + r * KMAX + 4 * tj, adjoint[q]);
       } else {
 #pragma unroll
-        for (unsigned j = 0; j < KMAX; ++j)
-          adjoint[j] = Compute(0);
+        for (int c = 0; c < 4; ++c)
+          adjoint[q][c] = ti < RG && r < K && 4 * tj + c < K
+                              ? output_adjoint[r * K + 4 * tj + c]
+                              : Compute(0);
       }
-#pragma unroll
-      for (unsigned j = 0; j < KMAX; ++j)
-        ratio[j] = ratio[j] > Compute(0) ? adjoint[j] / ratio[j] : Compute(0);
     }
-    // Left adjoint row `lane`: left[r][m] middle[m] sum_j right[m][j] ratio[r][j].
+    int unused = 0;
+    const Compute own = Node(op.y, op.w, unused);
+    if (lane < KMAX)
+      middle[lane] = own;
+    CopyWait<0>();
+    __syncwarp(mask);
+    Weigh(left, middle, weight);
+    __syncwarp(mask);
+    // Unnormalised output, recomputed with the forward's operation order, and
+    // ratio = adjoint / output.
+    Compute acc[TR][4];
+#pragma unroll
+    for (int q = 0; q < TR; ++q)
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        acc[q][c] = Compute(0);
+    Product(weight, right, acc);
+#pragma unroll
+    for (int q = 0; q < TR; ++q) {
+      const unsigned r = ti + q * RG;
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        acc[q][c] = acc[q][c] > Compute(0) ? adjoint[q][c] / acc[q][c] : Compute(0);
+      if (ti < RG && r < K)
+        Store4(ratio + r * P + 4 * tj, acc[q]);
+    }
+    __syncwarp(mask);
+    // Left adjoint: left[r][m] middle[m] sum_j right[m][j] ratio[r][j], this
+    // lane's elements r = ti + RG q, m = tj + CQ c, in place of the weights.
+#pragma unroll
+    for (int q = 0; q < TR; ++q)
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        acc[q][c] = Compute(0);
     {
-      Compute left_adjoint[KMAX];
+      const Compute *rows = ratio + (ti < RG ? ti : 0u) * P;
+      const Compute *columns = right + tj * P;
 #pragma unroll
-      for (unsigned mid = 0; mid < KMAX; ++mid) {
-        left_adjoint[mid] = Compute(0);
-        if (mid < K) {
-          Compute right[KMAX];
-          PathRow(op.z, mid, right);
-          Compute dot = Compute(0);
+      for (unsigned d0 = 0; d0 < KMAX; d0 += 4) {
+        if (d0 < K) {
+          Compute u[TR][4];
 #pragma unroll
-          for (unsigned j = 0; j < KMAX; ++j)
-            dot = fma(right[j], ratio[j], dot);
-          left_adjoint[mid] = left[mid] * middle[mid] * dot;
+          for (int q = 0; q < TR; ++q)
+            Load4(rows + q * RG * P + d0, u[q]);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            Compute w[4];
+            Load4(columns + c * CQ * P + d0, w);
+#pragma unroll
+            for (int q = 0; q < TR; ++q)
+#pragma unroll
+              for (int d = 0; d < 4; ++d)
+                acc[q][c] = fma(w[d], u[q][d], acc[q][c]);
+          }
         }
       }
-      if (active && lane < K)
-        StorePathAdjoint(op.x, lane, left_adjoint);
     }
-    // Right adjoint row m = lane: right[m][j] middle[m] sum_p left[p][m] ratio[p][j],
-    // with the ratio rows of the group in shared memory.
-    if (lane < K) {
+    if (ti < RG) {
 #pragma unroll
-      for (unsigned j = 0; j < KMAX; ++j)
-        if (j < K)
-          tile[lane * K + j] = ratio[j];
-    }
-    __syncwarp();
-    if (lane < K) {
-      Compute acc[KMAX];
+      for (int q = 0; q < TR; ++q) {
+        const unsigned r = ti + q * RG;
+        if (RG * TR == KMAX || r < KMAX)
 #pragma unroll
-      for (unsigned j = 0; j < KMAX; ++j)
-        acc[j] = Compute(0);
-      for (unsigned p = 0; p < K; ++p) {
-        const Compute left_p = PathElem(op.x, p, lane);
-#pragma unroll
-        for (unsigned j = 0; j < KMAX; ++j)
-          if (j < K)
-            acc[j] = fma(left_p, tile[p * K + j], acc[j]);
+          for (int c = 0; c < 4; ++c) {
+            Compute *w = weight + r * P + tj + CQ * c;
+            *w = *w * acc[q][c];
+          }
       }
-      const Compute own_middle = Select(middle, lane);
-      Compute right[KMAX];
-      PathRow(op.z, lane, right);
-      Compute right_adjoint[KMAX];
+    }
+    // Right adjoint: right[m][j] middle[m] sum_p left[p][m] ratio[p][j], this
+    // lane's elements m = TR ti + q, j = 4 tj + c, in place of the right factor.
+#pragma unroll
+    for (int q = 0; q < TR; ++q)
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        acc[q][c] = Compute(0);
+    {
+      const unsigned m0 = TR * (ti < RG ? ti : 0u);
+#pragma unroll 4
+      for (unsigned p = 0; p < K; ++p) {
+        Compute u[TR], w[4];
+        if constexpr (TR >= 4) {
+#pragma unroll
+          for (int part = 0; part < TR; part += 4) {
+            Compute four[4];
+            Load4(left + p * P + m0 + part, four);
+#pragma unroll
+            for (int d = 0; d < 4; ++d)
+              u[part + d] = four[d];
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < TR; ++q)
+            u[q] = left[p * P + m0 + q];
+        }
+        Load4(ratio + p * P + 4 * tj, w);
+#pragma unroll
+        for (int q = 0; q < TR; ++q)
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            acc[q][c] = fma(u[q], w[c], acc[q][c]);
+      }
+      __syncwarp(mask); // every lane is done with right, and weight is written
+      if (ti < RG) {
+#pragma unroll
+        for (int q = 0; q < TR; ++q) {
+          const unsigned m = m0 + q;
+          if (RG * TR == KMAX || m < KMAX) {
+            Compute v[4];
+            Load4(right + m * P + 4 * tj, v);
+            const Compute middle_m = middle[m];
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              v[c] = v[c] * middle_m * acc[q][c];
+            Store4(right + m * P + 4 * tj, v);
+          }
+        }
+      }
+    }
+    const auto same = [](auto &, unsigned, unsigned) {};
+    DrainAdjoint(op.x, weight, same);
+    __syncwarp(mask);
+    DrainAdjoint(op.z, right, same);
+    // Middle adjoint: the right adjoint's row sums.
+    if (lane < K) {
       Compute total = Compute(0);
 #pragma unroll
-      for (unsigned j = 0; j < KMAX; ++j) {
-        right_adjoint[j] = right[j] * own_middle * acc[j];
-        total += right_adjoint[j];
+      for (unsigned j = 0; j < KMAX; j += 4) {
+        if (j < K) {
+          Compute v[4];
+          Load4(right + lane * P + j, v);
+#pragma unroll
+          for (int d = 0; d < 4; ++d)
+            total += v[d];
+        }
       }
-      if (active) {
-        StorePathAdjoint(op.z, lane, right_adjoint);
-        NodeOut()[static_cast<std::size_t>(op.y & kMask) * K + lane] = static_cast<Scalar>(total);
-      }
+      NodeOutAt(op.y & kMask)[lane] = static_cast<Scalar>(total);
     }
-    __syncwarp();
   }
 };
 
-// Shared memory of a block: one K_P x K_P ratio tile per lane group (the
-// reverse compression kind only).
-template <typename Compute, int KMAX>
-constexpr unsigned GroupPhaseSmem(int kind) {
-  return kind == kPhaseCompressReverse
-             ? (kGroupPhaseThreads / GroupLanes<KMAX>()) * KMAX * KMAX *
-                   static_cast<unsigned>(sizeof(Compute))
-             : 0u;
+// Minimum resident blocks per SM (a register cap of 65536 / (128 n) per
+// thread), chosen so that no FP32 variant spills.
+template <int KMAX, bool kWide> constexpr int GroupPhaseMinBlocks(int kind) {
+  if (kWide)
+    return KMAX <= 16 ? 3 : 2;
+  return kind == kPhaseCompressReverse ? (KMAX <= 8 ? 6 : KMAX <= 20 ? 5 : 3)
+                                       : (KMAX <= 20 ? 8 : 5);
 }
 
-// One kind of one round: lane group g of the grid runs operation offset + g
-// (finish: thread t the root record of instance offset + t).
+// One kind of one round: lane group g of the grid runs operation offset + g /
+// items of item first_item + g % items (finish: thread t the root record).
 template <typename Scalar, typename Compute, int KMAX, int kKind>
 __global__ void __launch_bounds__(kGroupPhaseThreads,
-                                  GroupPhaseMinBlocks<KMAX, sizeof(Compute) == 8>())
+                                  GroupPhaseMinBlocks<KMAX, sizeof(Compute) == 8>(kKind))
     GroupPhaseKernel(PhaseArgs args) {
   using Ops = GroupPhaseOps<Scalar, Compute, KMAX>;
-  constexpr int G = Ops::G;
-  const Ops ops(args);
-  const std::uint32_t t = blockIdx.x * kGroupPhaseThreads + threadIdx.x;
-  if constexpr (kKind == kPhaseFinish) {
-    if (t < args.count)
-      ops.Finish(args.offset + t);
-  } else {
-    // Whole warps past the last group leave together (no shuffle partner
-    // of a live group leaves).
-    if ((t & ~31u) / G >= args.count)
-      return;
-    const std::uint32_t group = t / G;
-    const unsigned lane = threadIdx.x % G;
-    const bool active = group < args.count;
-    // A padding group of a live warp reads the last operation, writes nothing.
-    const std::uint32_t i = args.offset + (active ? group : args.count - 1);
-    if constexpr (kKind == kPhaseGather) {
-      ops.Gather(i, active, lane);
-    } else if constexpr (kKind == kPhaseCompress) {
-      ops.Compress(i, active, lane);
-    } else if constexpr (kKind == kPhaseRakeReverse) {
-      ops.RakeReverse(i, active, lane);
-    } else if constexpr (kKind == kPhaseCompressReverse) {
-      extern __shared__ __align__(16) unsigned char group_smem[];
-      Compute *tile = reinterpret_cast<Compute *>(group_smem) + (threadIdx.x / G) * KMAX * KMAX;
-      ops.CompressReverse(i, active, lane, tile);
-    }
+  constexpr int G = kKind == kPhaseFinish ? 1 : Ops::G;
+  constexpr int kElements = kGroupPhaseElements<KMAX, kKind>;
+  extern __shared__ __align__(16) unsigned char group_smem[];
+  const std::uint64_t t =
+      static_cast<std::uint64_t>(blockIdx.x) * kGroupPhaseThreads + threadIdx.x;
+  const auto g = static_cast<std::uint32_t>(t / G); // below 2^31 (the record index limit)
+  if (g >= args.count * args.items)
+    return;
+  std::uint32_t op = g, item = 0;
+  if (args.batch) {
+    op = g / args.items;
+    item = args.first_item + g % args.items;
   }
+  const std::uint32_t i = args.offset + op;
+  const Ops ops(args, item,
+                reinterpret_cast<Compute *>(group_smem) + threadIdx.x / G * kElements);
+  if constexpr (kKind == kPhaseFinish)
+    ops.Finish(i, args.batch ? item : i);
+  else if constexpr (kKind == kPhaseGather)
+    ops.Gather(i);
+  else if constexpr (kKind == kPhaseCompress)
+    ops.Compress(i);
+  else if constexpr (kKind == kPhaseRakeReverse)
+    ops.RakeReverse(i);
+  else if constexpr (kKind == kPhaseCompressReverse)
+    ops.CompressReverse(i);
 }
 
 } // namespace thmm

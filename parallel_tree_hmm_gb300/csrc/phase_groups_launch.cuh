@@ -12,7 +12,10 @@ namespace group_phase {
 template <typename Scalar, typename Compute, int KMAX, int kKind>
 cudaError_t LaunchKind(const PhaseArgs &args, cudaStream_t stream, int *blocks_per_sm) {
   auto kernel = GroupPhaseKernel<Scalar, Compute, KMAX, kKind>;
-  const unsigned smem = GroupPhaseSmem<Compute, KMAX>(kKind);
+  constexpr unsigned lanes = kKind == kPhaseFinish ? 1 : GroupLanes<KMAX>();
+  constexpr unsigned smem = kGroupPhaseThreads / lanes * kGroupPhaseElements<KMAX, kKind> *
+                            static_cast<unsigned>(sizeof(Compute));
+  static_assert(smem <= 227 * 1024, "shared memory per block");
   if (smem > 48 * 1024) {
     const cudaError_t status = cudaFuncSetAttribute(
         kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
@@ -22,13 +25,11 @@ cudaError_t LaunchKind(const PhaseArgs &args, cudaStream_t stream, int *blocks_p
   if (blocks_per_sm != nullptr)
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kernel,
                                                          kGroupPhaseThreads, smem);
-  if (args.count == 0)
+  if (args.count == 0 || args.items == 0)
     return cudaSuccess;
   // Finish: one thread per instance; the other kinds one lane group per
-  // operation.
-  const std::uint64_t threads =
-      kKind == kPhaseFinish ? static_cast<std::uint64_t>(args.count)
-                            : static_cast<std::uint64_t>(args.count) * GroupLanes<KMAX>();
+  // operation and item.
+  const std::uint64_t threads = static_cast<std::uint64_t>(args.count) * args.items * lanes;
   const std::uint64_t grid = (threads + kGroupPhaseThreads - 1) / kGroupPhaseThreads;
   if (grid > 0x7fffffffull)
     return cudaErrorInvalidConfiguration;

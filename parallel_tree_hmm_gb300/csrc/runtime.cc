@@ -485,9 +485,9 @@ struct Workspace {
     // Phase schedule. A forest gets records for every tree; the batch API
     // (one plan shared by every item, shared edge input) gets the records of
     // one tree, which every item reads (the shared-topology layout of
-    // phase_engine.cuh). The batch API's sum-product calls use it up to 4
-    // states and keep the per-tree engine above (LinearPhases).
-    if (PaddedStates(states) == 4 || !shared_edges || maximum || sampling) {
+    // phase_engine.cuh); the batch API above 32 states keeps the per-tree
+    // tensor-core engine.
+    if (states <= 32 || !shared_edges) {
       phase_batch = shared_edges;
       std::vector<PhaseInstance> phase_instances(phase_batch ? 1 : count);
       for (std::size_t i = 0; i < phase_instances.size(); ++i)
@@ -841,7 +841,7 @@ struct Workspace {
   }
   // Whether the sum-product calls have phase kernels in this workspace.
   bool LinearPhases() const {
-    return phase.enabled && phase.exponents_fit && (!phase_batch || states <= 4);
+    return phase.enabled && phase.exponents_fit;
   }
   bool UsePhases(int operation) const {
     return schedule == THMM_SCHEDULE_PHASES &&
@@ -902,6 +902,8 @@ struct Workspace {
     args.categorical = categorical ? 1u : 0u;
     args.edge_in = edge_in.ptr;
     args.states = static_cast<std::uint32_t>(states);
+    args.items = 1;
+    args.item_stride = 1;
     if (phase_batch) {
       args.batch = 1;
       args.first_item = a;
@@ -924,10 +926,6 @@ struct Workspace {
   int LaunchLogPhases(int operation, std::uint32_t a, std::uint32_t b) {
     const PhaseRanges &ranges = phase_batch ? PhaseRangesFor(0, 1) : PhaseRangesFor(a, b);
     PhaseArgs args = MakePhaseArgs(operation, a, b);
-    if (!phase_batch) { // one item
-      args.items = 1;
-      args.item_stride = 1;
-    }
     const std::size_t K = states, S = ScalarBytes();
     const std::uint64_t copies = phase_batch ? capacity : 1;
     const std::uint64_t rake_total = phase.rake_base[phase.rounds] * copies;
@@ -983,8 +981,6 @@ struct Workspace {
     const std::size_t compute_bytes = compute_f64 ? 8 : 4;
     unsigned char *work = scratch.as<unsigned char>();
     PhaseArgs args = MakePhaseArgs(operation, a, b);
-    if (shared_edge_input && !phase_batch)
-      args.edge_modulus = static_cast<std::uint32_t>(edges_per_item);
     args.nodes = work;
     args.comps = work + total_nodes * K * compute_bytes;
     const std::uint64_t copies = phase_batch ? capacity : 1;
