@@ -172,13 +172,21 @@ struct Workspace {
   int cta_cap[4] = {0, 0, 0, 0};
   float tuned_ms = 0.0f;
 
-  // Instantiated CUDA graphs of the device-only step, per operation and batch.
+  // Instantiated CUDA graphs of the device step, per operation and batch (at
+  // most kMaxGraphs, the oldest given up first).
   struct Graph {
     int operation;
     std::size_t batch;
     cudaGraphExec_t exec;
+    std::uint64_t launches;
   };
+  static constexpr std::size_t kMaxGraphs = 16;
   std::vector<Graph> graphs;
+  // Consecutive prepared calls of one operation and batch, launched one by
+  // one before their graph is built (EnqueuePrepared).
+  int repeated_operation = -1;
+  std::size_t repeated_batch = 0;
+  int repeats = 0;
 
   // Striped prepared calls. The instances of a call are cut into up to
   // kMaxStripes contiguous stripes of about equal node count; stripe c's
@@ -255,6 +263,7 @@ struct Workspace {
     for (Graph &graph : graphs)
       static_cast<void>(cudaGraphExecDestroy(graph.exec));
     graphs.clear();
+    repeats = 0;
   }
 
   void Clear() noexcept {
@@ -1066,8 +1075,15 @@ struct Workspace {
     for (const Graph &graph : graphs)
       if (graph.operation == operation && graph.batch == batch) {
         Check(cudaGraphLaunch(graph.exec, stream), "cudaGraphLaunch");
+        launches = graph.launches;
         return;
       }
+    if (graphs.size() >= kMaxGraphs) {
+      // Its last replay may still run.
+      Check(cudaStreamSynchronize(stream), "graph replay");
+      Check(cudaGraphExecDestroy(graphs.front().exec), "cudaGraphExecDestroy");
+      graphs.erase(graphs.begin());
+    }
     cudaGraph_t graph = nullptr;
     Check(cudaStreamBeginCapture(stream, cudaStreamCaptureModeRelaxed),
           "cudaStreamBeginCapture");
@@ -1084,8 +1100,31 @@ struct Workspace {
     const cudaError_t status = cudaGraphInstantiate(&exec, graph, 0);
     static_cast<void>(cudaGraphDestroy(graph));
     Check(status, "cudaGraphInstantiate");
-    graphs.push_back({operation, batch, exec});
+    graphs.push_back({operation, batch, exec, launches});
     Check(cudaGraphLaunch(exec, stream), "cudaGraphLaunch");
+  }
+
+  // The device step of a prepared call. Launching a chain of 20 to 100 small
+  // kernels one by one costs the host 2 to 3 us each, replaying its graph 10
+  // to 20 us in all; building the graph costs as much as some ten calls save,
+  // so it is built when an operation has been called kGraphAfter times in a
+  // row on one batch size.
+  static constexpr int kGraphAfter = 8;
+  void EnqueuePrepared(int operation, std::size_t batch) {
+    if (operation != repeated_operation || batch != repeated_batch) {
+      repeated_operation = operation;
+      repeated_batch = batch;
+      repeats = 0;
+    }
+    bool replay = repeats >= kGraphAfter;
+    for (const Graph &graph : graphs)
+      replay = replay || (graph.operation == operation && graph.batch == batch);
+    if (replay) {
+      EnqueueGraph(operation, batch);
+    } else {
+      ++repeats;
+      EnqueueDevice(operation, batch);
+    }
   }
 
   static int KernelSlot(int operation) {
@@ -1240,7 +1279,7 @@ struct Workspace {
       OrderObservations(stream);
     Check(cudaEventRecord(events[1], stream), "cudaEventRecord");
     Check(cudaEventRecord(events[2], stream), "cudaEventRecord");
-    EnqueueDevice(operation, batch);
+    EnqueuePrepared(operation, batch);
     Check(cudaEventRecord(events[3], stream), "cudaEventRecord");
     Check(cudaEventRecord(events[4], stream), "cudaEventRecord");
     const std::size_t S = ScalarBytes();
