@@ -101,8 +101,11 @@ __device__ __forceinline__ double ScalePow2(double v, int s) {
   return ldexp(v, s);
 }
 
-__device__ __forceinline__ float PortableExp(float x) { return thmm_expf(x); }
-__device__ __forceinline__ double PortableExp(double x) { return thmm_exp(x); }
+// exp(x) for x <= 0 (or NaN): the arguments of log-sum-exp.
+__device__ __forceinline__ float PortableExpNonPositive(float x) {
+  return thmm_expf_nonpositive(x);
+}
+__device__ __forceinline__ double PortableExpNonPositive(double x) { return thmm_exp(x); }
 __device__ __forceinline__ float PortableLog(float x) { return thmm_logf(x); }
 __device__ __forceinline__ double PortableLog(double x) { return thmm_log(x); }
 
@@ -1196,7 +1199,7 @@ __device__ __forceinline__ T LogSumExp(const T (&terms)[KMAX], unsigned K) {
 #pragma unroll
   for (unsigned j = 0; j < KMAX; ++j)
     if (j < K)
-      sum = sum + PortableExp(terms[j] - maximum);
+      sum = sum + PortableExpNonPositive(terms[j] - maximum);
   return maximum + PortableLog(sum);
 }
 
@@ -1212,7 +1215,7 @@ __device__ __forceinline__ unsigned SampleLogWeights(const T (&terms)[KMAX],
   for (unsigned j = 0; j < KMAX; ++j) {
     if (j < K && isfinite(terms[j])) {
       last = j;
-      cumulative = cumulative + PortableExp(terms[j] - normalizer);
+      cumulative = cumulative + PortableExpNonPositive(terms[j] - normalizer);
       if (uniform < cumulative)
         return j;
     }

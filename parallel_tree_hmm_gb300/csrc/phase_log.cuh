@@ -43,6 +43,92 @@ constexpr int kLogPhaseThreads = 128;
 // different banks.
 template <int KMAX> inline constexpr int kLogTile = KMAX * KMAX + 8;
 
+// Logarithms and exponentials four at a time, without branches: a branch per
+// element would put each some 20 to 30 instructions in a block of its own.
+// Elements outside the range of the short forms (subnormal or infinite
+// factors; exponents between -104 and -87) send the four to the general
+// functions, which give the same bits inside the range.
+__device__ __forceinline__ void PotentialLogs(float (&v)[4]) {
+  float out[4];
+  bool rare = false;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const unsigned bits = __float_as_uint(v[j]);
+    out[j] = v[j] > 0.0f ? thmm_logf_normal(bits, 0) : NegInf<float>();
+    rare = rare || (v[j] > 0.0f && bits - 0x00800000u >= 0x7f000000u);
+  }
+  if (rare) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      out[j] = PotentialLog(v[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    v[j] = out[j];
+}
+__device__ __forceinline__ void PotentialLogs(double (&v)[4]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    v[j] = PotentialLog(v[j]);
+}
+
+// sum + exp(x[0]) + ... + exp(x[3]), in that order, for x <= 0 (or NaN, which
+// the short form passes on).
+__device__ __forceinline__ float AddExps(float sum, const float (&x)[4]) {
+  float e[4];
+  if (fminf(fminf(x[0], x[1]), fminf(x[2], x[3])) >= -87.0f) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      e[j] = thmm_expf_short(x[j]);
+  } else {
+    // Zero factors: -inf. Between -104 and -87 the general function.
+    bool rare = false;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      e[j] = x[j] < -103.972084f ? 0.0f : thmm_expf_short(x[j]);
+      rare = rare || (x[j] < -87.0f && !(x[j] < -103.972084f));
+    }
+    if (rare) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        e[j] = thmm_expf(x[j]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    sum = sum + e[j];
+  return sum;
+}
+__device__ __forceinline__ double AddExps(double sum, const double (&x)[4]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    sum = sum + thmm_exp(x[j]);
+  return sum;
+}
+
+// LogSumExp (src/inference.cc:100-110) over terms[0..K), -inf from K on (which
+// changes neither the maximum nor, adding zeros, the sum).
+template <typename T, int KMAX>
+__device__ __forceinline__ T PaddedLogSumExp(const T (&terms)[KMAX], unsigned K) {
+  T maximum = NegInf<T>();
+#pragma unroll
+  for (unsigned j = 0; j < KMAX; ++j)
+    maximum = sizeof(T) == 4 ? static_cast<T>(fmaxf(maximum, terms[j])) // NaN: ignored too
+                             : maximum < terms[j] ? terms[j] : maximum;
+  if (!isfinite(maximum))
+    return maximum;
+  T sum = T(0);
+#pragma unroll
+  for (unsigned q = 0; q < KMAX; q += 4) {
+    if (q < K) {
+      const T x[4] = {terms[q] - maximum, terms[q + 1] - maximum, terms[q + 2] - maximum,
+                      terms[q + 3] - maximum};
+      sum = AddExps(sum, x);
+    }
+  }
+  return maximum + PortableLog(sum);
+}
+
 template <typename T, int KMAX, bool kSample> struct LogPhaseOps {
   static constexpr int G = GroupLanes<KMAX>();
   static constexpr int ROWS = (KMAX + G - 1) / G; // rows per lane: KMAX or 1
@@ -89,15 +175,11 @@ template <typename T, int KMAX, bool kSample> struct LogPhaseOps {
     return root ? root_potential[j] * emitted : emitted;
   }
 
-  // Log value of a node (every lane the whole vector).
+  // Log value of a node (every lane the whole vector, -inf past K).
   __device__ __forceinline__ void NodeVector(std::uint32_t ref, std::uint32_t obs, bool root,
                                              T (&out)[KMAX]) const {
-    if (ref & kFlag) {
-      Row(static_cast<const T *>(a.nodes) + Store(ref & kMask) * K, out);
-    } else if constexpr (G == 1) {
-#pragma unroll
-      for (unsigned j = 0; j < KMAX; ++j)
-        out[j] = j < K ? PotentialLog(InputElement(ref, obs, root, j)) : NegInf<T>();
+    if (G == 1 || (ref & kFlag)) {
+      NodeVectorAlone(ref, obs, root, out);
     } else {
       const T own =
           lane < K ? PotentialLog(InputElement(ref, obs, root, lane)) : NegInf<T>();
@@ -110,17 +192,18 @@ template <typename T, int KMAX, bool kSample> struct LogPhaseOps {
   __device__ __forceinline__ void NodeVectorAlone(std::uint32_t ref, std::uint32_t obs,
                                                   bool root, T (&out)[KMAX]) const {
     if (ref & kFlag) {
-      Row(static_cast<const T *>(a.nodes) + Store(ref & kMask) * K, out);
+      Row(static_cast<const T *>(a.nodes) + Store(ref & kMask) * K, NegInf<T>(), out);
     } else {
 #pragma unroll
       for (unsigned j = 0; j < KMAX; ++j)
-        out[j] = j < K ? PotentialLog(InputElement(ref, obs, root, j)) : NegInf<T>();
+        out[j] = j < K ? InputElement(ref, obs, root, j) : T(0);
+      Logs(out);
     }
   }
 
-  // K values from p (zero-padded), in 16-byte loads where every row starts on
+  // K values from p, `pad` past K, in 16-byte loads where every row starts on
   // a 16-byte boundary.
-  __device__ __forceinline__ void Row(const T *p, T (&out)[KMAX]) const {
+  __device__ __forceinline__ void Row(const T *p, T pad, T (&out)[KMAX]) const {
     constexpr unsigned kPer = 16 / sizeof(T);
     if (K % kPer == 0) {
 #pragma unroll
@@ -135,31 +218,53 @@ template <typename T, int KMAX, bool kSample> struct LogPhaseOps {
         } else {
 #pragma unroll
           for (unsigned j = 0; j < kPer; ++j)
-            out[q * kPer + j] = T(0);
+            out[q * kPer + j] = pad;
         }
       }
     } else {
 #pragma unroll
       for (unsigned j = 0; j < KMAX; ++j)
-        out[j] = j < K ? p[j] : T(0);
+        out[j] = j < K ? p[j] : pad;
     }
   }
+  // Logarithms in place (of factors, 0 past K: -inf there).
+  __device__ __forceinline__ void Logs(T (&v)[KMAX]) const {
+#pragma unroll
+    for (unsigned q = 0; q < KMAX; q += 4) {
+      if (q < K) {
+        T four[4] = {v[q], v[q + 1], v[q + 2], v[q + 3]};
+        PotentialLogs(four);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          v[q + j] = four[j];
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          v[q + j] = NegInf<T>();
+      }
+    }
+  }
+  // Log row r of a path, -inf past K.
   __device__ __forceinline__ void PathRow(std::uint32_t ref, unsigned r, T (&out)[KMAX]) const {
     if (ref & kFlag) {
-      Row(static_cast<const T *>(a.comps) + Store(ref & kMask) * KK + r * K, out);
+      Row(static_cast<const T *>(a.comps) + Store(ref & kMask) * KK + r * K, NegInf<T>(), out);
     } else {
-      Row(static_cast<const T *>(a.edge_in) + static_cast<std::size_t>(ref) * KK + r * K, out);
-#pragma unroll
-      for (unsigned j = 0; j < KMAX; ++j)
-        if (j < K)
-          out[j] = PotentialLog(out[j]);
+      Row(static_cast<const T *>(a.edge_in) + static_cast<std::size_t>(ref) * KK + r * K, T(0),
+          out);
+      Logs(out);
     }
   }
-  __device__ __forceinline__ T PathElement(std::uint32_t ref, unsigned i, unsigned j) const {
-    return (ref & kFlag)
-               ? static_cast<const T *>(a.comps)[Store(ref & kMask) * KK + i * K + j]
-               : PotentialLog(static_cast<const T *>(
-                     a.edge_in)[static_cast<std::size_t>(ref) * KK + i * K + j]);
+  // Log column j of a path, -inf past K.
+  __device__ __forceinline__ void PathColumn(std::uint32_t ref, unsigned j,
+                                             T (&out)[KMAX]) const {
+    const bool stored = (ref & kFlag) != 0;
+    const T *p = stored ? static_cast<const T *>(a.comps) + Store(ref & kMask) * KK
+                        : static_cast<const T *>(a.edge_in) + static_cast<std::size_t>(ref) * KK;
+#pragma unroll
+    for (unsigned m = 0; m < KMAX; ++m)
+      out[m] = m < K ? p[m * K + j] : stored ? NegInf<T>() : T(0);
+    if (!stored)
+      Logs(out);
   }
 
   // ---------------------------------------------------------- forward
@@ -172,18 +277,16 @@ template <typename T, int KMAX, bool kSample> struct LogPhaseOps {
 #pragma unroll
       for (unsigned j = 0; j < KMAX; ++j)
         row[j] = row[j] + leaf[j];
-      return LogSumExp<T, KMAX>(row, K);
+      return PaddedLogSumExp<T, KMAX>(row, K);
     } else {
       T best = row[0] + leaf[0];
       unsigned choice = 0;
 #pragma unroll
-      for (unsigned j = 1; j < KMAX; ++j) {
-        if (j < K) {
-          const T term = row[j] + leaf[j];
-          if (term > best) {
-            best = term;
-            choice = j;
-          }
+      for (unsigned j = 1; j < KMAX; ++j) { // terms past K are -inf and never win
+        const T term = row[j] + leaf[j];
+        if (term > best) {
+          best = term;
+          choice = j;
         }
       }
       a.rake_choices[Store(rake) * K + r] = static_cast<std::uint8_t>(choice);
@@ -292,9 +395,15 @@ template <typename T, int KMAX, bool kSample> struct LogPhaseOps {
           PathRow(op.z, m, rights[m]);
     } else {
       __syncwarp(mask); // the group's previous operation is done with the tile
-      if (lane < K) {
+      if (lane < KMAX) {
         T right[KMAX];
-        PathRow(op.z, lane, right);
+        if (lane < K) {
+          PathRow(op.z, lane, right);
+        } else {
+#pragma unroll
+          for (unsigned j = 0; j < KMAX; ++j)
+            right[j] = NegInf<T>();
+        }
 #pragma unroll
         for (unsigned j = 0; j < KMAX; ++j)
           tile[kSample ? j * KMAX + lane : lane * KMAX + j] = right[j];
@@ -321,8 +430,8 @@ template <typename T, int KMAX, bool kSample> struct LogPhaseOps {
               T terms[KMAX];
 #pragma unroll
               for (unsigned m = 0; m < KMAX; ++m)
-                terms[m] = m < K ? head[m] + rights[m][j] : T(0);
-              out[j] = LogSumExp<T, KMAX>(terms, K);
+                terms[m] = m < K ? head[m] + rights[m][j] : NegInf<T>();
+              out[j] = PaddedLogSumExp<T, KMAX>(terms, K);
             }
           }
           StoreRow<KMAX>(dst, K, out);
@@ -332,7 +441,7 @@ template <typename T, int KMAX, bool kSample> struct LogPhaseOps {
 #pragma unroll
             for (unsigned m = 0; m < KMAX; ++m)
               terms[m] = head[m] + tile[j * KMAX + m];
-            dst[j] = LogSumExp<T, KMAX>(terms, K);
+            dst[j] = PaddedLogSumExp<T, KMAX>(terms, K);
           }
         }
       } else {
@@ -410,14 +519,14 @@ template <typename T, int KMAX, bool kSample> struct LogPhaseOps {
     unsigned choice = 0;
     T result;
     if constexpr (kSample) {
-      result = LogSumExp<T, KMAX>(terms, K);
+      result = PaddedLogSumExp<T, KMAX>(terms, K);
       if (isfinite(result))
         choice = Draw(terms, result, node);
     } else {
       result = terms[0];
 #pragma unroll
       for (unsigned j = 1; j < KMAX; ++j) {
-        if (j < K && terms[j] > result) {
+        if (terms[j] > result) {
           result = terms[j];
           choice = j;
         }
@@ -441,7 +550,7 @@ template <typename T, int KMAX, bool kSample> struct LogPhaseOps {
 #pragma unroll
       for (unsigned j = 0; j < KMAX; ++j)
         terms[j] = terms[j] + leaf[j];
-      const T normalizer = LogSumExp<T, KMAX>(terms, K);
+      const T normalizer = PaddedLogSumExp<T, KMAX>(terms, K);
       a.states_out[Io(leaf_node)] = Draw(terms, normalizer, leaf_node);
     } else {
       a.states_out[Io(leaf_node)] = a.rake_choices[Store(i) * K + parent_state];
@@ -454,13 +563,14 @@ template <typename T, int KMAX, bool kSample> struct LogPhaseOps {
     const unsigned parent_state = a.states_out[Io(end.x)];
     const unsigned child_state = a.states_out[Io(end.y)];
     if constexpr (kSample) {
-      T middle[KMAX], terms[KMAX];
+      T middle[KMAX], terms[KMAX], right[KMAX];
       NodeVectorAlone(op.y, op.w, false, middle);
       PathRow(op.x, parent_state, terms);
+      PathColumn(op.z, child_state, right);
 #pragma unroll
       for (unsigned m = 0; m < KMAX; ++m)
-        terms[m] = m < K ? terms[m] + middle[m] + PathElement(op.z, m, child_state) : T(0);
-      const T normalizer = LogSumExp<T, KMAX>(terms, K);
+        terms[m] = terms[m] + middle[m] + right[m];
+      const T normalizer = PaddedLogSumExp<T, KMAX>(terms, K);
       a.states_out[Io(middle_node)] = Draw(terms, normalizer, middle_node);
     } else {
       a.states_out[Io(middle_node)] =

@@ -107,8 +107,52 @@ THMM_MATH_FN double thmm_u2d(uint64_t bits) {
 #define THMM_LN2_LO 1.9082149292705877000220372080672226e-10
 #define THMM_LOG2E 1.4426950408889634073599246810018921
 
+/* f / b, correctly rounded, for b = 2 + f and f as thmm_logf_normal forms them.
+ * On the device: the approximate reciprocal y and one correction of q = f y by
+ * its residual (Markstein's method), q + (f - q b) y. That this rounds
+ * correctly depends on f: all 2^23 values of it were compared with the division
+ * (tests/test_gpu_portable_math.py does it again), and no other f reaches it.
+ * The general division checks the range of its operands first, which cost
+ * about a quarter of a logarithm. */
+THMM_MATH_FN float thmm_log_quotient(float f, float b) {
+#if defined(__CUDA_ARCH__)
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+  const float q = __fmul_rn(f, y);
+  return __fmaf_rn(__fmaf_rn(-q, b, f), y, q);
+#else
+  return f / b;
+#endif
+}
+
+/* log(u2f(bits) * 2^scale) for the bits of a normal positive float. Taking the
+ * bits of sqrt(1/2) (0x3f3504f4) off leaves the exponent of the fold into
+ * [sqrt(1/2), sqrt(2)) in the upper bits. */
+THMM_MATH_FN float thmm_logf_normal(uint32_t bits, int scale) {
+  const uint32_t fold = bits - 0x3f3504f4u;
+  const int e = ((int)fold >> 23) + scale;
+  const float m = thmm_u2f(bits - (fold & 0xff800000u));
+  const float f = THMM_SUBF(m, 1.0f);
+  const float s = thmm_log_quotient(f, THMM_ADDF(2.0f, f));
+  const float z = THMM_MULF(s, s);
+  /* R = z (2/3 + z (2/5 + z (2/7 + z 2/9))) */
+  float r = THMM_FMAF(z, 0.222222222f, 0.285714286f);
+  r = THMM_FMAF(z, r, 0.4f);
+  r = THMM_FMAF(z, r, 0.666666667f);
+  r = THMM_MULF(z, r);
+  const float half_f2 = THMM_MULF(THMM_MULF(0.5f, f), f);
+  /* e as a float without a conversion: 2^23 + 2^22 + e, less 2^23 + 2^22. */
+  const float ef = THMM_SUBF(thmm_u2f(0x4b400000u + (uint32_t)e), 12582912.0f);
+  /* log = e ln2_hi + (f - (half_f2 - (s (half_f2 + R) + e ln2_lo))) */
+  const float tail = THMM_FMAF(s, THMM_ADDF(half_f2, r), THMM_MULF(ef, THMM_LN2_LO_F));
+  const float body = THMM_SUBF(f, THMM_SUBF(half_f2, tail));
+  return THMM_FMAF(ef, THMM_LN2_HI_F, body);
+}
+
 THMM_MATH_FN float thmm_logf(float x) {
   const uint32_t bits = thmm_f2u(x);
+  if (bits - 0x00800000u < 0x7f000000u) /* normal and positive */
+    return thmm_logf_normal(bits, 0);
   if (x != x)
     return x;
   if (x < 0.0f)
@@ -117,36 +161,7 @@ THMM_MATH_FN float thmm_logf(float x) {
     return thmm_u2f(0xff800000u);
   if (bits == 0x7f800000u)
     return x;
-  int exponent_bias = 0;
-  uint32_t b = bits;
-  if (b < 0x00800000u) { /* subnormal: scale by 2^25 exactly */
-    b = thmm_f2u(THMM_MULF(x, 33554432.0f));
-    exponent_bias = -25;
-  }
-  int e = (int)((b >> 23) & 0xffu) - 127 + exponent_bias;
-  uint32_t mantissa = b & 0x007fffffu;
-  /* m in [1, 2); fold m > sqrt(2) into [sqrt(1/2), 1). */
-  if (mantissa > 0x003504f3u) {
-    mantissa |= 0x3f000000u; /* m / 2 */
-    e += 1;
-  } else {
-    mantissa |= 0x3f800000u;
-  }
-  const float m = thmm_u2f(mantissa);
-  const float f = THMM_SUBF(m, 1.0f);
-  const float s = THMM_DIVF(f, THMM_ADDF(2.0f, f));
-  const float z = THMM_MULF(s, s);
-  /* R = z (2/3 + z (2/5 + z (2/7 + z 2/9))) */
-  float r = THMM_FMAF(z, 0.222222222f, 0.285714286f);
-  r = THMM_FMAF(z, r, 0.4f);
-  r = THMM_FMAF(z, r, 0.666666667f);
-  r = THMM_MULF(z, r);
-  const float half_f2 = THMM_MULF(THMM_MULF(0.5f, f), f);
-  const float ef = (float)e;
-  /* log = e ln2_hi + (f - (half_f2 - (s (half_f2 + R) + e ln2_lo))) */
-  const float tail = THMM_FMAF(s, THMM_ADDF(half_f2, r), THMM_MULF(ef, THMM_LN2_LO_F));
-  const float body = THMM_SUBF(f, THMM_SUBF(half_f2, tail));
-  return THMM_FMAF(ef, THMM_LN2_HI_F, body);
+  return thmm_logf_normal(thmm_f2u(THMM_MULF(x, 33554432.0f)), -25); /* subnormal */
 }
 
 THMM_MATH_FN float thmm_expf(float x) {
@@ -178,6 +193,34 @@ THMM_MATH_FN float thmm_expf(float x) {
   /* n < -126: scale by 2^(n + 64) then by 2^-64. */
   return THMM_MULF(THMM_MULF(p, thmm_u2f((uint32_t)(n + 64 + 127) << 23)),
                    thmm_u2f((uint32_t)(-64 + 127) << 23));
+}
+
+/* thmm_expf, value for value, for the arguments of a log-sum-exp (x <= 0, or
+ * NaN), which come in by the millions. There n = ceil(x / ln 2 - 1/2); adding
+ * 2^23 + 2^22 rounded upwards leaves it in the low bits of the sum, with no
+ * conversions (a quarter of the multiply-add rate or less on the device). Below
+ * -87 the result may be subnormal: the general function. */
+THMM_MATH_FN float thmm_expf_short(float x) { /* -87 <= x <= 0 */
+  const float t = THMM_SUBF(THMM_MULF(x, THMM_LOG2E_F), 0.5f);
+#if defined(__CUDA_ARCH__)
+  const float shifted = __fadd_ru(t, 12582912.0f);
+#else
+  const float shifted = ceilf(t) + 12582912.0f;
+#endif
+  const float nf = THMM_SUBF(shifted, 12582912.0f);
+  float r = THMM_FMAF(-nf, THMM_LN2_HI_F, x);
+  r = THMM_FMAF(-nf, THMM_LN2_LO_F, r);
+  float p = THMM_FMAF(r, 1.98412698e-04f, 1.38888889e-03f);
+  p = THMM_FMAF(r, p, 8.33333333e-03f);
+  p = THMM_FMAF(r, p, 4.16666667e-02f);
+  p = THMM_FMAF(r, p, 1.66666667e-01f);
+  p = THMM_FMAF(r, p, 0.5f);
+  p = THMM_MULF(THMM_MULF(r, r), p);
+  p = THMM_ADDF(1.0f, THMM_ADDF(r, p));
+  return THMM_MULF(p, thmm_u2f((thmm_f2u(shifted) << 23) + 0x3f800000u));
+}
+THMM_MATH_FN float thmm_expf_nonpositive(float x) {
+  return x <= 0.0f && x >= -87.0f ? thmm_expf_short(x) : thmm_expf(x);
 }
 
 THMM_MATH_FN double thmm_log(double x) {
