@@ -26,14 +26,16 @@ cudaError_t LaunchKind(const PhaseArgs &args, cudaStream_t stream, int *blocks_p
   } else if (args.batch) {
     return cudaErrorInvalidValue; // no tail in the shared-topology layout
   }
-  auto kernel = PhaseKernel<Scalar, Compute, kKind>;
+  // One thread per operation, or one warp or block per tree for the tails.
+  const bool block_tail = kTail && args.count < kTailBlockTrees;
+  auto kernel = block_tail ? PhaseKernel<Scalar, Compute, kKind, kTail ? kPhaseThreads : 1>
+                           : PhaseKernel<Scalar, Compute, kKind, kTail ? 32 : 1>;
   if (blocks_per_sm != nullptr)
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kernel,
                                                          kPhaseThreads, 0);
   if (args.count == 0)
     return cudaSuccess;
-  // One thread per operation, or one warp per tree for the tail kinds.
-  const unsigned per_block = kTail ? kPhaseThreads / 32 : kPhaseThreads;
+  const unsigned per_block = block_tail ? 1u : kTail ? kPhaseThreads / 32 : kPhaseThreads;
   const unsigned grid = (args.count + per_block - 1) / per_block;
   kernel<<<grid, kPhaseThreads, 0, stream>>>(args);
   return cudaGetLastError();

@@ -64,15 +64,74 @@ struct BatchIndex {
   }
 };
 
-template <typename Scalar, typename Compute, class Index> struct PhaseOps {
+// Shared memory of a block for the matrix stores below: one 4 x 4 matrix per
+// thread at a pitch of 20 floats, whose 16-byte rows fall on different banks.
+constexpr int kMatrixPitch = 20;
+constexpr int kMatrixTile = 32 * kMatrixPitch; // one warp
+
+// kWarpStores: every lane of a warp runs an operation (some perhaps not live),
+// and the lanes store their matrices together (single-precision K = 4).
+template <typename Scalar, typename Compute, class Index, bool kWarpStores = false>
+struct PhaseOps {
   static constexpr int KMAX = 4;
   const PhaseArgs &a;
   Index ix;
   unsigned K;
   unsigned KK;
+  bool live;
+  float *tile; // this warp's kMatrixTile floats
 
-  __device__ PhaseOps(const PhaseArgs &args, const Index &index)
-      : a(args), ix(index), K(args.states), KK(args.states * args.states) {}
+  __device__ PhaseOps(const PhaseArgs &args, const Index &index, bool is_live = true,
+                      float *warp_tile = nullptr)
+      : a(args), ix(index), K(args.states), KK(args.states * args.states), live(is_live),
+        tile(warp_tile) {}
+
+  // A matrix leaves row by row: BeginMatrix, PutRow for every row, EndMatrix.
+  // A thread's own four 16-byte stores would each write half a sector in 32
+  // places; through shared memory, four lanes write a matrix as two whole
+  // sectors.
+  __device__ __forceinline__ bool Together() const {
+    return kWarpStores && sizeof(Scalar) == 4 && sizeof(Compute) == 4 && K == KMAX;
+  }
+  __device__ __forceinline__ void BeginMatrix() const {
+    if (Together())
+      __syncwarp(); // the tile's last matrices have left
+  }
+  template <bool kStreaming, typename D>
+  __device__ __forceinline__ void PutRow(D *dst, unsigned q, const Compute (&row)[KMAX]) const {
+    if (Together())
+      StoreRow<KMAX>(tile + (threadIdx.x & 31u) * kMatrixPitch + 4 * q, K, row);
+    else if (live && q < K) {
+      if constexpr (kStreaming)
+        StoreRowStreaming<KMAX>(dst + q * K, K, row);
+      else
+        StoreRow<KMAX>(dst + q * K, K, row);
+    }
+  }
+  // `dst`: where this lane's matrix goes; bit 0 of the address passed around
+  // asks for streaming (evict-first) stores.
+  __device__ __forceinline__ void EndMatrix(void *dst, bool streaming) const {
+    if (!Together())
+      return;
+    const unsigned lane = threadIdx.x & 31u;
+    __syncwarp();
+    const unsigned long long own =
+        live ? reinterpret_cast<unsigned long long>(dst) | (streaming ? 1ull : 0ull) : 0ull;
+#pragma unroll
+    for (unsigned s = 0; s < 4; ++s) {
+      const unsigned from = 8 * s + lane / 4, row = lane % 4;
+      const unsigned long long to = __shfl_sync(kFull, own, from);
+      if (to != 0) {
+        const float4 v =
+            *reinterpret_cast<const float4 *>(tile + from * kMatrixPitch + 4 * row);
+        float4 *p = reinterpret_cast<float4 *>(to & ~1ull) + row;
+        if (to & 1ull)
+          __stcs(p, v);
+        else
+          *p = v;
+      }
+    }
+  }
 
   // Input factor vector of `node`: dense row, or the reference's categorical
   // (root ? root_potential : 1) * emission[observation]
@@ -236,16 +295,17 @@ template <typename Scalar, typename Compute, class Index> struct PhaseOps {
     const int s = Exponent(m);
     const std::size_t at = ix.Comp(i);
     Compute *dst = static_cast<Compute *>(a.comps) + at * KK;
+    BeginMatrix();
 #pragma unroll
     for (int q = 0; q < KMAX; ++q) {
-      if (q < static_cast<int>(K)) {
 #pragma unroll
-        for (unsigned j = 0; j < KMAX; ++j)
-          out[q][j] = ScalePow2(out[q][j], -s);
-        StoreRow<KMAX>(dst + q * K, K, out[q]);
-      }
+      for (unsigned j = 0; j < KMAX; ++j)
+        out[q][j] = ScalePow2(out[q][j], -s);
+      PutRow<false>(dst, q, out[q]);
     }
-    a.comp_exp[at] = e + s;
+    EndMatrix(dst, false);
+    if (live)
+      a.comp_exp[at] = e + s;
   }
 
   // log Z = ln 2 * (root exponent) + log(sum(root)), as LinearEngine::Run.
@@ -284,14 +344,24 @@ template <typename Scalar, typename Compute, class Index> struct PhaseOps {
   }
 
   // ---------------------------------------------------------- adjoint
-  __device__ __forceinline__ void StorePathAdjoint(std::uint32_t ref, unsigned r,
-                                                   const Compute (&row)[KMAX]) const {
+  // The adjoint of path `ref`, row by row as above.
+  __device__ __forceinline__ Compute *MuAt(std::uint32_t ref) const {
+    return static_cast<Compute *>(a.comp_mu) + ix.Comp(ref & kMask) * KK;
+  }
+  __device__ __forceinline__ Scalar *EdgeOutAt(std::uint32_t ref) const {
+    return static_cast<Scalar *>(a.edge_out) + ix.Out(ref) * KK;
+  }
+  __device__ __forceinline__ void PutAdjointRow(std::uint32_t ref, unsigned q,
+                                                const Compute (&row)[KMAX]) const {
     if (ref & kFlag)
-      StoreRow<KMAX>(static_cast<Compute *>(a.comp_mu) + ix.Comp(ref & kMask) * KK + r * K, K,
-                     row);
+      PutRow<false>(MuAt(ref), q, row);
     else
-      StoreRowStreaming<KMAX>(static_cast<Scalar *>(a.edge_out) + ix.Out(ref) * KK + r * K, K,
-                              row);
+      PutRow<true>(EdgeOutAt(ref), q, row);
+  }
+  __device__ __forceinline__ void EndAdjoint(std::uint32_t ref) const {
+    const bool stored = (ref & kFlag) != 0;
+    EndMatrix(stored ? static_cast<void *>(MuAt(ref)) : static_cast<void *>(EdgeOutAt(ref)),
+              !stored);
   }
 
   __device__ __forceinline__ void RakeReverse(std::uint32_t i) const {
@@ -304,6 +374,7 @@ template <typename Scalar, typename Compute, class Index> struct PhaseOps {
     LoadRow<KMAX>(node_out + ix.Io(op.w) * K, K, parent_adjoint);
     Compute ratio[KMAX];
     Compute rows[KMAX][KMAX];
+    BeginMatrix();
 #pragma unroll
     for (int q = 0; q < KMAX; ++q) {
       PathRow(op.x, q, rows[q]);
@@ -312,14 +383,13 @@ template <typename Scalar, typename Compute, class Index> struct PhaseOps {
       for (unsigned j = 0; j < KMAX; ++j)
         unnormalised = fma(rows[q][j], leaf[j], unnormalised);
       ratio[q] = unnormalised > Compute(0) ? parent_adjoint[q] / unnormalised : Compute(0);
-      if (q < static_cast<int>(K)) {
-        Compute w[KMAX];
+      Compute w[KMAX];
 #pragma unroll
-        for (unsigned j = 0; j < KMAX; ++j)
-          w[j] = ratio[q] * rows[q][j] * leaf[j];
-        StorePathAdjoint(op.x, q, w);
-      }
+      for (unsigned j = 0; j < KMAX; ++j)
+        w[j] = ratio[q] * rows[q][j] * leaf[j];
+      PutAdjointRow(op.x, q, w);
     }
+    EndAdjoint(op.x);
     Compute adjoint[KMAX];
 #pragma unroll
     for (unsigned j = 0; j < KMAX; ++j) {
@@ -329,7 +399,8 @@ template <typename Scalar, typename Compute, class Index> struct PhaseOps {
         column = fma(ratio[p], rows[p][j], column);
       adjoint[j] = leaf[j] * column;
     }
-    StoreRow<KMAX>(node_out + ix.Io(op.y & kMask) * K, K, adjoint);
+    if (live)
+      StoreRow<KMAX>(node_out + ix.Io(op.y & kMask) * K, K, adjoint);
   }
 
   __device__ __forceinline__ void CompressReverse(std::uint32_t i) const {
@@ -379,6 +450,7 @@ template <typename Scalar, typename Compute, class Index> struct PhaseOps {
 #pragma unroll
     for (unsigned mid = 0; mid < KMAX; ++mid)
       PathRow(op.z, mid, rights[mid]);
+    BeginMatrix();
 #pragma unroll
     for (int q = 0; q < KMAX; ++q) {
       Compute left_adjoint[KMAX];
@@ -393,9 +465,10 @@ template <typename Scalar, typename Compute, class Index> struct PhaseOps {
           left_adjoint[mid] = left[q][mid] * middle[mid] * dot;
         }
       }
-      if (q < static_cast<int>(K))
-        StorePathAdjoint(op.x, q, left_adjoint);
+      PutAdjointRow(op.x, q, left_adjoint);
     }
+    EndAdjoint(op.x);
+    BeginMatrix();
     Compute middle_adjoint[KMAX];
 #pragma unroll
     for (unsigned mid = 0; mid < KMAX; ++mid) {
@@ -411,17 +484,23 @@ template <typename Scalar, typename Compute, class Index> struct PhaseOps {
         total += right_adjoint[j];
       }
       middle_adjoint[mid] = total;
-      if (mid < K)
-        StorePathAdjoint(op.z, mid, right_adjoint);
+      PutAdjointRow(op.z, mid, right_adjoint);
     }
-    StoreRow<KMAX>(static_cast<Scalar *>(a.node_out) + ix.Io(op.y & kMask) * K, K,
-                   middle_adjoint);
+    EndAdjoint(op.z);
+    if (live)
+      StoreRow<KMAX>(static_cast<Scalar *>(a.node_out) + ix.Io(op.y & kMask) * K, K,
+                     middle_adjoint);
   }
 };
 
-// Tail rounds of one tree per warp (kPhaseTailForward / kPhaseTailReverse):
-// the lanes take the operations of a step in turn, with a warp barrier
-// (which also orders the lanes' global-memory accesses) between steps.
+// Tail rounds of one tree per team of kTeam threads (kPhaseTailForward /
+// kPhaseTailReverse): a warp or a block, whose threads take the operations of
+// a step in turn, with a barrier (which also orders their global-memory
+// accesses) between steps. With many trees a warp each fills the chip; below
+// kTailBlockTrees a block each does, and a step of a large tree takes a
+// quarter of the passes.
+constexpr std::uint32_t kTailBlockTrees = 1024;
+
 // Starts moving `count` 16-byte records from `p` into L2 (a hint).
 __device__ __forceinline__ void PrefetchRecords(const void *p, std::uint32_t count) {
   if (count != 0)
@@ -429,14 +508,20 @@ __device__ __forceinline__ void PrefetchRecords(const void *p, std::uint32_t cou
                  : "memory");
 }
 
-template <typename Scalar, typename Compute, bool kReverse>
+template <typename Scalar, typename Compute, bool kReverse, int kTeam>
 __device__ __forceinline__ void TailTree(const PhaseOps<Scalar, Compute, ForestIndex> &ops,
                                          const PhaseArgs &a, std::uint32_t item) {
-  const unsigned lane = threadIdx.x & 31u;
+  const unsigned lane = threadIdx.x % kTeam;
+  const auto sync = [] {
+    if constexpr (kTeam == 32)
+      __syncwarp();
+    else
+      __syncthreads();
+  };
   const uint4 tree = a.tail_items[item];
   // The walk below is a chain of dependent loads per round; first bring
   // every tail round's records of this tree into L2 (lane e: round e).
-  for (std::uint32_t e = lane; e < tree.z; e += 32) {
+  for (std::uint32_t e = lane; e < tree.z; e += kTeam) {
     const uint4 round = a.tail_rounds[tree.y + e];
     const uint2 rakes = a.tail_rakes[tree.y + e];
     PrefetchRecords(a.gathers + round.x, round.y);
@@ -447,28 +532,37 @@ __device__ __forceinline__ void TailTree(const PhaseOps<Scalar, Compute, ForestI
     const std::uint32_t at = tree.y + (kReverse ? tree.z - 1 - e : e);
     const uint4 round = a.tail_rounds[at];
     if constexpr (!kReverse) {
-      for (std::uint32_t i = lane; i < round.y; i += 32)
+      for (std::uint32_t i = lane; i < round.y; i += kTeam)
         ops.Gather(round.x + i);
-      __syncwarp();
-      for (std::uint32_t i = lane; i < round.w; i += 32)
+      sync();
+      for (std::uint32_t i = lane; i < round.w; i += kTeam)
         ops.Compress(round.z + i);
-      __syncwarp();
+      sync();
     } else {
-      for (std::uint32_t i = lane; i < round.w; i += 32)
+      for (std::uint32_t i = lane; i < round.w; i += kTeam)
         ops.CompressReverse(round.z + i);
-      __syncwarp();
+      sync();
       const uint2 rakes = a.tail_rakes[at];
-      for (std::uint32_t i = lane; i < rakes.y; i += 32)
+      for (std::uint32_t i = lane; i < rakes.y; i += kTeam)
         ops.RakeReverse(rakes.x + i);
-      __syncwarp();
+      sync();
     }
   }
 }
 
+// Kinds that store matrices: whole warps run them.
+template <int kKind>
+inline constexpr bool kStoresMatrices =
+    kKind == kPhaseCompress || kKind == kPhaseRakeReverse || kKind == kPhaseCompressReverse;
+
 template <typename Scalar, typename Compute, class Index, int kKind>
 __device__ __forceinline__ void RunOp(const PhaseArgs &args, const Index &index,
-                                      std::uint32_t i, std::uint32_t value) {
-  const PhaseOps<Scalar, Compute, Index> ops(args, index);
+                                      std::uint32_t i, std::uint32_t value, bool live) {
+  constexpr bool kTogether =
+      kStoresMatrices<kKind> && sizeof(Scalar) == 4 && sizeof(Compute) == 4;
+  __shared__ __align__(16) float tiles[kTogether ? kPhaseThreads / 32 * kMatrixTile : 1];
+  const PhaseOps<Scalar, Compute, Index, kTogether> ops(
+      args, index, live, kTogether ? tiles + threadIdx.x / 32 * kMatrixTile : nullptr);
   if constexpr (kKind == kPhaseGather)
     ops.Gather(i);
   else if constexpr (kKind == kPhaseCompress)
@@ -482,21 +576,22 @@ __device__ __forceinline__ void RunOp(const PhaseArgs &args, const Index &index,
 }
 
 // Forest layout: thread t runs operation offset + t (finish: instance), or
-// warp w the tail of tree offset + w.
-template <typename Scalar, typename Compute, int kKind>
+// team w of kTeam threads the tail of tree offset + w.
+template <typename Scalar, typename Compute, int kKind, int kTeam = 1>
 __global__ void __launch_bounds__(kPhaseThreads) PhaseKernel(PhaseArgs args) {
   if constexpr (kKind == kPhaseTailForward || kKind == kPhaseTailReverse) {
-    const std::uint32_t w = blockIdx.x * (kPhaseThreads / 32) + threadIdx.x / 32;
+    const std::uint32_t w = blockIdx.x * (kPhaseThreads / kTeam) + threadIdx.x / kTeam;
     if (w >= args.count)
       return;
     const PhaseOps<Scalar, Compute, ForestIndex> ops(args, ForestIndex{});
-    TailTree<Scalar, Compute, kKind == kPhaseTailReverse>(ops, args, args.offset + w);
+    TailTree<Scalar, Compute, kKind == kPhaseTailReverse, kTeam>(ops, args, args.offset + w);
   } else {
     const std::uint32_t t = blockIdx.x * kPhaseThreads + threadIdx.x;
-    if (t >= args.count)
+    if ((kStoresMatrices<kKind> ? t & ~31u : t) >= args.count)
       return;
-    const std::uint32_t i = args.offset + t;
-    RunOp<Scalar, Compute, ForestIndex, kKind>(args, ForestIndex{}, i, i);
+    const bool live = t < args.count; // a lane past the end repeats the last operation
+    const std::uint32_t i = args.offset + (live ? t : args.count - 1);
+    RunOp<Scalar, Compute, ForestIndex, kKind>(args, ForestIndex{}, i, i, live);
   }
 }
 
@@ -504,16 +599,20 @@ __global__ void __launch_bounds__(kPhaseThreads) PhaseKernel(PhaseArgs args) {
 // batch item first_item + t % items (finish: the root record for that item).
 template <typename Scalar, typename Compute, int kKind>
 __global__ void __launch_bounds__(kPhaseThreads) BatchPhaseKernel(PhaseArgs args) {
-  const std::uint64_t t = static_cast<std::uint64_t>(blockIdx.x) * kPhaseThreads + threadIdx.x;
-  if (t >= static_cast<std::uint64_t>(args.count) * args.items)
+  // Below 2^31 in all (the record index limit).
+  const std::uint32_t total = args.count * args.items;
+  std::uint32_t t = blockIdx.x * kPhaseThreads + threadIdx.x;
+  if ((kStoresMatrices<kKind> ? t & ~31u : t) >= total)
     return;
+  const bool live = t < total;
+  t = live ? t : total - 1;
   BatchIndex index;
-  index.item = args.first_item + static_cast<std::uint32_t>(t % args.items);
+  index.item = args.first_item + t % args.items;
   index.stride = args.item_stride;
   index.nodes = args.item_nodes;
   index.edges = args.item_edges;
-  const std::uint32_t i = args.offset + static_cast<std::uint32_t>(t / args.items);
-  RunOp<Scalar, Compute, BatchIndex, kKind>(args, index, i, index.item);
+  const std::uint32_t i = args.offset + t / args.items;
+  RunOp<Scalar, Compute, BatchIndex, kKind>(args, index, i, index.item, live);
 }
 
 } // namespace thmm

@@ -798,13 +798,16 @@ struct Workspace {
   }
 
   // Rounds of the phase schedule run grid-wide (0: the first round with
-  // fewer than 2^17 gathers and compressions); uploads the tail records of
-  // the rest. A tail of more than 2^20 trees stays grid-wide, and so do the
+  // fewer than 2^17 gathers and compressions, or 256 a tree where that is
+  // less: two passes of a block); uploads the tail records of the rest. A tail of more than 2^20 trees stays grid-wide, and so do the
   // batch layout (every item has every round) and every state count above 4.
+  std::uint32_t AutomaticRounds() const {
+    return phase.AutoTailRound(std::min<std::uint64_t>(1u << 17, 256 * capacity));
+  }
   void SetPhaseRounds(std::uint32_t rounds) {
     if (!phase.enabled)
       return;
-    std::uint32_t wanted = rounds != 0 ? rounds : phase.AutoTailRound(1u << 17);
+    std::uint32_t wanted = rounds != 0 ? rounds : AutomaticRounds();
     wanted = std::max<std::uint32_t>(wanted, 1);
     if (phase_batch || states > 4)
       wanted = phase.rounds; // no tail kinds above 4 states
@@ -1208,7 +1211,7 @@ struct Workspace {
     if (LinearPhases() && !IsLogDomain(operation)) {
       schedule = THMM_SCHEDULE_PHASES;
       std::vector<std::uint32_t> tried_rounds;
-      const std::uint32_t automatic = phase.AutoTailRound(1u << 17);
+      const std::uint32_t automatic = AutomaticRounds();
       for (std::uint32_t rounds : {automatic, 1u, 2u, 3u, 4u, 5u, 6u, 8u, phase.rounds}) {
         SetPhaseRounds(rounds);
         if (std::find(tried_rounds.begin(), tried_rounds.end(), phase_rounds) !=
