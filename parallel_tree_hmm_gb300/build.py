@@ -55,6 +55,7 @@ SOURCES = [
     "engine_wide.cu",
     "engine_phase.cu",
     "engine_wide_phase.cu",
+    "engine_wide_stream.cu",
     "engine_phase_groups_32_f64.cu",
     "engine_phase_groups_32_f32.cu",
     "engine_phase_groups_28_f32.cu",

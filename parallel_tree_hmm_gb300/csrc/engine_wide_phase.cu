@@ -52,12 +52,16 @@ cudaError_t LaunchWideTyped(int kind, const PhaseArgs &args, cudaStream_t stream
   case kPhaseGather:
     return LaunchWideKind<KP, kPhaseGather>(args, stream, blocks_per_sm);
   case kPhaseCompress:
+    if (args.states % 4 == 0)
+      return LaunchWideStream(kind, args, stream, blocks_per_sm);
     return LaunchWideKind<KP, kPhaseCompress>(args, stream, blocks_per_sm);
   case kPhaseFinish:
     return LaunchWideKind<KP, kPhaseFinish>(args, stream, blocks_per_sm);
   case kPhaseRakeReverse:
     return LaunchWideKind<KP, kPhaseRakeReverse>(args, stream, blocks_per_sm);
   case kPhaseCompressReverse:
+    if (args.states % 4 == 0)
+      return LaunchWideStream(kind, args, stream, blocks_per_sm);
     return LaunchWideKind<KP, kPhaseCompressReverse>(args, stream, blocks_per_sm);
   default:
     return cudaErrorInvalidValue; // no tail kinds: every round runs grid-wide

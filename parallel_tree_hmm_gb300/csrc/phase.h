@@ -193,6 +193,9 @@ cudaError_t LaunchPhase(int scalar_bytes, bool compute_f64, int kind, const Phas
                         cudaStream_t stream, int *blocks_per_sm);
 cudaError_t LaunchWidePhase(int kind, const PhaseArgs &args, cudaStream_t stream,
                             int *blocks_per_sm);
+// The compress kinds of K a multiple of 4 among those (wide_stream.cuh).
+cudaError_t LaunchWideStream(int kind, const PhaseArgs &args, cudaStream_t stream,
+                             int *blocks_per_sm);
 // 4 < K <= 32: one lane group per operation (phase_groups.cuh), per padded
 // state count and arithmetic type.
 #define THMM_GROUP_PHASE_LAUNCHER(name)                                                    \

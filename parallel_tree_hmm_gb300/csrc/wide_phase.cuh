@@ -350,11 +350,10 @@ __device__ __forceinline__ void StageChunk(const XS &x, const YS &y, unsigned K,
 }
 
 // Issues the tensor-core steps of depth chunk `chunk` of a product whose
-// operands are staged (hi/lo, or BF16 in the hi parts) and waits for them
-// (bounded). Returns false if the wait timed out.
+// operands are staged (hi/lo, or BF16 in the hi parts), after a CTA barrier.
 template <int KP, bool kSplit>
-__device__ bool MmaChunk(unsigned char *smem, PhaseShared &sh, std::uint32_t &phase,
-                         std::uint32_t tmem, unsigned chunk, bool bf16) {
+__device__ __forceinline__ void IssueChunk(unsigned char *smem, PhaseShared &sh,
+                                           std::uint32_t tmem, unsigned chunk, bool bf16) {
   using L = PhaseLayout<KP>;
   umma::FenceOperands();
   umma::FenceBeforeSync();
@@ -395,10 +394,21 @@ __device__ bool MmaChunk(unsigned char *smem, PhaseShared &sh, std::uint32_t &ph
     }
     umma::Commit(&sh.barrier);
   }
+}
+
+// Waits (bounded) for the chunk issued last. Returns false on a time-out.
+__device__ __forceinline__ bool WaitChunk(PhaseShared &sh, std::uint32_t &phase) {
   const bool ok = umma::Wait(&sh.barrier, phase);
   phase ^= 1u;
   umma::FenceAfterSync();
   return ok;
+}
+
+template <int KP, bool kSplit>
+__device__ bool MmaChunk(unsigned char *smem, PhaseShared &sh, std::uint32_t &phase,
+                         std::uint32_t tmem, unsigned chunk, bool bf16) {
+  IssueChunk<KP, kSplit>(smem, sh, tmem, chunk, bf16);
+  return WaitChunk(sh, phase);
 }
 
 // Tensor-memory lanes 0..127 (one per thread), columns from `tmem`:
