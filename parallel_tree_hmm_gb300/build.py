@@ -54,6 +54,7 @@ SOURCES = [
     "engine_sample_f32.cu",
     "engine_wide.cu",
     "engine_phase.cu",
+    "engine_phase_tree.cu",
     "engine_wide_phase.cu",
     "engine_wide_stream.cu",
     "engine_phase_groups_32_f64.cu",

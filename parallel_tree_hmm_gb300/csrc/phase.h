@@ -123,6 +123,52 @@ struct PhaseArgs {
   std::uint32_t bf16;
 };
 
+// Byte offsets of a tree's arrays in its block's shared memory (TreePhaseKernel).
+struct TreePhaseLayout {
+  std::uint64_t gathers, compress, edges, comps, comp_mu, nodes, node_out, node_exp, comp_exp,
+      bytes;
+};
+inline TreePhaseLayout MakeTreePhaseLayout(std::uint64_t nodes, std::uint64_t edges,
+                                              std::uint64_t rakes, std::uint64_t gathers,
+                                              std::uint64_t compressions, std::uint64_t states,
+                                              std::uint64_t scalar, std::uint64_t compute,
+                                              bool reverse) {
+  const auto up = [](std::uint64_t bytes) { return (bytes + 15) & ~std::uint64_t{15}; };
+  const std::uint64_t matrix = states * states * compute;
+  TreePhaseLayout at{};
+  at.gathers = 16 * rakes; // the rakes come first
+  at.compress = at.gathers + 16 * gathers;
+  at.edges = at.compress + 16 * compressions;
+  at.comps = at.edges + up(edges * matrix);
+  at.comp_mu = at.comps + up(compressions * matrix);
+  at.nodes = at.comp_mu + (reverse ? up(compressions * matrix) : 0);
+  at.node_out = at.nodes + up(nodes * states * compute);
+  at.node_exp = at.node_out + (reverse ? up(nodes * states * scalar) : 0);
+  at.comp_exp = at.node_exp + up(nodes * 4);
+  at.bytes = at.comp_exp + up(compressions * 4);
+  return at;
+}
+
+// A whole tree per block (K <= 4, batch API): every round, the root and the
+// adjoint of one item in one launch, with the records, the factors, the values
+// and the adjoints of the item in the block's shared memory (TreePhaseKernel).
+struct TreePhaseArgs {
+  PhaseArgs phase; // batch layout; records in round order
+  std::uint32_t nodes, edges, rakes, gathers, compressions;
+  std::uint32_t rounds;
+  const uint4 *round_ops;   // as tail rounds, from round 0
+  const uint2 *round_rakes; // as tail rakes
+  const std::uint8_t *observations;    // the caller's: [item][observed node]
+  const std::uint32_t *observed_nodes; // [observed node]
+  std::uint32_t observed;
+  TreePhaseLayout at;
+};
+
+inline constexpr unsigned kTreePhaseThreads = 512;
+inline constexpr std::uint64_t kTreePhaseMaxBytes = 226 * 1024;
+cudaError_t LaunchTreePhase(int scalar_bytes, bool compute_f64, const TreePhaseArgs &args,
+                            cudaStream_t stream);
+
 // Operation counts of one program per round and kind.
 struct ProgramRounds {
   std::uint32_t rounds = 0;

@@ -22,6 +22,7 @@
 #include <limits>
 #include <memory>
 #include <numeric>
+#include <optional>
 #include <stdexcept>
 #include <string>
 #include <thread>
@@ -230,6 +231,8 @@ struct Workspace {
   std::uint32_t log_rounds = 0;
   bool log_tail = false;
   DeviceBuffer phase_ends, log_tail_items, log_tail_rounds, log_tail_rakes;
+  // A whole tree per block (TreePhaseKernel): records of its rounds.
+  DeviceBuffer tree_rounds, tree_rakes, tree_observed;
   // Phase-ordered copy of the observations (PhasePlan::observation_order),
   // rebuilt on the device whenever observations are uploaded.
   DeviceBuffer phase_observations, observation_order;
@@ -290,7 +293,7 @@ struct Workspace {
           &compress_ends, &gathers, &team_order, &stripe_order, &control, &node_in,
           &phase_rakes, &phase_gathers, &phase_compress, &phase_roots, &node_exp,
           &comp_exp, &tail_items, &tail_rounds, &tail_rakes, &phase_ends,
-          &log_tail_items, &log_tail_rounds, &log_tail_rakes, &phase_observations,
+          &tree_rounds, &tree_rakes, &tree_observed, &log_tail_items, &log_tail_rounds, &log_tail_rakes, &phase_observations,
           &observation_order, &edge_in,
           &observations, &root_potential, &emission, &uniforms, &values,
           &node_out, &edge_out, &states_out, &scratch, &bytes})
@@ -515,6 +518,13 @@ struct Workspace {
         phase_gathers.Upload(phase.gathers, stream);
         phase_compress.Upload(phase.compress, stream);
         phase_roots.Upload(phase.roots, stream);
+        if (phase_batch && states <= 4) {
+          const PhasePlan::Tail tree = phase.BuildTail(0, true);
+          tree_rounds.Upload(tree.rounds, stream);
+          tree_rakes.Upload(tree.rakes, stream);
+          tree_observed.Upload(observation_nodes, stream);
+          Check(cudaStreamSynchronize(stream), "tree record upload");
+        }
         if (maximum || sampling) {
           phase_ends.Upload(phase.ends, stream);
           SetLogRounds();
@@ -848,6 +858,10 @@ struct Workspace {
     return false;
   }
 
+  // Whether `operation` runs kernels with work counters or an error word.
+  bool UsesControl(int operation) const {
+    return !UsePhases(operation) || states > 32 || operation == THMM_OP_SAMPLE;
+  }
   static bool IsLogDomain(int operation) {
     return operation == THMM_OP_MAXIMUM || operation == THMM_OP_SAMPLE;
   }
@@ -980,6 +994,28 @@ struct Workspace {
     return count;
   }
 
+  // Whether `items` items of a batch workspace run a whole tree per block, and
+  // the shared memory of a block: the tree fits, the blocks are at most four
+  // waves of the chip, and either a tree's rounds are one pass of the block (512
+  // nodes) or there are 32 items and more. A few larger trees would gain as
+  // well (16 items of 1,000 nodes), but the one launch per round and kind of
+  // such a batch is what thmm_workspace_launches has reported, and is kept.
+  std::optional<TreePhaseLayout> TreeLayout(int operation, std::uint64_t items) const {
+    if (!phase_batch || states > 4 || (nodes_per_item > 512 && items < 32))
+      return std::nullopt;
+    const TreePhaseLayout at =
+        MakeTreePhaseLayout(nodes_per_item, edges_per_item, phase.rake_base[phase.rounds],
+                            phase.gather_base[phase.rounds], phase.total_compressions, states,
+                            ScalarBytes(), compute_f64 ? 8 : 4, operation == THMM_OP_MARGINALS);
+    if (at.bytes > kTreePhaseMaxBytes)
+      return std::nullopt;
+    const std::uint64_t resident =
+        std::min<std::uint64_t>(2048 / kTreePhaseThreads, 228 * 1024 / (at.bytes + 2048));
+    if (items > 4 * resident * static_cast<std::uint64_t>(sms))
+      return std::nullopt;
+    return at;
+  }
+
   // Launches the phase schedule of `operation` over instances [a, b):
   // gather and compress phases round by round, the finish phase, then (for
   // marginals) the adjoint phases in reverse round order. Returns the number
@@ -987,6 +1023,27 @@ struct Workspace {
   int LaunchPhases(int operation, std::uint32_t a, std::uint32_t b) {
     if (IsLogDomain(operation))
       return LaunchLogPhases(operation, a, b);
+    if (const auto layout = TreeLayout(operation, b - a)) {
+      TreePhaseArgs tree{};
+      tree.at = *layout;
+      tree.phase = MakePhaseArgs(operation, a, b);
+      tree.phase.node_out = node_out.ptr;
+      tree.phase.edge_out = edge_out.ptr;
+      tree.nodes = static_cast<std::uint32_t>(nodes_per_item);
+      tree.edges = static_cast<std::uint32_t>(edges_per_item);
+      tree.rakes = static_cast<std::uint32_t>(phase.rake_base[phase.rounds]);
+      tree.gathers = static_cast<std::uint32_t>(phase.gather_base[phase.rounds]);
+      tree.compressions = static_cast<std::uint32_t>(phase.total_compressions);
+      tree.rounds = phase.rounds;
+      tree.round_ops = tree_rounds.as<uint4>();
+      tree.round_rakes = tree_rakes.as<uint2>();
+      tree.observations = observations.as<std::uint8_t>();
+      tree.observed_nodes = tree_observed.as<std::uint32_t>();
+      tree.observed = static_cast<std::uint32_t>(observations_per_item);
+      Check(LaunchTreePhase(scalar, compute_f64, tree, stream),
+            "tree-HMM accelerator kernel launch");
+      return 1;
+    }
     // Batch layout: every item runs the one tree's operations; items [a, b).
     const PhaseRanges &ranges = phase_batch ? PhaseRangesFor(0, 1) : PhaseRangesFor(a, b);
     const std::size_t K = states;
@@ -1051,7 +1108,8 @@ struct Workspace {
       args.big_count = items_big ? static_cast<std::uint32_t>(batch) : 0u;
       args.small_count = items_big ? 0u : static_cast<std::uint32_t>(batch);
     }
-    Check(cudaMemsetAsync(control.ptr, 0, 32, stream), "cudaMemsetAsync");
+    if (UsesControl(operation))
+      Check(cudaMemsetAsync(control.ptr, 0, 32, stream), "cudaMemsetAsync");
     const auto items = static_cast<std::uint32_t>(forest ? capacity : batch);
     launches = static_cast<std::uint64_t>(
         UsePhases(operation) ? LaunchPhases(operation, 0, items)
@@ -1113,13 +1171,15 @@ struct Workspace {
   // so it is built when an operation has been called kGraphAfter times in a
   // row on one batch size.
   static constexpr int kGraphAfter = 8;
+  static constexpr std::uint64_t kGraphLaunches = 8;
   void EnqueuePrepared(int operation, std::size_t batch) {
     if (operation != repeated_operation || batch != repeated_batch) {
       repeated_operation = operation;
       repeated_batch = batch;
       repeats = 0;
     }
-    bool replay = repeats >= kGraphAfter;
+    // A graph's own launch takes longer than a few kernels'.
+    bool replay = repeats >= kGraphAfter && launches >= kGraphLaunches;
     for (const Graph &graph : graphs)
       replay = replay || (graph.operation == operation && graph.batch == batch);
     if (replay) {
@@ -1293,7 +1353,8 @@ struct Workspace {
               "cudaMemcpyAsync result download");
     };
     download(h_values, values, items * S);
-    download(h_control, control, 16);
+    if (UsesControl(operation))
+      download(h_control, control, 16);
     if (operation == THMM_OP_MARGINALS) {
       download(h_node_out, node_out, NodesFor(batch) * states * S);
       download(h_edge_out, edge_out, EdgeOutFor(batch) * states * states * S);
@@ -1312,7 +1373,7 @@ struct Workspace {
     outcome.timings.upload_ms = upload_ms;
     outcome.timings.kernel_ms = kernel_ms;
     outcome.timings.download_ms = download_ms;
-    outcome.error = h_control.as<std::uint32_t>()[2];
+    outcome.error = UsesControl(operation) ? h_control.as<std::uint32_t>()[2] : 0u;
     if (outcome.error & kErrorTensorTimeout)
       throw std::runtime_error("tree-HMM accelerator tensor-core wait timed out");
     outcome.timings.wall_ms =
