@@ -8,8 +8,11 @@ namespace {
 template <int KP, bool kReverse>
 cudaError_t LaunchStreamKind(const PhaseArgs &args, cudaStream_t stream, int *blocks_per_sm) {
   using S = wide::StreamLayout<KP, kReverse>;
-  auto kernel = args.bf16 ? wide::WideStreamKernel<KP, kReverse, true>
-                          : wide::WideStreamKernel<KP, kReverse, false>;
+  const bool exact = args.states == KP;
+  auto kernel = args.bf16 ? (exact ? wide::WideStreamKernel<KP, kReverse, true, true>
+                                   : wide::WideStreamKernel<KP, kReverse, true, false>)
+                          : (exact ? wide::WideStreamKernel<KP, kReverse, false, true>
+                                   : wide::WideStreamKernel<KP, kReverse, false, false>);
   cudaError_t status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             static_cast<int>(S::kBytes));
   if (status == cudaSuccess)

@@ -27,8 +27,8 @@
 // products. All loads of a stage are issued before its stores, with no branch
 // between them.
 // Measured on one GB300: marginals of 64 path-heavy trees x 2000 nodes, K = 64,
-// 6.82 -> 4.78 ms; 64 x 500 nodes, K = 128, 9.13 -> 5.24 ms (DRAM at 3.0 to 3.4
-// TB/s in the large launches, the tensor pipe 16 to 19 % busy). What is left is
+// 6.82 -> 4.52 ms; 64 x 500 nodes, K = 128, 9.13 -> 5.17 ms (DRAM at 3.0 to 3.7
+// TB/s in the large launches, the tensor pipe 17 to 21 % busy). What is left is
 // latency: two CTAs (one at K_P = 128) take turns at barriers, products and
 // tensor-memory reads.
 #ifndef THMM_WIDE_STREAM_CUH_
@@ -63,7 +63,8 @@ template <int KP, bool kReverse> struct StreamLayout {
                 "TMEM columns");
 };
 
-template <int KP, bool kReverse, bool kBf16> struct StreamOps {
+// kExact: K == KP, so that the compiler folds the bounds and the strides.
+template <int KP, bool kReverse, bool kBf16, bool kExact> struct StreamOps {
   using L = PhaseLayout<KP>;
   using S = StreamLayout<KP, kReverse>;
   static constexpr unsigned T = S::kThreads, kWarps = T / 32;
@@ -96,7 +97,7 @@ template <int KP, bool kReverse, bool kBf16> struct StreamOps {
   __device__ StreamOps(const PhaseArgs &args, PhaseShared &shared, unsigned char *dynamic_smem,
                        std::uint32_t tmem_base, std::uint32_t &mma_phase, bool &status)
       : a(args), sh(shared), smem(dynamic_smem), tmem(tmem_base), phase(mma_phase), ok(status),
-        K(args.states), KK(args.states * args.states), warp(threadIdx.x / 32),
+        K(kExact ? KP : args.states), KK(K * K), warp(threadIdx.x / 32),
         lane(threadIdx.x & 31u) {}
 
   __device__ __forceinline__ const float *PathPtr(std::uint32_t ref) const {
@@ -556,7 +557,7 @@ template <int KP, bool kReverse, bool kBf16> struct StreamOps {
 
 // The compress kinds for K a multiple of 4: a persistent grid, CTA b taking
 // operations b, b + grid, ...
-template <int KP, bool kReverse, bool kBf16>
+template <int KP, bool kReverse, bool kBf16, bool kExact>
 __global__ void __launch_bounds__(PhaseLayout<KP>::kThreads,
                                   StreamLayout<KP, kReverse>::kResident)
     WideStreamKernel(PhaseArgs args) {
@@ -574,7 +575,7 @@ __global__ void __launch_bounds__(PhaseLayout<KP>::kThreads,
   __syncthreads();
   umma::FenceAfterSync();
   {
-    const StreamOps<KP, kReverse, kBf16> ops(args, sh, stream_smem, sh.tmem, phase, ok);
+    const StreamOps<KP, kReverse, kBf16, kExact> ops(args, sh, stream_smem, sh.tmem, phase, ok);
     if (blockIdx.x < args.count)
       ops.Run(blockIdx.x, gridDim.x);
   }
