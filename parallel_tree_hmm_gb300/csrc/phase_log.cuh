@@ -585,13 +585,25 @@ template <typename T, int KMAX, bool kSample> struct LogPhaseOps {
 // record and one edge matrix of a batch together. The tail kind runs the
 // last rounds, the root and the last rounds' top-down steps of one tree per
 // CTA, with a CTA barrier between steps.
-template <typename T, int KMAX, bool kSample, int kKind>
-__global__ void __launch_bounds__(kLogPhaseThreads, KMAX <= 8 && sizeof(T) == 4 ? 4 : 2)
+// A tail block's passes over a step are dependent trips to memory, so where
+// every block has an SM of its own it gets as many threads as the registers
+// allow: 48 uneven trees, MAP at K = 8, 278 us a call with 128 threads, 256 us
+// with 512; 320 trees 1.30 ms with 128, 1.34 ms with 512.
+template <typename T, int KMAX>
+inline constexpr int kLogTailThreads = sizeof(T) == 4 && KMAX <= 8    ? 512
+                                       : sizeof(T) == 4 && KMAX <= 20 ? 256
+                                                                      : kLogPhaseThreads;
+constexpr std::uint64_t kLogTailBlocks = 152; // SMs
+
+template <typename T, int KMAX, bool kSample, int kKind, int kThreads>
+__global__ void __launch_bounds__(kThreads, kThreads > kLogPhaseThreads      ? 1
+                                            : KMAX <= 8 && sizeof(T) == 4 ? 4
+                                                                          : 2)
     LogPhaseKernel(PhaseArgs args) {
   using Ops = LogPhaseOps<T, KMAX, kSample>;
   constexpr int G = Ops::G;
   constexpr bool kTile = G > 1 && (kKind == kPhaseCompress || kKind == kPhaseTailForward);
-  __shared__ __align__(16) T tiles[kTile ? (kLogPhaseThreads / G) * kLogTile<KMAX> : 1];
+  __shared__ __align__(16) T tiles[kTile ? (kThreads / G) * kLogTile<KMAX> : 1];
   T *tile = kTile ? tiles + threadIdx.x / G * kLogTile<KMAX> : nullptr;
   if constexpr (kKind == kPhaseTailForward) {
     const uint4 tree = args.tail_items[args.batch ? 0u : args.offset + blockIdx.x];
@@ -600,11 +612,11 @@ __global__ void __launch_bounds__(kLogPhaseThreads, KMAX <= 8 && sizeof(T) == 4 
     const unsigned group = threadIdx.x / G;
     for (std::uint32_t e = 0; e < tree.z; ++e) {
       const uint4 round = args.tail_rounds[tree.y + e];
-      for (std::uint32_t i = group; i < round.y; i += kLogPhaseThreads / G)
+      for (std::uint32_t i = group; i < round.y; i += kThreads / G)
         ops.Gather(round.x + i);
       __syncthreads();
       if (round.w != 0) {
-        for (std::uint32_t i = group; i < round.w; i += kLogPhaseThreads / G)
+        for (std::uint32_t i = group; i < round.w; i += kThreads / G)
           ops.Compress(round.z + i);
         __syncthreads();
       }
@@ -615,12 +627,12 @@ __global__ void __launch_bounds__(kLogPhaseThreads, KMAX <= 8 && sizeof(T) == 4 
     for (std::uint32_t e = tree.z; e-- > 0;) {
       const uint4 round = args.tail_rounds[tree.y + e];
       if (round.w != 0) {
-        for (std::uint32_t i = threadIdx.x; i < round.w; i += kLogPhaseThreads)
+        for (std::uint32_t i = threadIdx.x; i < round.w; i += kThreads)
           ops.ExpandCompress(round.z + i);
         __syncthreads();
       }
       const uint2 rakes = args.tail_rakes[tree.y + e];
-      for (std::uint32_t i = threadIdx.x; i < rakes.y; i += kLogPhaseThreads)
+      for (std::uint32_t i = threadIdx.x; i < rakes.y; i += kThreads)
         ops.ExpandRake(rakes.x + i);
       __syncthreads();
     }
@@ -628,8 +640,8 @@ __global__ void __launch_bounds__(kLogPhaseThreads, KMAX <= 8 && sizeof(T) == 4 
     constexpr bool kGroups = kKind == kPhaseGather || kKind == kPhaseCompress;
     const std::uint32_t t =
         kGroups ? static_cast<std::uint32_t>(
-                      (static_cast<std::uint64_t>(blockIdx.x) * kLogPhaseThreads + threadIdx.x) / G)
-                : blockIdx.x * kLogPhaseThreads + threadIdx.x;
+                      (static_cast<std::uint64_t>(blockIdx.x) * kThreads + threadIdx.x) / G)
+                : blockIdx.x * kThreads + threadIdx.x;
     if (t >= args.count * args.items) // below 2^31 (the record index limit)
       return;
     std::uint32_t op = t, item = 0;
@@ -667,7 +679,15 @@ cudaError_t LaunchLogKind(const PhaseArgs &args, cudaStream_t stream) {
     return cudaSuccess;
   if (grid > 0x7fffffffull)
     return cudaErrorInvalidConfiguration;
-  LogPhaseKernel<T, KMAX, kSample, kKind>
+  if constexpr (kKind == kPhaseTailForward) {
+    constexpr int kWide = kLogTailThreads<T, KMAX>;
+    if (grid <= kLogTailBlocks) {
+      LogPhaseKernel<T, KMAX, kSample, kKind, kWide>
+          <<<static_cast<unsigned>(grid), kWide, 0, stream>>>(args);
+      return cudaGetLastError();
+    }
+  }
+  LogPhaseKernel<T, KMAX, kSample, kKind, kLogPhaseThreads>
       <<<static_cast<unsigned>(grid), kLogPhaseThreads, 0, stream>>>(args);
   return cudaGetLastError();
 }
