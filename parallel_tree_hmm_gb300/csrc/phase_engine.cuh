@@ -108,15 +108,15 @@ struct PhaseOps {
         StoreRow<KMAX>(dst + q * K, K, row);
     }
   }
-  // `dst`: where this lane's matrix goes; bit 0 of the address passed around
-  // asks for streaming (evict-first) stores.
-  __device__ __forceinline__ void EndMatrix(void *dst, bool streaming) const {
+  // `dst`: where this lane's matrix goes. Ordinary stores: evicted first, the
+  // marginals of 4,096 sites left L2 before their neighbours came (622 against
+  // 610 us a step).
+  __device__ __forceinline__ void EndMatrix(void *dst) const {
     if (!Together())
       return;
     const unsigned lane = threadIdx.x & 31u;
     __syncwarp();
-    const unsigned long long own =
-        live ? reinterpret_cast<unsigned long long>(dst) | (streaming ? 1ull : 0ull) : 0ull;
+    const unsigned long long own = live ? reinterpret_cast<unsigned long long>(dst) : 0ull;
 #pragma unroll
     for (unsigned s = 0; s < 4; ++s) {
       const unsigned from = 8 * s + lane / 4, row = lane % 4;
@@ -124,11 +124,7 @@ struct PhaseOps {
       if (to != 0) {
         const float4 v =
             *reinterpret_cast<const float4 *>(tile + from * kMatrixPitch + 4 * row);
-        float4 *p = reinterpret_cast<float4 *>(to & ~1ull) + row;
-        if (to & 1ull)
-          __stcs(p, v);
-        else
-          *p = v;
+        reinterpret_cast<float4 *>(to)[row] = v;
       }
     }
   }
@@ -206,6 +202,29 @@ struct PhaseOps {
   __device__ __forceinline__ static int Exponent(Compute m) {
     return m > Compute(0) ? Pow2Exponent(m) : 0;
   }
+  // FP64 arithmetic is bound by its pipe (a warp instruction every 14 cycles
+  // per SM), so it skips the terms past K; FP32 runs them, which is cheaper
+  // than the tests.
+  __device__ __forceinline__ bool Counts(unsigned j) const {
+    return sizeof(Compute) == 4 || j < K;
+  }
+  // Exponent of the largest of v (0 where none is positive), without FP64
+  // comparisons where that one is a normal number.
+  template <int N> __device__ __forceinline__ static int MaxExponent(const Compute (&v)[N]) {
+    if constexpr (sizeof(Compute) == 8) {
+      int hi = 0;
+#pragma unroll
+      for (int j = 0; j < N; ++j)
+        hi = max(hi, __double2hiint(v[j]));
+      if (hi >= 0x00100000 && hi < 0x7ff00000)
+        return (hi >> 20) - 1022;
+    }
+    Compute m = Compute(0);
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      m = m < v[j] ? v[j] : m;
+    return Exponent(m);
+  }
 
   // ---------------------------------------------------------- forward
   __device__ __forceinline__ void Gather(std::uint32_t i) const {
@@ -228,7 +247,6 @@ struct PhaseOps {
       Node(rake.y, rake.z, leaf, e);
       e += PathExp(rake.x);
       Compute message[KMAX];
-      Compute m = Compute(0);
 #pragma unroll
       for (int q = 0; q < KMAX; ++q) {
         Compute row[KMAX];
@@ -236,23 +254,22 @@ struct PhaseOps {
         Compute dot = Compute(0);
 #pragma unroll
         for (unsigned j = 0; j < KMAX; ++j)
-          dot = fma(row[j], leaf[j], dot);
+          if (Counts(q) && Counts(j))
+            dot = fma(row[j], leaf[j], dot);
         message[q] = dot;
-        m = m < dot ? dot : m;
       }
-      int s = Exponent(m);
-      e += s;
-      m = Compute(0);
-#pragma unroll
-      for (int q = 0; q < KMAX; ++q) {
-        v[q] = v[q] * ScalePow2(message[q], -s);
-        m = m < v[q] ? v[q] : m;
-      }
-      s = Exponent(m);
+      int s = MaxExponent(message);
       e += s;
 #pragma unroll
       for (int q = 0; q < KMAX; ++q)
-        v[q] = ScalePow2(v[q], -s);
+        if (Counts(q))
+          v[q] = v[q] * ScalePow2(message[q], -s);
+      s = MaxExponent(v);
+      e += s;
+#pragma unroll
+      for (int q = 0; q < KMAX; ++q)
+        if (Counts(q))
+          v[q] = ScalePow2(v[q], -s);
     }
     StoreRow<KMAX>(dst, K, v);
     a.node_exp[at] = e;
@@ -279,20 +296,17 @@ struct PhaseOps {
         PathRow(op.z, mid, right);
 #pragma unroll
         for (int q = 0; q < KMAX; ++q) {
-          const Compute weight = left[q][mid] * middle[mid];
+          if (Counts(q)) {
+            const Compute weight = left[q][mid] * middle[mid];
 #pragma unroll
-          for (unsigned j = 0; j < KMAX; ++j)
-            out[q][j] = fma(weight, right[j], out[q][j]);
+            for (unsigned j = 0; j < KMAX; ++j)
+              if (Counts(j))
+                out[q][j] = fma(weight, right[j], out[q][j]);
+          }
         }
       }
     }
-    Compute m = Compute(0);
-#pragma unroll
-    for (int q = 0; q < KMAX; ++q)
-#pragma unroll
-      for (unsigned j = 0; j < KMAX; ++j)
-        m = m < out[q][j] ? out[q][j] : m;
-    const int s = Exponent(m);
+    const int s = MaxExponent(reinterpret_cast<const Compute(&)[KMAX * KMAX]>(out));
     const std::size_t at = ix.Comp(i);
     Compute *dst = static_cast<Compute *>(a.comps) + at * KK;
     BeginMatrix();
@@ -300,10 +314,11 @@ struct PhaseOps {
     for (int q = 0; q < KMAX; ++q) {
 #pragma unroll
       for (unsigned j = 0; j < KMAX; ++j)
-        out[q][j] = ScalePow2(out[q][j], -s);
+        if (Counts(q) && Counts(j))
+          out[q][j] = ScalePow2(out[q][j], -s);
       PutRow<false>(dst, q, out[q]);
     }
-    EndMatrix(dst, false);
+    EndMatrix(dst);
     if (live)
       a.comp_exp[at] = e + s;
   }
@@ -360,8 +375,7 @@ struct PhaseOps {
   }
   __device__ __forceinline__ void EndAdjoint(std::uint32_t ref) const {
     const bool stored = (ref & kFlag) != 0;
-    EndMatrix(stored ? static_cast<void *>(MuAt(ref)) : static_cast<void *>(EdgeOutAt(ref)),
-              !stored);
+    EndMatrix(stored ? static_cast<void *>(MuAt(ref)) : static_cast<void *>(EdgeOutAt(ref)));
   }
 
   __device__ __forceinline__ void RakeReverse(std::uint32_t i) const {
@@ -379,25 +393,33 @@ struct PhaseOps {
     for (int q = 0; q < KMAX; ++q) {
       PathRow(op.x, q, rows[q]);
       Compute unnormalised = Compute(0);
+      Compute w[KMAX] = {};
+      ratio[q] = Compute(0);
+      if (Counts(q)) {
 #pragma unroll
-      for (unsigned j = 0; j < KMAX; ++j)
-        unnormalised = fma(rows[q][j], leaf[j], unnormalised);
-      ratio[q] = unnormalised > Compute(0) ? parent_adjoint[q] / unnormalised : Compute(0);
-      Compute w[KMAX];
+        for (unsigned j = 0; j < KMAX; ++j)
+          if (Counts(j))
+            unnormalised = fma(rows[q][j], leaf[j], unnormalised);
+        ratio[q] = unnormalised > Compute(0) ? parent_adjoint[q] / unnormalised : Compute(0);
 #pragma unroll
-      for (unsigned j = 0; j < KMAX; ++j)
-        w[j] = ratio[q] * rows[q][j] * leaf[j];
+        for (unsigned j = 0; j < KMAX; ++j)
+          if (Counts(j))
+            w[j] = ratio[q] * rows[q][j] * leaf[j];
+      }
       PutAdjointRow(op.x, q, w);
     }
     EndAdjoint(op.x);
-    Compute adjoint[KMAX];
+    Compute adjoint[KMAX] = {};
 #pragma unroll
     for (unsigned j = 0; j < KMAX; ++j) {
-      Compute column = Compute(0);
+      if (Counts(j)) {
+        Compute column = Compute(0);
 #pragma unroll
-      for (int p = 0; p < KMAX; ++p)
-        column = fma(ratio[p], rows[p][j], column);
-      adjoint[j] = leaf[j] * column;
+        for (int p = 0; p < KMAX; ++p)
+          if (Counts(p))
+            column = fma(ratio[p], rows[p][j], column);
+        adjoint[j] = leaf[j] * column;
+      }
     }
     if (live)
       StoreRow<KMAX>(node_out + ix.Io(op.y & kMask) * K, K, adjoint);
@@ -425,10 +447,13 @@ struct PhaseOps {
         PathRow(op.z, mid, right);
 #pragma unroll
         for (int q = 0; q < KMAX; ++q) {
-          const Compute weight = left[q][mid] * middle[mid];
+          if (Counts(q)) {
+            const Compute weight = left[q][mid] * middle[mid];
 #pragma unroll
-          for (unsigned j = 0; j < KMAX; ++j)
-            ratio[q][j] = fma(weight, right[j], ratio[q][j]);
+            for (unsigned j = 0; j < KMAX; ++j)
+              if (Counts(j))
+                ratio[q][j] = fma(weight, right[j], ratio[q][j]);
+          }
         }
       }
     }
@@ -444,7 +469,9 @@ struct PhaseOps {
       }
 #pragma unroll
       for (unsigned j = 0; j < KMAX; ++j)
-        ratio[q][j] = ratio[q][j] > Compute(0) ? adjoint[j] / ratio[q][j] : Compute(0);
+        ratio[q][j] = Counts(q) && Counts(j) && ratio[q][j] > Compute(0)
+                          ? adjoint[j] / ratio[q][j]
+                          : Compute(0);
     }
     Compute rights[KMAX][KMAX];
 #pragma unroll
@@ -457,11 +484,12 @@ struct PhaseOps {
 #pragma unroll
       for (unsigned mid = 0; mid < KMAX; ++mid) {
         left_adjoint[mid] = Compute(0);
-        if (mid < K) {
+        if (mid < K && Counts(q)) {
           Compute dot = Compute(0);
 #pragma unroll
           for (unsigned j = 0; j < KMAX; ++j)
-            dot = fma(rights[mid][j], ratio[q][j], dot);
+            if (Counts(j))
+              dot = fma(rights[mid][j], ratio[q][j], dot);
           left_adjoint[mid] = left[q][mid] * middle[mid] * dot;
         }
       }
@@ -472,16 +500,19 @@ struct PhaseOps {
     Compute middle_adjoint[KMAX];
 #pragma unroll
     for (unsigned mid = 0; mid < KMAX; ++mid) {
-      Compute right_adjoint[KMAX];
+      Compute right_adjoint[KMAX] = {};
       Compute total = Compute(0);
 #pragma unroll
       for (unsigned j = 0; j < KMAX; ++j) {
-        Compute acc = Compute(0);
+        if (Counts(mid) && Counts(j)) {
+          Compute acc = Compute(0);
 #pragma unroll
-        for (int p = 0; p < KMAX; ++p)
-          acc = fma(left[p][mid], ratio[p][j], acc);
-        right_adjoint[j] = rights[mid][j] * middle[mid] * acc;
-        total += right_adjoint[j];
+          for (int p = 0; p < KMAX; ++p)
+            if (Counts(p))
+              acc = fma(left[p][mid], ratio[p][j], acc);
+          right_adjoint[j] = rights[mid][j] * middle[mid] * acc;
+          total += right_adjoint[j];
+        }
       }
       middle_adjoint[mid] = total;
       PutAdjointRow(op.z, mid, right_adjoint);
@@ -575,10 +606,18 @@ __device__ __forceinline__ void RunOp(const PhaseArgs &args, const Index &index,
     ops.CompressReverse(i);
 }
 
+// Minimum resident blocks per SM (a register cap) of the kind that would
+// otherwise take a few registers too many for one more block.
+template <typename Scalar, typename Compute, int kKind, bool kBatch>
+inline constexpr int kPhaseMinBlocks =
+    kKind == kPhaseCompressReverse && sizeof(Compute) == 4 ? (kBatch ? 6 : 7) : 0;
+
 // Forest layout: thread t runs operation offset + t (finish: instance), or
 // team w of kTeam threads the tail of tree offset + w.
 template <typename Scalar, typename Compute, int kKind, int kTeam = 1>
-__global__ void __launch_bounds__(kPhaseThreads) PhaseKernel(PhaseArgs args) {
+__global__ void
+__launch_bounds__(kPhaseThreads, kPhaseMinBlocks<Scalar, Compute, kKind, false>)
+    PhaseKernel(PhaseArgs args) {
   if constexpr (kKind == kPhaseTailForward || kKind == kPhaseTailReverse) {
     const std::uint32_t w = blockIdx.x * (kPhaseThreads / kTeam) + threadIdx.x / kTeam;
     if (w >= args.count)
@@ -598,7 +637,8 @@ __global__ void __launch_bounds__(kPhaseThreads) PhaseKernel(PhaseArgs args) {
 // Shared-topology layout: thread t runs operation offset + t / items of
 // batch item first_item + t % items (finish: the root record for that item).
 template <typename Scalar, typename Compute, int kKind>
-__global__ void __launch_bounds__(kPhaseThreads) BatchPhaseKernel(PhaseArgs args) {
+__global__ void __launch_bounds__(kPhaseThreads, kPhaseMinBlocks<Scalar, Compute, kKind, true>)
+    BatchPhaseKernel(PhaseArgs args) {
   // Below 2^31 in all (the record index limit).
   const std::uint32_t total = args.count * args.items;
   std::uint32_t t = blockIdx.x * kPhaseThreads + threadIdx.x;
