@@ -125,20 +125,22 @@ struct PhaseArgs {
 
 // Byte offsets of a tree's arrays in its block's shared memory (TreePhaseKernel).
 struct TreePhaseLayout {
-  std::uint64_t gathers, compress, edges, comps, comp_mu, nodes, node_out, node_exp, comp_exp,
+  std::uint64_t gathers, compress, rounds, round_rakes, edges, comps, comp_mu, nodes, node_out, node_exp, comp_exp,
       bytes;
 };
 inline TreePhaseLayout MakeTreePhaseLayout(std::uint64_t nodes, std::uint64_t edges,
-                                              std::uint64_t rakes, std::uint64_t gathers,
-                                              std::uint64_t compressions, std::uint64_t states,
-                                              std::uint64_t scalar, std::uint64_t compute,
-                                              bool reverse) {
+                                           std::uint64_t rakes, std::uint64_t gathers,
+                                           std::uint64_t compressions, std::uint64_t rounds,
+                                           std::uint64_t states, std::uint64_t scalar,
+                                           std::uint64_t compute, bool reverse) {
   const auto up = [](std::uint64_t bytes) { return (bytes + 15) & ~std::uint64_t{15}; };
   const std::uint64_t matrix = states * states * compute;
   TreePhaseLayout at{};
   at.gathers = 16 * rakes; // the rakes come first
   at.compress = at.gathers + 16 * gathers;
-  at.edges = at.compress + 16 * compressions;
+  at.rounds = at.compress + 16 * compressions;
+  at.round_rakes = at.rounds + 16 * rounds;
+  at.edges = at.round_rakes + up(8 * rounds);
   at.comps = at.edges + up(edges * matrix);
   at.comp_mu = at.comps + up(compressions * matrix);
   at.nodes = at.comp_mu + (reverse ? up(compressions * matrix) : 0);

@@ -489,8 +489,10 @@ template <typename Scalar, typename Compute, int KMAX> struct GroupPhaseOps {
       a.comp_exp[Store(i)] = e + s;
   }
 
-  // log Z = ln 2 * (root exponent) + log(sum(root)), as LinearEngine::Run
-  // (one thread): root record i, result of instance `value`.
+  // log Z = ln 2 * (root exponent) + log(sum(root)), as LinearEngine::Run: root
+  // record i, result of instance `value`. Every lane forms the sum; lane j
+  // divides for state j (FP64 divisions one after the other in one thread took
+  // most of the launch's 14 us at K = 20).
   __device__ __forceinline__ void Finish(std::uint32_t i, std::uint32_t value) const {
     const uint2 rec = a.roots[i];
     const std::uint32_t node = rec.x & kMask;
@@ -512,15 +514,11 @@ template <typename Scalar, typename Compute, int KMAX> struct GroupPhaseOps {
     const double log_z = !(sum > 0.0)
                              ? -INFINITY
                              : fma(static_cast<double>(total), 0.6931471805599453094, log(sum));
-    static_cast<Scalar *>(a.values)[value] = static_cast<Scalar>(a.raw ? exp(log_z) : log_z);
-    if (a.reverse) {
-      Scalar *root_out = NodeOutAt(node);
-      const bool finite = log_z > -INFINITY;
-#pragma unroll
-      for (unsigned j = 0; j < KMAX; ++j)
-        if (j < K)
-          root_out[j] =
-              static_cast<Scalar>(finite ? static_cast<double>(root[j]) / sum : 0.0);
+    if (lane == 0)
+      static_cast<Scalar *>(a.values)[value] = static_cast<Scalar>(a.raw ? exp(log_z) : log_z);
+    if (a.reverse && lane < K) {
+      const double own = static_cast<double>(Select(root, lane));
+      NodeOutAt(node)[lane] = static_cast<Scalar>(log_z > -INFINITY ? own / sum : 0.0);
     }
   }
 
@@ -748,13 +746,13 @@ template <int KMAX, bool kWide> constexpr int GroupPhaseMinBlocks(int kind) {
 }
 
 // One kind of one round: lane group g of the grid runs operation offset + g /
-// items of item first_item + g % items (finish: thread t the root record).
+// items of item first_item + g % items (finish: the root record).
 template <typename Scalar, typename Compute, int KMAX, int kKind>
 __global__ void __launch_bounds__(kGroupPhaseThreads,
                                   GroupPhaseMinBlocks<KMAX, sizeof(Compute) == 8>(kKind))
     GroupPhaseKernel(PhaseArgs args) {
   using Ops = GroupPhaseOps<Scalar, Compute, KMAX>;
-  constexpr int G = kKind == kPhaseFinish ? 1 : Ops::G;
+  constexpr int G = Ops::G;
   constexpr int kElements = kGroupPhaseElements<KMAX, kKind>;
   extern __shared__ __align__(16) unsigned char group_smem[];
   const std::uint64_t t =

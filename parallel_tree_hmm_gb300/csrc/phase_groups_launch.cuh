@@ -12,7 +12,7 @@ namespace group_phase {
 template <typename Scalar, typename Compute, int KMAX, int kKind>
 cudaError_t LaunchKind(const PhaseArgs &args, cudaStream_t stream, int *blocks_per_sm) {
   auto kernel = GroupPhaseKernel<Scalar, Compute, KMAX, kKind>;
-  constexpr unsigned lanes = kKind == kPhaseFinish ? 1 : GroupLanes<KMAX>();
+  constexpr unsigned lanes = GroupLanes<KMAX>();
   constexpr unsigned smem = kGroupPhaseThreads / lanes * kGroupPhaseElements<KMAX, kKind> *
                             static_cast<unsigned>(sizeof(Compute));
   static_assert(smem <= 227 * 1024, "shared memory per block");
@@ -27,8 +27,7 @@ cudaError_t LaunchKind(const PhaseArgs &args, cudaStream_t stream, int *blocks_p
                                                          kGroupPhaseThreads, smem);
   if (args.count == 0 || args.items == 0)
     return cudaSuccess;
-  // Finish: one thread per instance; the other kinds one lane group per
-  // operation and item.
+  // One lane group per operation (finish: instance) and item.
   const std::uint64_t threads = static_cast<std::uint64_t>(args.count) * args.items * lanes;
   const std::uint64_t grid = (threads + kGroupPhaseThreads - 1) / kGroupPhaseThreads;
   if (grid > 0x7fffffffull)

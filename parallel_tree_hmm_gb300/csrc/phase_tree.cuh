@@ -258,6 +258,16 @@ __device__ __forceinline__ void CopyIn(std::uint32_t count, Load load, Put put) 
   }
 }
 
+// Starts copying `count` records (of 8 or 16 bytes) into shared memory.
+template <typename T>
+__device__ __forceinline__ void CopyAsyncAll(T *dst, const T *src, std::uint32_t count) {
+  for (std::uint32_t i = threadIdx.x; i < count; i += kTreePhaseThreads)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                     static_cast<unsigned>(__cvta_generic_to_shared(dst + i))),
+                 "l"(src + i), "n"(sizeof(T))
+                 : "memory");
+}
+
 // Block b takes item first_item + b.
 template <typename Scalar, typename Compute, int K>
 __global__ void __launch_bounds__(kTreePhaseThreads) TreePhaseKernel(TreePhaseArgs args) {
@@ -282,21 +292,20 @@ __global__ void __launch_bounds__(kTreePhaseThreads) TreePhaseKernel(TreePhaseAr
   ops.mask = 0xfu << (t & 28u);
 
   const Scalar *edge_in = static_cast<const Scalar *>(in.edge_in);
+  // The records by asynchronous copies, under the loads of the factors.
+  uint4 *rounds = reinterpret_cast<uint4 *>(tree_smem + at.rounds);
+  uint2 *round_rakes = reinterpret_cast<uint2 *>(tree_smem + at.round_rakes);
+  CopyAsyncAll(ops.rakes, in.rakes, args.rakes);
+  CopyAsyncAll(ops.gathers, in.gathers, args.gathers);
+  CopyAsyncAll(ops.compress, in.compress, args.compressions);
+  CopyAsyncAll(rounds, args.round_ops, args.rounds);
+  CopyAsyncAll(round_rakes, args.round_rakes, args.rounds);
+  const std::uint32_t root = in.roots[0].x & kMask;
   CopyIn<Scalar>(
       args.edges * (K * K), [&](std::uint32_t i) { return edge_in[i]; },
       [&](std::uint32_t i, Scalar v) { ops.edges[i] = static_cast<Compute>(v); });
-  CopyIn<uint4>(
-      args.rakes, [&](std::uint32_t i) { return in.rakes[i]; },
-      [&](std::uint32_t i, uint4 v) { ops.rakes[i] = v; });
-  CopyIn<uint4>(
-      args.gathers, [&](std::uint32_t i) { return in.gathers[i]; },
-      [&](std::uint32_t i, uint4 v) { ops.gathers[i] = v; });
-  CopyIn<uint4>(
-      args.compressions, [&](std::uint32_t i) { return in.compress[i]; },
-      [&](std::uint32_t i, uint4 v) { ops.compress[i] = v; });
   for (std::uint32_t i = t; i < args.nodes; i += kTreePhaseThreads)
     ops.node_exp[i] = 0;
-  const std::uint32_t root = in.roots[0].x & kMask;
   if (!in.categorical) {
     const Scalar *node_in = static_cast<const Scalar *>(in.node_in) + item * args.nodes * K;
     CopyIn<Scalar>(
@@ -328,12 +337,13 @@ __global__ void __launch_bounds__(kTreePhaseThreads) TreePhaseKernel(TreePhaseAr
           }
         });
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
 
   constexpr unsigned kGroups = kTreePhaseThreads / 4;
   const unsigned g = t / 4;
   for (std::uint32_t e = 0; e < args.rounds; ++e) {
-    const uint4 round = args.round_ops[e];
+    const uint4 round = rounds[e];
     for (std::uint32_t i = g; i < round.y; i += kGroups)
       ops.Gather(round.x + i);
     __syncthreads();
@@ -363,15 +373,15 @@ __global__ void __launch_bounds__(kTreePhaseThreads) TreePhaseKernel(TreePhaseAr
     return;
   __syncthreads();
   for (std::uint32_t e = args.rounds; e-- > 0;) {
-    const uint4 round = args.round_ops[e];
+    const uint4 round = rounds[e];
     if (round.w != 0) {
       for (std::uint32_t i = g; i < round.w; i += kGroups)
         ops.CompressReverse(round.z + i);
       __syncthreads();
     }
-    const uint2 round_rakes = args.round_rakes[e];
-    for (std::uint32_t i = g; i < round_rakes.y; i += kGroups)
-      ops.RakeReverse(round_rakes.x + i);
+    const uint2 leaves = round_rakes[e];
+    for (std::uint32_t i = g; i < leaves.y; i += kGroups)
+      ops.RakeReverse(leaves.x + i);
     __syncthreads();
   }
   Scalar *out = static_cast<Scalar *>(in.node_out) + item * args.nodes * K;

@@ -1005,8 +1005,8 @@ struct Workspace {
       return std::nullopt;
     const TreePhaseLayout at =
         MakeTreePhaseLayout(nodes_per_item, edges_per_item, phase.rake_base[phase.rounds],
-                            phase.gather_base[phase.rounds], phase.total_compressions, states,
-                            ScalarBytes(), compute_f64 ? 8 : 4, operation == THMM_OP_MARGINALS);
+                            phase.gather_base[phase.rounds], phase.total_compressions,
+                            phase.rounds, states, ScalarBytes(), compute_f64 ? 8 : 4, operation == THMM_OP_MARGINALS);
     if (at.bytes > kTreePhaseMaxBytes)
       return std::nullopt;
     const std::uint64_t resident =
