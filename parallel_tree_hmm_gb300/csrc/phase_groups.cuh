@@ -118,7 +118,8 @@ template <int kPending> __device__ __forceinline__ void CopyWait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
 }
 
-template <typename Scalar, typename Compute, int KMAX> struct GroupPhaseOps {
+// kExact: K == KMAX, so that the compiler folds the bounds and the strides.
+template <typename Scalar, typename Compute, int KMAX, bool kExact> struct GroupPhaseOps {
   using Tile = GroupTile<KMAX>;
   static constexpr int G = Tile::G, CQ = Tile::CQ, TR = Tile::TR, RG = Tile::RG, P = Tile::P;
   const PhaseArgs &a;
@@ -133,7 +134,7 @@ template <typename Scalar, typename Compute, int KMAX> struct GroupPhaseOps {
 
   __device__ __forceinline__ GroupPhaseOps(const PhaseArgs &args, std::uint32_t batch_item,
                                            Compute *group_smem)
-      : a(args), K(args.states), KK(args.states * args.states), item(batch_item),
+      : a(args), K(kExact ? KMAX : args.states), KK(K * K), item(batch_item),
         stride(args.item_stride), lane(threadIdx.x % G),
         mask(G == 32 ? kFull : ((1u << (G & 31)) - 1u) << (threadIdx.x % 32 / G * G)),
         ti(lane / CQ), tj(lane % CQ), smem(group_smem) {}
@@ -747,11 +748,11 @@ template <int KMAX, bool kWide> constexpr int GroupPhaseMinBlocks(int kind) {
 
 // One kind of one round: lane group g of the grid runs operation offset + g /
 // items of item first_item + g % items (finish: the root record).
-template <typename Scalar, typename Compute, int KMAX, int kKind>
+template <typename Scalar, typename Compute, int KMAX, int kKind, bool kExact>
 __global__ void __launch_bounds__(kGroupPhaseThreads,
                                   GroupPhaseMinBlocks<KMAX, sizeof(Compute) == 8>(kKind))
     GroupPhaseKernel(PhaseArgs args) {
-  using Ops = GroupPhaseOps<Scalar, Compute, KMAX>;
+  using Ops = GroupPhaseOps<Scalar, Compute, KMAX, kExact>;
   constexpr int G = Ops::G;
   constexpr int kElements = kGroupPhaseElements<KMAX, kKind>;
   extern __shared__ __align__(16) unsigned char group_smem[];
