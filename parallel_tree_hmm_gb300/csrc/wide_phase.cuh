@@ -19,15 +19,16 @@
 //     own renormalisation exponent (comp_exp minus its inputs' exponents)
 //     instead of recomputing the forward product, so a reverse compression
 //     takes two tensor-core products instead of three;
-//   * operand staging maps threads so that both the global loads (runs of
-//     16-byte quads) and the shared-memory stores (eight rows of a core
-//     matrix per 128-byte wavefront) are conflict-free, with a batch of
-//     loads in flight per thread, and the next operation's matrices are
-//     prefetched into L2 while the current one is worked on;
+//   * a rake's next path is prefetched into L2 while the current operation is
+//     worked on (K % 4 == 0);
 //   * at K_P = 64 the X operand's padded rows 64..127 are not stored: the
 //     MMA tile has M = 128, and the lanes of rows >= 64 read whatever follows
 //     the live rows (the lo part, the Y operand), results nobody reads, so
 //     a CTA holds 64 KB of operands instead of 96 KB and three CTAs fit an SM.
+// The tensor-core kinds here run where K % 4 != 0: such rows have no aligned
+// 16-byte quads, and operands are staged element by element. For the other K
+// the two kinds are pipelines of their own (wide_stream.cuh), which share this
+// file's layout and product steps.
 // Every tensor-core wait is bounded; a wait that gives up sets
 // kErrorTensorTimeout in the error word and the host reports an error.
 #ifndef THMM_WIDE_PHASE_CUH_
@@ -49,15 +50,10 @@ template <int KP> struct PhaseLayout {
   // Threads per CTA: 256 at KP = 64 (three CTAs per SM), 512 at KP = 128 (one
   // CTA per SM); warps w, w + 4, ... share TMEM lane quarter w and split the
   // columns. The kernels wait on global loads and barriers, so warps in
-  // flight count for more than registers: against half the threads the dense
-  // K = 64 step (64 trees x 2000 nodes) went from 7.70 to 6.82 ms although
-  // 80 registers spill a little, the K = 128 one (64 x 500) from 12.9 to
-  // 9.1 ms. Two CTAs of 256 threads without spills took 9.4 ms at K = 64.
+  // flight count for more than registers: against half the threads, with all
+  // kinds in these kernels, the dense K = 64 step (64 trees x 2000 nodes) went
+  // from 7.70 to 6.82 ms, the K = 128 one (64 x 500) from 12.9 to 9.1 ms.
   static constexpr unsigned kThreads = KP == 64 ? 256u : 512u;
-  // Quads of each operand whose loads a thread has in flight: with 24 warps
-  // per SM at KP = 64 one is faster than two (6.82 against 7.74 ms), for the
-  // registers; at KP = 128 two (9.13 against 9.44 ms).
-  static constexpr unsigned kBatch = KP == 64 ? 1 : 2;
   static constexpr unsigned kPart = KP * kChunk * 4;
   static constexpr unsigned kXh = 0, kXl = kPart, kYh = 2 * kPart, kYl = 3 * kPart;
   static constexpr unsigned kVectorsAt = 4 * kPart;
@@ -111,8 +107,8 @@ __device__ __forceinline__ int ExponentOf(float m) { return m > 0.0f ? Pow2Expon
 
 // ------------------------------------------------------------ operand sources
 // A product operand element (r, d): row r of the operand, depth d. Row
-// sources read element (r, d) at p[r * K + d] (four consecutive depths per
-// 16-byte Quad); column sources at p[d * K + r].
+// sources read element (r, d) at p[r * K + d], column sources at
+// p[d * K + r].
 struct Rows {
   static constexpr bool kColumns = false;
   const float *p;
@@ -120,16 +116,6 @@ struct Rows {
   __device__ __forceinline__ float At(unsigned K, unsigned r, unsigned d) const {
     const float v = p[static_cast<std::size_t>(r) * K + d];
     return scale != nullptr ? v * scale[d] : v;
-  }
-  __device__ __forceinline__ float4 Quad(unsigned K, unsigned r, unsigned d) const {
-    float4 v = *reinterpret_cast<const float4 *>(p + static_cast<std::size_t>(r) * K + d);
-    if (scale != nullptr) {
-      v.x *= scale[d];
-      v.y *= scale[d + 1];
-      v.z *= scale[d + 2];
-      v.w *= scale[d + 3];
-    }
-    return v;
   }
 };
 struct Columns {
@@ -168,12 +154,6 @@ struct RatioRows {
     const std::size_t at = static_cast<std::size_t>(r) * K + d;
     return ratio(mu[at], stored[at]);
   }
-  __device__ __forceinline__ float4 Quad(unsigned K, unsigned r, unsigned d) const {
-    const std::size_t at = static_cast<std::size_t>(r) * K + d;
-    const float4 m = *reinterpret_cast<const float4 *>(mu + at);
-    const float4 s = *reinterpret_cast<const float4 *>(stored + at);
-    return make_float4(ratio(m.x, s.x), ratio(m.y, s.y), ratio(m.z, s.z), ratio(m.w, s.w));
-  }
 };
 struct RatioColumns {
   static constexpr bool kColumns = true;
@@ -191,75 +171,6 @@ struct RatioColumns {
 // = the chunk's part of [0, K)) in TF32 hi/lo parts (bf16: as BF16 in `hi`);
 // padded depths of the chunk are zero (cleared once per launch, and again
 // for a later, shorter chunk), padded rows are never read.
-//
-// K % 4 == 0: each thread moves quads (4 consecutive depths of one row) in
-// passes of kBatch (PhaseLayout): all loads of a pass for both operands are issued before
-// any store, so a thread has up to 2 kBatch global loads in flight.
-//   * Row sources: a warp takes 8 rows x 4 quads, so its global loads are
-//     64-byte runs of 8 rows and its 16-byte shared-memory stores fill whole
-//     128-byte core-matrix rows (4 wavefronts for 512 bytes);
-//   * column sources: a warp takes 32 consecutive rows of one quad of
-//     depths, four coalesced 128-byte loads and one 16-byte store per thread.
-// This thread's walk over the quad slots of an operand chunk: slot
-// threadIdx.x, then every T-th. The row and quad of each slot are
-// advanced incrementally (one division when the walk starts, none per slot).
-//   * Row sources: slot idx is lane t = idx % 32 of group g = idx / 32, row
-//     (g / quad_groups) * 8 + t % 8, quad (g % quad_groups) * 4 + t / 8;
-//   * column sources: row idx % K, quad idx / K.
-template <class Src, unsigned T> struct QuadCursor {
-  unsigned K, quads, quad_groups;
-  unsigned major, minor; // rows: g / quad_groups, g % quad_groups; columns: q, r
-  unsigned step_major, step_minor;
-  unsigned lane_row, lane_quad;
-  __device__ __forceinline__ QuadCursor(unsigned states, unsigned depth)
-      : K(states), quads(depth / 4), quad_groups((depth / 4 + 3) / 4) {
-    if constexpr (Src::kColumns) {
-      major = threadIdx.x / K;
-      minor = threadIdx.x % K;
-      step_major = T / K;
-      step_minor = T % K;
-      lane_row = lane_quad = 0;
-    } else {
-      const unsigned g = threadIdx.x >> 5, t = threadIdx.x & 31u;
-      major = g / quad_groups;
-      minor = g % quad_groups;
-      step_major = (T / 32) / quad_groups;
-      step_minor = (T / 32) % quad_groups;
-      lane_row = t & 7u;
-      lane_quad = t >> 3;
-    }
-  }
-  __device__ __forceinline__ unsigned Row() const {
-    return Src::kColumns ? minor : major * 8 + lane_row;
-  }
-  __device__ __forceinline__ unsigned Quad() const {
-    return Src::kColumns ? major : minor * 4 + lane_quad;
-  }
-  // Slots remain (this one may still be padding).
-  __device__ __forceinline__ bool More() const {
-    return Src::kColumns ? major < quads : major * 8 < K;
-  }
-  __device__ __forceinline__ bool Valid() const { return More() && Row() < K && Quad() < quads; }
-  __device__ __forceinline__ void Advance() {
-    const unsigned limit = Src::kColumns ? K : quad_groups;
-    major += step_major;
-    minor += step_minor;
-    if (minor >= limit) {
-      minor -= limit;
-      ++major;
-    }
-  }
-};
-
-template <class Src>
-__device__ __forceinline__ float4 LoadQuad(const Src &src, unsigned K, unsigned r, unsigned d) {
-  if constexpr (Src::kColumns)
-    return make_float4(src.At(K, r, d), src.At(K, r, d + 1), src.At(K, r, d + 2),
-                       src.At(K, r, d + 3));
-  else
-    return src.Quad(K, r, d);
-}
-
 template <bool kBf16>
 __device__ __forceinline__ void Put(unsigned char *hi, unsigned char *lo, unsigned r,
                                    unsigned d, float v) {
@@ -289,7 +200,8 @@ __device__ __forceinline__ void ClearTail(unsigned K, unsigned depth, unsigned c
     Put<kBf16>(hi, lo, idx / pad, depth + idx % pad, 0.0f);
 }
 
-// Any K: one element per slot (used when K % 4 != 0).
+// One element per thread and step: rows of K % 4 != 0 floats have no aligned
+// quads (the other K go to wide_stream.cuh).
 template <bool kBf16, unsigned T, class Src>
 __device__ __forceinline__ void StageScalar(const Src &src, unsigned K, unsigned d0,
                                             unsigned depth, unsigned char *hi,
@@ -303,7 +215,7 @@ __device__ __forceinline__ void StageScalar(const Src &src, unsigned K, unsigned
 }
 
 // Stages depth chunk d0 of both operands of a product.
-template <bool kBf16, unsigned T, unsigned kBatch, class XS, class YS>
+template <bool kBf16, unsigned T, class XS, class YS>
 __device__ __forceinline__ void StageChunk(const XS &x, const YS &y, unsigned K, unsigned d0,
                                            unsigned char *xh, unsigned char *xl,
                                            unsigned char *yh, unsigned char *yl) {
@@ -312,41 +224,8 @@ __device__ __forceinline__ void StageChunk(const XS &x, const YS &y, unsigned K,
     ClearTail<kBf16, T>(K, depth, xh, xl);
     ClearTail<kBf16, T>(K, depth, yh, yl);
   }
-  if (K % 4 != 0) {
-    StageScalar<kBf16, T>(x, K, d0, depth, xh, xl);
-    StageScalar<kBf16, T>(y, K, d0, depth, yh, yl);
-    return;
-  }
-  QuadCursor<XS, T> xs(K, depth);
-  QuadCursor<YS, T> ys(K, depth);
-#pragma unroll 1
-  while (xs.More() || ys.More()) {
-    float4 xv[kBatch], yv[kBatch];
-    unsigned xr[kBatch], xq[kBatch], yr[kBatch], yq[kBatch];
-    bool xok[kBatch], yok[kBatch];
-#pragma unroll
-    for (unsigned b = 0; b < kBatch; ++b) {
-      xok[b] = xs.Valid();
-      xr[b] = xs.Row();
-      xq[b] = xs.Quad();
-      xs.Advance();
-      yok[b] = ys.Valid();
-      yr[b] = ys.Row();
-      yq[b] = ys.Quad();
-      ys.Advance();
-      if (xok[b])
-        xv[b] = LoadQuad(x, K, xr[b], d0 + 4 * xq[b]);
-      if (yok[b])
-        yv[b] = LoadQuad(y, K, yr[b], d0 + 4 * yq[b]);
-    }
-#pragma unroll
-    for (unsigned b = 0; b < kBatch; ++b) {
-      if (xok[b])
-        Put4<kBf16>(xh, xl, xr[b], 4 * xq[b], xv[b]);
-      if (yok[b])
-        Put4<kBf16>(yh, yl, yr[b], 4 * yq[b], yv[b]);
-    }
-  }
+  StageScalar<kBf16, T>(x, K, d0, depth, xh, xl);
+  StageScalar<kBf16, T>(y, K, d0, depth, yh, yl);
 }
 
 // Issues the tensor-core steps of depth chunk `chunk` of a product whose
@@ -432,68 +311,12 @@ __device__ bool PhaseProduct(unsigned char *smem, PhaseShared &sh, std::uint32_t
     const unsigned d0 = chunk * kChunk;
     constexpr unsigned T = L::kThreads;
     if (bf16)
-      StageChunk<true, T, L::kBatch>(x, y, K, d0, xh, nullptr, yh, nullptr);
+      StageChunk<true, T>(x, y, K, d0, xh, nullptr, yh, nullptr);
     else
-      StageChunk<false, T, L::kBatch>(x, y, K, d0, xh, xl, yh, yl);
+      StageChunk<false, T>(x, y, K, d0, xh, xl, yh, yl);
     ok = MmaChunk<KP, kSplit>(smem, sh, phase, tmem, chunk, bf16) && ok;
   }
   return ok;
-}
-
-// Stages depth chunk d0 of one operand (K % 4 == 0), loads batched as in
-// StageChunk.
-template <bool kBf16, unsigned T, unsigned kBatch, class Src>
-__device__ __forceinline__ void StageOne(const Src &src, unsigned K, unsigned d0,
-                                         unsigned char *hi, unsigned char *lo) {
-  const unsigned depth = K - d0 < kChunk ? K - d0 : kChunk;
-  QuadCursor<Src, T> cursor(K, depth);
-#pragma unroll 1
-  while (cursor.More()) {
-    float4 v[kBatch];
-    unsigned rows[kBatch], quads[kBatch];
-    bool ok[kBatch];
-#pragma unroll
-    for (unsigned b = 0; b < kBatch; ++b) {
-      ok[b] = cursor.Valid();
-      rows[b] = cursor.Row();
-      quads[b] = cursor.Quad();
-      cursor.Advance();
-      if (ok[b])
-        v[b] = LoadQuad(src, K, rows[b], d0 + 4 * quads[b]);
-    }
-#pragma unroll
-    for (unsigned b = 0; b < kBatch; ++b)
-      if (ok[b])
-        Put4<kBf16>(hi, lo, rows[b], 4 * quads[b], v[b]);
-  }
-}
-
-// Y(n, d) = X(d, n) for n, d < K (KP = 64: one depth chunk holds the whole
-// staged operand): copies the staged hi and lo parts (BF16: hi) element by
-// element, so the transpose holds exactly the values staged in X. A warp
-// moves an 8 x 4 block of X per step: its reads cover one core matrix row
-// set (32 distinct banks), its writes two.
-template <bool kBf16, unsigned T>
-__device__ __forceinline__ void TransposeStaged(unsigned K, const unsigned char *xh,
-                                                const unsigned char *xl, unsigned char *yh,
-                                                unsigned char *yl) {
-  const unsigned warp = threadIdx.x / 32, lane = threadIdx.x & 31u;
-  const unsigned row_blocks = (K + 7) / 8, col_blocks = (K + 3) / 4;
-  for (unsigned block = warp; block < row_blocks * col_blocks; block += T / 32) {
-    const unsigned d = (block / col_blocks) * 8 + lane / 4;
-    const unsigned n = (block % col_blocks) * 4 + lane % 4;
-    if (d < K && n < K) {
-      if constexpr (kBf16) {
-        *reinterpret_cast<unsigned short *>(yh + CoreOffset16(n, d)) =
-            *reinterpret_cast<const unsigned short *>(xh + CoreOffset16(d, n));
-      } else {
-        const std::uint32_t from = umma::CoreOffset(d, n, kSbo);
-        const std::uint32_t to = umma::CoreOffset(n, d, kSbo);
-        *reinterpret_cast<float *>(yh + to) = *reinterpret_cast<const float *>(xh + from);
-        *reinterpret_cast<float *>(yl + to) = *reinterpret_cast<const float *>(xl + from);
-      }
-    }
-  }
 }
 
 // One operation of a wide phase kind, executed by the whole CTA.
@@ -577,37 +400,6 @@ template <int KP> struct WideOps {
     return 0;
   }
 
-  // Row stride (floats) of a K x K tile staged in the operand buffers: K + 4,
-  // so that the 16-byte row writes of eight consecutive rows (one per
-  // thread) and the row reads of the coalesced passes are conflict-free.
-  __device__ __forceinline__ unsigned TileStride() const { return K + 4; }
-  // Writes columns [c, c + 32) ∩ [0, K) of row j of a tile (K % 4 == 0).
-  __device__ __forceinline__ void TileRow(float *tile, unsigned j, unsigned c,
-                                          const float (&row)[32]) const {
-#pragma unroll
-    for (unsigned q = 0; q < 32; q += 4)
-      if (c + q < K)
-        *reinterpret_cast<float4 *>(tile + j * TileStride() + c + q) =
-            make_float4(row[q], row[q + 1], row[q + 2], row[q + 3]);
-  }
-
-  // This thread's walk over the quads of a row-major K x K matrix (K % 4 ==
-  // 0): quad threadIdx.x, then every kThreads-th, as (row, first column).
-  struct TileWalk {
-    unsigned quads, row, column, step_rows, step_quads;
-    __device__ __forceinline__ explicit TileWalk(unsigned K)
-        : quads(K / 4), row(threadIdx.x / (K / 4)), column(4 * (threadIdx.x % (K / 4))),
-          step_rows(kThreads / (K / 4)), step_quads(kThreads % (K / 4)) {}
-    __device__ __forceinline__ void Advance() {
-      row += step_rows;
-      column += 4 * step_quads;
-      if (column >= 4 * quads) {
-        column -= 4 * quads;
-        ++row;
-      }
-    }
-  };
-
   // Rows per warp whose loads are in flight together (MatVec, RakeReverse).
   static constexpr unsigned kRows = KP == 64 ? 8 : 4;
 
@@ -651,15 +443,7 @@ template <int KP> struct WideOps {
     if (K % 4 != 0)
       return;
     const std::uint32_t bytes = KK * 4u;
-    if constexpr (kKind == kPhaseCompress || kKind == kPhaseCompressReverse) {
-      const uint4 op = a.compress[i];
-      umma::PrefetchL2(PathPtr(op.x), bytes);
-      umma::PrefetchL2(PathPtr(op.z), bytes);
-      if constexpr (kKind == kPhaseCompressReverse) {
-        umma::PrefetchL2(CompMu() + static_cast<std::size_t>(i) * KK, bytes);
-        umma::PrefetchL2(Comps() + static_cast<std::size_t>(i) * KK, bytes);
-      }
-    } else if constexpr (kKind == kPhaseRakeReverse) {
+    if constexpr (kKind == kPhaseRakeReverse) {
       umma::PrefetchL2(PathPtr(a.rakes[i].x), bytes);
     } else if constexpr (kKind == kPhaseGather) {
       const uint4 op = a.gathers[i];
@@ -731,36 +515,15 @@ template <int KP> struct WideOps {
     }
     const int s = ExponentOf(CtaMax<kThreads>(m, sh));
     float *out = Comps() + static_cast<std::size_t>(i) * KK;
-    if (K % 4 == 0) {
-      // Rows through the (now idle) operand buffers, then coalesced stores.
-      float *tile = reinterpret_cast<float *>(smem);
 #pragma unroll 1
-      for (unsigned c = c0; c < c0 + kPartColumns; c += 32) {
-        float values[32];
-        SplitSum32<KP>(lane_base, c, values, a.bf16 != 0);
-        if (row < K) {
+    for (unsigned c = c0; c < c0 + kPartColumns; c += 32) {
+      float values[32];
+      SplitSum32<KP>(lane_base, c, values, a.bf16 != 0);
+      if (row < K) {
 #pragma unroll
-          for (unsigned q = 0; q < 32; ++q)
-            values[q] = ScalePow2(values[q], -s);
-          TileRow(tile, row, c, values);
-        }
-      }
-      __syncthreads();
-#pragma unroll 4
-      for (TileWalk w(K); w.row < K; w.Advance())
-        *reinterpret_cast<float4 *>(out + static_cast<std::size_t>(w.row) * K + w.column) =
-            *reinterpret_cast<const float4 *>(tile + w.row * TileStride() + w.column);
-    } else {
-#pragma unroll 1
-      for (unsigned c = c0; c < c0 + kPartColumns; c += 32) {
-        float values[32];
-        SplitSum32<KP>(lane_base, c, values, a.bf16 != 0);
-        if (row < K) {
-#pragma unroll
-          for (unsigned q = 0; q < 32; ++q)
-            if (c + q < K)
-              out[static_cast<std::size_t>(row) * K + c + q] = ScalePow2(values[q], -s);
-        }
+        for (unsigned q = 0; q < 32; ++q)
+          if (c + q < K)
+            out[static_cast<std::size_t>(row) * K + c + q] = ScalePow2(values[q], -s);
       }
     }
     if (threadIdx.x == 0)
@@ -887,147 +650,60 @@ template <int KP> struct WideOps {
     const float *stored = Comps() + static_cast<std::size_t>(i) * KK;
     // P1[r][m] = sum_c R[r][c] right[m][c];  P2[m][c] = sum_r left[r][m] R[r][c].
     const Ratio ratio_of(shift);
-    if (KP == 64 && K % 4 == 0) {
-      // P1 stages R as its X operand; P2's Y operand is that staged R,
-      // transposed in shared memory, so R is formed once per compression.
-      using L = PhaseLayout<KP>;
-      unsigned char *const xh = smem + L::kXh, *const xl = smem + L::kXl;
-      unsigned char *const yh = smem + L::kYh, *const yl = smem + L::kYl;
-      const bool bf16 = a.bf16 != 0;
-      if (bf16)
-        StageChunk<true, kThreads, L::kBatch>(RatioRows{mu, stored, ratio_of},
-                                              Rows{right, nullptr}, K, 0, xh, nullptr, yh,
-                                              nullptr);
-      else
-        StageChunk<false, kThreads, L::kBatch>(RatioRows{mu, stored, ratio_of},
-                                               Rows{right, nullptr}, K, 0, xh, xl, yh, yl);
-      ok = MmaChunk<KP, false>(smem, sh, phase, tmem, 0, bf16) && ok;
-      if (bf16)
-        TransposeStaged<true, kThreads>(K, xh, xl, yh, yl);
-      else
-        TransposeStaged<false, kThreads>(K, xh, xl, yh, yl);
-      __syncthreads();
-      if (bf16)
-        StageOne<true, kThreads, L::kBatch>(Columns{left}, K, 0, xh, nullptr);
-      else
-        StageOne<false, kThreads, L::kBatch>(Columns{left}, K, 0, xh, xl);
-      ok = MmaChunk<KP, false>(smem, sh, phase, tmem + KP, 0, bf16) && ok;
-    } else {
-      ok = PhaseProduct<KP, false>(smem, sh, phase, tmem, K, RatioRows{mu, stored, ratio_of},
-                                   Rows{right, nullptr}, a.bf16 != 0) &&
-           ok;
-      ok = PhaseProduct<KP, false>(smem, sh, phase, tmem + KP, K, Columns{left},
-                                   RatioColumns{mu, stored, ratio_of}, a.bf16 != 0) &&
-           ok;
-    }
+    ok = PhaseProduct<KP, false>(smem, sh, phase, tmem, K, RatioRows{mu, stored, ratio_of},
+                                 Rows{right, nullptr}, a.bf16 != 0) &&
+         ok;
+    ok = PhaseProduct<KP, false>(smem, sh, phase, tmem + KP, K, Columns{left},
+                                 RatioColumns{mu, stored, ratio_of}, a.bf16 != 0) &&
+         ok;
     // Accumulator row `row` (TMEM lane), columns [c0, c0 + kPartColumns).
     const unsigned row = threadIdx.x % 128, c0 = (threadIdx.x / 128) * kPartColumns;
     const std::uint32_t lane_base = tmem + ((row & ~31u) << 16);
     float *left_out = AdjointOf(op.x);
     float *right_out = AdjointOf(op.z);
     float total = 0.0f;
-    if (K % 4 == 0) {
-      // Each product's rows go through the (now idle) operand buffers; the
-      // adjoints are then formed and stored in coalesced passes.
-      float *tile = reinterpret_cast<float *>(smem);
-      const auto stage_rows = [&](std::uint32_t column) {
+    // Row-per-thread stores (tcgen05.ld is warp-collective: every lane
+    // loads, rows >= K discard). The parts' partial middle adjoints meet
+    // in the msg and ratio vectors.
+    const float *left_row = left + static_cast<std::size_t>(row) * K;
+    const float *right_row = right + static_cast<std::size_t>(row) * K;
+    const float middle_row = row < K ? middle[row] : 0.0f;
 #pragma unroll 1
-        for (unsigned c = c0; c < c0 + kPartColumns; c += 32) {
-          float values[32];
-          umma::Load32(lane_base + column + c, values);
-          if (row < K)
-            TileRow(tile, row, c, values);
-        }
-        __syncthreads();
-      };
-      // Left adjoint left[r][m] middle[m] P1[r][m].
-      stage_rows(0);
-#pragma unroll 4
-      for (TileWalk w(K); w.row < K; w.Advance()) {
-        const unsigned r = w.row, c = w.column;
-        const std::size_t at = static_cast<std::size_t>(r) * K + c;
-        const float4 l = *reinterpret_cast<const float4 *>(left + at);
-        const float4 p = *reinterpret_cast<const float4 *>(tile + r * TileStride() + c);
-        *reinterpret_cast<float4 *>(left_out + at) =
-            make_float4(l.x * middle[c] * p.x, l.y * middle[c + 1] * p.y,
-                        l.z * middle[c + 2] * p.z, l.w * middle[c + 3] * p.w);
-      }
-      __syncthreads();
-      // Right adjoint right[m][c] middle[m] P2[m][c], kept in the tile for
-      // the middle adjoint (its row sums).
-      stage_rows(KP);
-#pragma unroll 4
-      for (TileWalk w(K); w.row < K; w.Advance()) {
-        const unsigned r = w.row, c = w.column;
-        const std::size_t at = static_cast<std::size_t>(r) * K + c;
-        const float4 rr = *reinterpret_cast<const float4 *>(right + at);
-        float4 *p = reinterpret_cast<float4 *>(tile + r * TileStride() + c);
-        const float mr = middle[r];
-        const float4 v = *p;
-        const float4 adjoint =
-            make_float4(rr.x * mr * v.x, rr.y * mr * v.y, rr.z * mr * v.z, rr.w * mr * v.w);
-        *reinterpret_cast<float4 *>(right_out + at) = adjoint;
-        *p = adjoint;
-      }
-      __syncthreads();
-      if (j < K) {
-        const float *row_values = tile + j * TileStride();
-        for (unsigned c = 0; c < K; c += 4) {
-          const float4 v = *reinterpret_cast<const float4 *>(row_values + c);
-          total += v.x;
-          total += v.y;
-          total += v.z;
-          total += v.w;
-        }
-      }
-    } else {
-      // Row-per-thread stores (tcgen05.ld is warp-collective: every lane
-      // loads, rows >= K discard). The halves' partial middle adjoints meet
-      // in the msg and ratio vectors.
-      const float *left_row = left + static_cast<std::size_t>(row) * K;
-      const float *right_row = right + static_cast<std::size_t>(row) * K;
-      const float middle_row = row < K ? middle[row] : 0.0f;
-#pragma unroll 1
-      for (unsigned c = c0; c < c0 + kPartColumns; c += 32) {
-        float p1[32];
-        umma::Load32(lane_base + c, p1);
-        if (row < K) {
+    for (unsigned c = c0; c < c0 + kPartColumns; c += 32) {
+      float p1[32];
+      umma::Load32(lane_base + c, p1);
+      if (row < K) {
 #pragma unroll
-          for (unsigned q = 0; q < 32; ++q)
-            if (c + q < K)
-              left_out[static_cast<std::size_t>(row) * K + c + q] =
-                  left_row[c + q] * middle[c + q] * p1[q];
-        }
+        for (unsigned q = 0; q < 32; ++q)
+          if (c + q < K)
+            left_out[static_cast<std::size_t>(row) * K + c + q] =
+                left_row[c + q] * middle[c + q] * p1[q];
       }
-      float partial = 0.0f;
+    }
+    float partial = 0.0f;
 #pragma unroll 1
-      for (unsigned c = c0; c < c0 + kPartColumns; c += 32) {
-        float p2[32];
-        umma::Load32(lane_base + KP + c, p2);
-        if (row < K) {
+    for (unsigned c = c0; c < c0 + kPartColumns; c += 32) {
+      float p2[32];
+      umma::Load32(lane_base + KP + c, p2);
+      if (row < K) {
 #pragma unroll
-          for (unsigned q = 0; q < 32; ++q) {
-            if (c + q < K) {
-              const float adjoint = right_row[c + q] * middle_row * p2[q];
-              right_out[static_cast<std::size_t>(row) * K + c + q] = adjoint;
-              partial += adjoint;
-            }
+        for (unsigned q = 0; q < 32; ++q) {
+          if (c + q < K) {
+            const float adjoint = right_row[c + q] * middle_row * p2[q];
+            right_out[static_cast<std::size_t>(row) * K + c + q] = adjoint;
+            partial += adjoint;
           }
         }
       }
-      // v, leaf, msg and (past middle) ratio are free here: one vector per
-      // part of the columns.
-      float *const parts[4] = {msg, ratio, v, leaf};
-      if (kParts == 1) {
-        total = partial;
-      } else {
-        parts[threadIdx.x / 128][row] = partial;
-        __syncthreads();
-        if (j < K)
-          for (unsigned h = 0; h < kParts; ++h)
-            total += parts[h][j];
-      }
     }
+    // v, leaf, msg and (past middle) ratio are free here: one vector per
+    // part of the columns.
+    float *const parts[4] = {msg, ratio, v, leaf};
+    parts[threadIdx.x / 128][row] = partial;
+    __syncthreads();
+    if (j < K)
+      for (unsigned h = 0; h < kParts; ++h)
+        total += parts[h][j];
     if (j < K)
       NodeOut()[static_cast<std::size_t>(op.y & kMask) * K + j] = total;
     umma::FenceBeforeSync();
@@ -1062,7 +738,7 @@ __global__ void __launch_bounds__(PhaseLayout<KP>::kThreads, KP == 64 ? 3 : 1)
   WideOps<KP> ops(args, sh, dynamic_smem, vectors, kTensor ? sh.tmem : 0u, phase, ok);
   for (std::uint32_t t = blockIdx.x; t < args.count; t += gridDim.x) {
     const std::uint32_t i = args.offset + t;
-    if constexpr (kKind != kPhaseFinish) {
+    if constexpr (kKind == kPhaseGather || kKind == kPhaseRakeReverse) {
       if (threadIdx.x == 0) {
         if (t == blockIdx.x)
           ops.template Prefetch<kKind>(i);
