@@ -7,9 +7,11 @@
 // the kAll/kFactors/kNone residency rules for categorical inputs, six CUDA
 // events for the upload/kernel/download split plus a wall clock, and the same
 // exception classes (reported here as status codes). Where the reference
-// launches one kernel per primitive batch and phase, a prepared call here
-// launches one persistent kernel (engine.cuh) after a small memset, two for
-// marginals (forward sweep, then adjoint sweep).
+// launches one kernel per primitive batch and phase of one topology, a prepared
+// call here launches one per round and kind for all trees (phase.h), from a
+// CUDA graph once the call repeats; or one kernel for a small batch up to four
+// states (phase_tree.cuh); or the persistent per-tree engines (engine.cuh,
+// wide_engine.cuh), one launch and two for marginals.
 #include "thmm_gb300.h"
 
 #include <algorithm>
@@ -878,8 +880,10 @@ struct Workspace {
   // operations, shared out over the trees, are at most four passes of a CTA
   // (512 threads' worth; 64 operations at 8 states). From there a grid-wide
   // launch would do less than its own launch costs, and one CTA per tree runs
-  // the remaining rounds, the root and their top-down steps in one launch. A
-  // forest of more than 2^20 trees stays grid-wide (its tail records).
+  // the remaining rounds, the root and their top-down steps in one launch. At one
+  // (four, sixteen) passes: MAP of 48 trees of up to 6,000 nodes, K = 8, 273
+  // (257, 314) us, sampling of 320 trees of up to 50,000 nodes 1,943 (1,948,
+  // 1,984). A forest of more than 2^20 trees stays grid-wide (its tail records).
   void SetLogRounds() {
     const std::uint64_t lanes = states <= 4 ? 1 : states <= 8 ? 8 : states <= 16 ? 16 : 32;
     const std::uint64_t trees = phase.instance_program.size(); // 1 in the batch layout
@@ -995,23 +999,29 @@ struct Workspace {
   }
 
   // Whether `items` items of a batch workspace run a whole tree per block, and
-  // the shared memory of a block: the tree fits, the blocks are at most four
+  // the shared memory of a block: the tree fits, the blocks are at most three
   // waves of the chip, and either a tree's rounds are one pass of the block (512
-  // nodes) or there are 32 items and more. A few larger trees would gain as
-  // well (16 items of 1,000 nodes), but the one launch per round and kind of
-  // such a batch is what thmm_workspace_launches has reported, and is kept.
+  // nodes) or there are 32 items and more. Measured, a launch per round and kind
+  // -> a block per item, marginals at K = 4: 32 to 152 items of 999 nodes 96 to
+  // 111 -> 27 us, 608 (two waves) 121 -> 96, 1,216 (four) 164 -> 188; 399 nodes,
+  // 1,216 items (under three waves) 100 -> 76, 2,432 125 -> 146; 99 nodes, 1,216
+  // items (two) 66 -> 51, 2,432 (four) 72 -> 100. A few larger trees would gain
+  // as well (8 items of 999 nodes, 98 -> 27), but the one launch per round and
+  // kind of such a batch is what thmm_workspace_launches has reported, and is
+  // kept.
   std::optional<TreePhaseLayout> TreeLayout(int operation, std::uint64_t items) const {
     if (!phase_batch || states > 4 || (nodes_per_item > 512 && items < 32))
       return std::nullopt;
     const TreePhaseLayout at =
         MakeTreePhaseLayout(nodes_per_item, edges_per_item, phase.rake_base[phase.rounds],
                             phase.gather_base[phase.rounds], phase.total_compressions,
-                            phase.rounds, states, ScalarBytes(), compute_f64 ? 8 : 4, operation == THMM_OP_MARGINALS);
+                            phase.rounds, states, ScalarBytes(), compute_f64 ? 8 : 4,
+                            operation == THMM_OP_MARGINALS);
     if (at.bytes > kTreePhaseMaxBytes)
       return std::nullopt;
     const std::uint64_t resident =
         std::min<std::uint64_t>(2048 / kTreePhaseThreads, 228 * 1024 / (at.bytes + 2048));
-    if (items > 4 * resident * static_cast<std::uint64_t>(sms))
+    if (items > 3 * resident * static_cast<std::uint64_t>(sms))
       return std::nullopt;
     return at;
   }
@@ -1167,9 +1177,11 @@ struct Workspace {
 
   // The device step of a prepared call. Launching a chain of 20 to 100 small
   // kernels one by one costs the host 2 to 3 us each, replaying its graph 10
-  // to 20 us in all; building the graph costs as much as some ten calls save,
-  // so it is built when an operation has been called kGraphAfter times in a
-  // row on one batch size.
+  // to 20 us in all (64 items of 999 nodes, K = 4, 29 launches: 219 -> 204 us a
+  // call; MAP of 48 trees, K = 8: 296 -> 290 us; fewer launches than
+  // kGraphLaunches: no gain, 85.6 against 87.4 us). Building the graph costs as
+  // much as some ten calls save, so it is built when an operation has been
+  // called kGraphAfter times in a row on one batch size.
   static constexpr int kGraphAfter = 8;
   static constexpr std::uint64_t kGraphLaunches = 8;
   void EnqueuePrepared(int operation, std::size_t batch) {
