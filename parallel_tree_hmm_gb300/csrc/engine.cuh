@@ -1,4 +1,6 @@
-// Persistent tree-contraction kernels for sm_103a.
+// Persistent per-tree contraction kernels for sm_103a (THMM_SCHEDULE_TEAMS and
+// the forests whose exponents do not fit the phase schedule's; the default
+// schedule is phase.h's), and the arithmetic that both schedules share.
 //
 // Work decomposition. A *team* contracts one tree instance at a time: a whole
 // CTA (128 threads) for large trees, a single warp for small ones. Instances

@@ -1,5 +1,5 @@
 // Level-synchronous phase schedule of the sum-product calls (every state
-// count up to 128).
+// count up to 128) and of MAP and sampling (up to 32 states, phase_log.cuh).
 //
 // The per-tree engine (engine.cuh) contracts one tree per team and walks the
 // tree's plan step by step with a team barrier in between; a tree has 20-50
@@ -11,8 +11,11 @@
 // and the adjoint sweep
 //   compress-reverse(R-1), rake-reverse(R-1), ..., compress-reverse(0),
 //   rake-reverse(0),
-// one thread per operation, with no barriers inside a launch. The
-// operations of one round of one tree are independent (a btrc primitive
+// MAP and sampling the same forward kinds and then their states from the root
+// down, round by round. An operation is taken by a thread (K <= 4,
+// phase_engine.cuh), a lane group (K <= 32, phase_groups.cuh) or a CTA
+// (K <= 128, wide_phase.cuh, wide_stream.cuh), with no barriers between
+// operations. The operations of one round of one tree are independent (a btrc primitive
 // batch), and different trees never share an operand, so each launch is
 // embarrassingly parallel.
 //
@@ -45,16 +48,17 @@ enum PhaseKind : int {
   kPhaseFinish = 2,          // log Z (and the root marginal) per instance
   kPhaseRakeReverse = 3,     // adjoint of the round's rakes
   kPhaseCompressReverse = 4, // adjoint of the round's compressions
-  kPhaseTailForward = 5,     // rounds >= the tail round, one warp per tree
-  kPhaseTailReverse = 6,     // their adjoint, one warp per tree
+  kPhaseTailForward = 5,     // rounds >= the tail round, one warp or block per tree
+  kPhaseTailReverse = 6,     // their adjoint, one warp or block per tree
 };
 
 // The last rounds of a forest hold few operations (rounds 5 and later of the
 // uneven K=4 forest hold 0.4 % of them) but one launch each, and a launch
 // costs microseconds however little it does. From the tail round on, the
-// schedule can switch to one warp per tree that walks the tree's remaining
-// rounds with a warp barrier between steps (the same operation functions,
-// so the same bits). Tail records:
+// schedule can switch to one warp or block per tree that walks the tree's
+// remaining rounds with a barrier between steps (the same operation functions,
+// so the same bits): the sum-product kinds at K <= 4, MAP and sampling at every
+// K, which also come back down these rounds in the same launch. Tail records:
 //   tail item   uint4: instance, first tail round entry, tail rounds, 0
 //   tail round  uint4: first gather, gathers, first compression, compressions
 //   tail rakes  uint2: first rake, rakes (of the same round)
@@ -125,8 +129,8 @@ struct PhaseArgs {
 
 // Byte offsets of a tree's arrays in its block's shared memory (TreePhaseKernel).
 struct TreePhaseLayout {
-  std::uint64_t gathers, compress, rounds, round_rakes, edges, comps, comp_mu, nodes, node_out, node_exp, comp_exp,
-      bytes;
+  std::uint64_t gathers, compress, rounds, round_rakes, edges, comps, comp_mu, nodes, node_out,
+      node_exp, comp_exp, bytes;
 };
 inline TreePhaseLayout MakeTreePhaseLayout(std::uint64_t nodes, std::uint64_t edges,
                                            std::uint64_t rakes, std::uint64_t gathers,

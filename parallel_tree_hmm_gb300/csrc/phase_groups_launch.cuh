@@ -12,9 +12,9 @@ namespace group_phase {
 template <typename Scalar, typename Compute, int KMAX, int kKind>
 cudaError_t LaunchKind(const PhaseArgs &args, cudaStream_t stream, int *blocks_per_sm) {
   // Single precision is bound by instruction issue (53-60 % of the issue
-  // slots in the large rounds), which folded bounds shorten: a gradient step
-  // of 64 trees of 4,000 nodes at K = 20 2,202 -> 2,141 us, 64 sites of one
-  // tree 386 -> 377 us. Double is bound by its pipe and keeps one variant.
+  // slots in the large rounds), which folded bounds shorten: a marginal step
+  // of 256 trees of 5,000 nodes at K = 20 2,202 -> 2,141 us, 500 items on a
+  // 399-node tree 386 -> 377 us. Double is bound by its pipe and keeps one variant.
   auto kernel = GroupPhaseKernel<Scalar, Compute, KMAX, kKind, false>;
   if constexpr (sizeof(Compute) == 4) {
     if (args.states == KMAX)
