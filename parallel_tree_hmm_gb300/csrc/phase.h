@@ -108,6 +108,7 @@ struct PhaseArgs {
   // of a batch whose stored objects are `item_stride` items apart, each with
   // item_nodes nodes and item_edges edges. A forest is one item at stride 1.
   std::uint32_t batch;
+  std::uint32_t input_paths; // every path of the launch is an input edge (round 0)
   std::uint32_t first_item;
   std::uint32_t items;
   std::uint64_t item_stride;

@@ -5,10 +5,19 @@
 #define THMM_PHASE_GROUPS_LAUNCH_CUH_
 
 #include "phase_groups.cuh"
+#include "phase_items.cuh"
 
 namespace thmm {
 namespace group_phase {
 
+// Warps of 32 items from which a launch runs an item per lane: one per SM
+// sub-partition (608). Fewer are bound by a warp's own chain. Marginals at
+// K = 20, lane groups -> an item per lane: 61 nodes, 64 items (some 60 warps)
+// 66 -> 96 us; 399 nodes, 64 items (400) 119 -> 123; 128 items (800) 160 -> 162;
+// 500 items (3,200) 449 -> 402; 1,999 nodes, 64 items (2,000) 328 -> 300, 500
+// items 1,899 -> 1,614. K = 8, 1,000 items of 1,999 nodes 1,273 -> 989; K = 32,
+// 200 items of 999 nodes 745 -> 686.
+constexpr std::uint64_t kItemWarps = 608;
 template <typename Scalar, typename Compute, int KMAX, int kKind>
 cudaError_t LaunchKind(const PhaseArgs &args, cudaStream_t stream, int *blocks_per_sm) {
   // Single precision is bound by instruction issue (53-60 % of the issue
@@ -35,6 +44,25 @@ cudaError_t LaunchKind(const PhaseArgs &args, cudaStream_t stream, int *blocks_p
                                                          kGroupPhaseThreads, smem);
   if (args.count == 0 || args.items == 0)
     return cudaSuccess;
+  if constexpr (sizeof(Compute) == 4 &&
+                (kKind == kPhaseGather || kKind == kPhaseRakeReverse)) {
+    const std::uint64_t warps =
+        static_cast<std::uint64_t>(args.count) * ((args.items + 31) / 32);
+    auto by_item = ItemPhaseKernel<Scalar, KMAX, kKind, true>;
+    if constexpr (kKind == kPhaseGather) {
+      if (args.states != KMAX)
+        by_item = ItemPhaseKernel<Scalar, KMAX, kKind, false>;
+    }
+    // Rake adjoints of other K write unaligned rows and gain nothing (K = 13,
+    // 500 items of 399 nodes: 308 us, with both kinds 337, with gathers 287).
+    if (args.batch && args.input_paths && args.items >= 32 && warps >= kItemWarps &&
+        (kKind == kPhaseGather || args.states == KMAX)) {
+      constexpr unsigned per_block = kItemPhaseThreads / 32;
+      by_item<<<static_cast<unsigned>((warps + per_block - 1) / per_block), kItemPhaseThreads, 0,
+                stream>>>(args);
+      return cudaGetLastError();
+    }
+  }
   // One lane group per operation (finish: instance) and item.
   const std::uint64_t threads = static_cast<std::uint64_t>(args.count) * args.items * lanes;
   const std::uint64_t grid = (threads + kGroupPhaseThreads - 1) / kGroupPhaseThreads;

@@ -1090,6 +1090,7 @@ struct Workspace {
             tail_instances.begin()};
     const std::uint32_t grid_rounds = std::min(phase_rounds, phase.rounds);
     for (std::uint32_t r = 0; r < grid_rounds; ++r) {
+      args.input_paths = r == 0;
       launch(kPhaseGather, ranges.gather[r]);
       launch(kPhaseCompress, ranges.compress[r]);
     }
@@ -1099,6 +1100,7 @@ struct Workspace {
     if (operation == THMM_OP_MARGINALS) {
       launch(kPhaseTailReverse, tail);
       for (std::uint32_t r = grid_rounds; r-- > 0;) {
+        args.input_paths = r == 0;
         launch(kPhaseCompressReverse, ranges.compress[r]);
         launch(kPhaseRakeReverse, ranges.rake[r]);
       }
