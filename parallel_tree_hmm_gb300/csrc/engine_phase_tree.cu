@@ -8,8 +8,10 @@ template <typename Scalar, typename Compute, int K>
 cudaError_t LaunchTree(const TreePhaseArgs &args, cudaStream_t stream) {
   auto kernel = TreePhaseKernel<Scalar, Compute, K>;
   if (args.at.bytes > 48 * 1024) {
+    // The limit belongs to the kernel and not to the launch: every workspace and
+    // thread sets the same one, or one would lower it under another's launch.
     const cudaError_t status = cudaFuncSetAttribute(
-        kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(args.at.bytes));
+        kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTreePhaseMaxBytes));
     if (status != cudaSuccess)
       return status;
   }
