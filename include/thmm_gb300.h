@@ -335,9 +335,10 @@ thmm_status thmm_categorical_posterior_marginals(
  * only the device work of `operation` on the workspace stream, reading the
  * inputs left resident by the previous prepared call of the same workspace;
  * no host copies and no synchronisation. The step (work-counter memset and
- * kernel launches) is captured into a CUDA graph on its first use per
- * operation and batch and replayed afterwards; a new tuning or reservation
- * drops the graphs. `nodes_out` (optional) receives the number of tree nodes
+ * kernel launches) is built into a CUDA graph on its first use per operation
+ * and batch and replayed afterwards (with 256 graphs kept, once it has been
+ * enqueued nine times in a row); no stream is captured. A new tuning or
+ * reservation drops the graphs. `nodes_out` (optional) receives the number of tree nodes
  * processed. */
 thmm_status thmm_enqueue(thmm_workspace *workspace, int operation,
                          uint64_t *nodes_out);

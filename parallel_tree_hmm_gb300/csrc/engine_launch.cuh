@@ -11,7 +11,7 @@ namespace thmm {
 // when `blocks_per_sm` is non-null. Linear engines get one K*K scratch tile
 // per lane group in shared memory for the reverse sweep.
 template <class Engine, typename Buffer, bool kGroupTiles>
-cudaError_t LaunchOrQuery(const EngineArgs &args, int grid, cudaStream_t stream,
+cudaError_t LaunchOrQuery(const EngineArgs &args, int grid, LaunchStream stream,
                           int *blocks_per_sm) {
   // Group tiles are only used when several lanes share an operation.
   const std::size_t smem = kGroupTiles && Engine::G > 1
@@ -27,8 +27,7 @@ cudaError_t LaunchOrQuery(const EngineArgs &args, int grid, cudaStream_t stream,
   if (blocks_per_sm != nullptr)
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kernel,
                                                          kThreads, smem);
-  kernel<<<grid, kThreads, smem, stream>>>(args);
-  return cudaGetLastError();
+  return LaunchOn(stream, kernel, grid, kThreads, smem, args);
 }
 
 // Launches (or queries) the sum-product kernel of one part for padded state
@@ -36,7 +35,7 @@ cudaError_t LaunchOrQuery(const EngineArgs &args, int grid, cudaStream_t stream,
 // compiles in its own translation unit.
 template <typename Scalar, typename Compute, int kPart, bool kSmall>
 cudaError_t LaunchLinearHalf(unsigned kmax, const EngineArgs &args, int grid,
-                             cudaStream_t stream, int *blocks_per_sm) {
+                             LaunchStream stream, int *blocks_per_sm) {
   if constexpr (kSmall) {
     switch (kmax) {
     case 4:
@@ -70,7 +69,7 @@ cudaError_t LaunchLinearHalf(unsigned kmax, const EngineArgs &args, int grid,
 
 template <template <typename, int> class Engine, typename T>
 cudaError_t LaunchLogTyped(unsigned kmax, const EngineArgs &args, int grid,
-                           cudaStream_t stream, int *blocks_per_sm) {
+                           LaunchStream stream, int *blocks_per_sm) {
   switch (kmax) {
   case 4:
     return LaunchOrQuery<Engine<T, 4>, T, false>(args, grid, stream, blocks_per_sm);

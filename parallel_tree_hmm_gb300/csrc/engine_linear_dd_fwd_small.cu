@@ -6,7 +6,7 @@
 namespace thmm {
 
 cudaError_t LaunchLinearDDForwardSmall(unsigned kmax, const EngineArgs &args, int grid,
-                          cudaStream_t stream, int *blocks_per_sm) {
+                          LaunchStream stream, int *blocks_per_sm) {
   return LaunchLinearHalf<double, double, kLinearForward, true>(kmax, args, grid, stream, blocks_per_sm);
 }
 

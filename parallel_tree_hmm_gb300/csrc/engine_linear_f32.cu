@@ -7,7 +7,7 @@ namespace thmm {
 
 cudaError_t LaunchLinearF32(bool compute_f64, unsigned kmax, int part,
                             const EngineArgs &args, int grid,
-                            cudaStream_t stream, int *blocks_per_sm) {
+                            LaunchStream stream, int *blocks_per_sm) {
   if (kmax > 32)
     return compute_f64 ? cudaErrorInvalidValue
                        : LaunchWide(kmax, part, args, grid, stream, blocks_per_sm);

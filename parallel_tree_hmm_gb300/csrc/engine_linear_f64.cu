@@ -6,7 +6,7 @@ namespace thmm {
 
 cudaError_t LaunchLinearF64(bool compute_f64, unsigned kmax, int part,
                             const EngineArgs &args, int grid,
-                            cudaStream_t stream, int *blocks_per_sm) {
+                            LaunchStream stream, int *blocks_per_sm) {
   if (kmax > 32)
     return cudaErrorInvalidValue;
   const bool small = kmax <= 16;

@@ -6,7 +6,7 @@
 namespace thmm {
 
 cudaError_t LaunchLinearFFReverseLarge(unsigned kmax, const EngineArgs &args, int grid,
-                          cudaStream_t stream, int *blocks_per_sm) {
+                          LaunchStream stream, int *blocks_per_sm) {
   return LaunchLinearHalf<float, float, kLinearReverse, false>(kmax, args, grid, stream, blocks_per_sm);
 }
 

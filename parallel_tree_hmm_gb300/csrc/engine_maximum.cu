@@ -5,7 +5,7 @@
 namespace thmm {
 
 cudaError_t LaunchMaximum(int scalar_bytes, unsigned kmax,
-                          const EngineArgs &args, int grid, cudaStream_t stream,
+                          const EngineArgs &args, int grid, LaunchStream stream,
                           int *blocks_per_sm) {
   return scalar_bytes == 8 ? LaunchMaximumF64(kmax, args, grid, stream, blocks_per_sm)
                            : LaunchMaximumF32(kmax, args, grid, stream, blocks_per_sm);

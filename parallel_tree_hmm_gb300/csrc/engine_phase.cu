@@ -6,7 +6,7 @@ namespace thmm {
 namespace {
 
 template <typename Scalar, typename Compute, int kKind>
-cudaError_t LaunchKind(const PhaseArgs &args, cudaStream_t stream, int *blocks_per_sm) {
+cudaError_t LaunchKind(const PhaseArgs &args, LaunchStream stream, int *blocks_per_sm) {
   constexpr bool kTail = kKind == kPhaseTailForward || kKind == kPhaseTailReverse;
   if constexpr (!kTail) {
     if (args.batch) {
@@ -20,8 +20,7 @@ cudaError_t LaunchKind(const PhaseArgs &args, cudaStream_t stream, int *blocks_p
       const std::uint64_t grid = (threads + kPhaseThreads - 1) / kPhaseThreads;
       if (grid > 0x7fffffffull)
         return cudaErrorInvalidConfiguration;
-      kernel<<<static_cast<unsigned>(grid), kPhaseThreads, 0, stream>>>(args);
-      return cudaGetLastError();
+      return LaunchOn(stream, kernel, static_cast<unsigned>(grid), kPhaseThreads, 0, args);
     }
   } else if (args.batch) {
     return cudaErrorInvalidValue; // no tail in the shared-topology layout
@@ -37,12 +36,11 @@ cudaError_t LaunchKind(const PhaseArgs &args, cudaStream_t stream, int *blocks_p
     return cudaSuccess;
   const unsigned per_block = block_tail ? 1u : kTail ? kPhaseThreads / 32 : kPhaseThreads;
   const unsigned grid = (args.count + per_block - 1) / per_block;
-  kernel<<<grid, kPhaseThreads, 0, stream>>>(args);
-  return cudaGetLastError();
+  return LaunchOn(stream, kernel, grid, kPhaseThreads, 0, args);
 }
 
 template <typename Scalar, typename Compute>
-cudaError_t LaunchTyped(int kind, const PhaseArgs &args, cudaStream_t stream,
+cudaError_t LaunchTyped(int kind, const PhaseArgs &args, LaunchStream stream,
                         int *blocks_per_sm) {
   switch (kind) {
   case kPhaseGather:
@@ -93,7 +91,7 @@ cudaError_t LaunchObservationGather(const std::uint8_t *observations,
 }
 
 cudaError_t LaunchPhase(int scalar_bytes, bool compute_f64, int kind, const PhaseArgs &args,
-                        cudaStream_t stream, int *blocks_per_sm) {
+                        LaunchStream stream, int *blocks_per_sm) {
   if (args.states > 32)
     return scalar_bytes == 4 && !compute_f64 && !args.batch
                ? LaunchWidePhase(kind, args, stream, blocks_per_sm)

@@ -5,7 +5,7 @@
 namespace thmm {
 
 cudaError_t LaunchGroupPhase20F32(int scalar_bytes, int kind, const PhaseArgs &args,
-                                   cudaStream_t stream, int *blocks_per_sm) {
+                                   LaunchStream stream, int *blocks_per_sm) {
   return group_phase::Launch<float, 20>(scalar_bytes, kind, args, stream, blocks_per_sm);
 }
 

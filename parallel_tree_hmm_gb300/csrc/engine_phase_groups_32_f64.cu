@@ -4,7 +4,7 @@
 namespace thmm {
 
 cudaError_t LaunchGroupPhase32F64(int scalar_bytes, int kind, const PhaseArgs &args,
-                                   cudaStream_t stream, int *blocks_per_sm) {
+                                   LaunchStream stream, int *blocks_per_sm) {
   return group_phase::Launch<double, 32>(scalar_bytes, kind, args, stream, blocks_per_sm);
 }
 

@@ -3,7 +3,7 @@
 
 namespace thmm {
 
-cudaError_t LaunchPhaseSampleF32(int kind, const PhaseArgs &args, cudaStream_t stream) {
+cudaError_t LaunchPhaseSampleF32(int kind, const PhaseArgs &args, LaunchStream stream) {
   return LaunchLog<float, true>(kind, args, stream);
 }
 

@@ -3,7 +3,7 @@
 
 namespace thmm {
 
-cudaError_t LaunchPhaseSampleF64(int kind, const PhaseArgs &args, cudaStream_t stream) {
+cudaError_t LaunchPhaseSampleF64(int kind, const PhaseArgs &args, LaunchStream stream) {
   return LaunchLog<double, true>(kind, args, stream);
 }
 

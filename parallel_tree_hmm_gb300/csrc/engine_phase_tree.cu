@@ -5,7 +5,7 @@ namespace thmm {
 namespace {
 
 template <typename Scalar, typename Compute, int K>
-cudaError_t LaunchTree(const TreePhaseArgs &args, cudaStream_t stream) {
+cudaError_t LaunchTree(const TreePhaseArgs &args, LaunchStream stream) {
   auto kernel = TreePhaseKernel<Scalar, Compute, K>;
   if (args.at.bytes > 48 * 1024) {
     // The limit belongs to the kernel and not to the launch: every workspace and
@@ -17,12 +17,11 @@ cudaError_t LaunchTree(const TreePhaseArgs &args, cudaStream_t stream) {
   }
   if (args.phase.items == 0)
     return cudaSuccess;
-  kernel<<<args.phase.items, kTreePhaseThreads, args.at.bytes, stream>>>(args);
-  return cudaGetLastError();
+  return LaunchOn(stream, kernel, args.phase.items, kTreePhaseThreads, args.at.bytes, args);
 }
 
 template <typename Scalar, typename Compute>
-cudaError_t LaunchStates(const TreePhaseArgs &args, cudaStream_t stream) {
+cudaError_t LaunchStates(const TreePhaseArgs &args, LaunchStream stream) {
   switch (args.phase.states) {
   case 1:
     return LaunchTree<Scalar, Compute, 1>(args, stream);
@@ -40,7 +39,7 @@ cudaError_t LaunchStates(const TreePhaseArgs &args, cudaStream_t stream) {
 } // namespace
 
 cudaError_t LaunchTreePhase(int scalar_bytes, bool compute_f64, const TreePhaseArgs &args,
-                            cudaStream_t stream) {
+                            LaunchStream stream) {
   if (scalar_bytes == 8)
     return compute_f64 ? LaunchStates<double, double>(args, stream)
                        : LaunchStates<double, float>(args, stream);

@@ -5,7 +5,7 @@
 namespace thmm {
 
 cudaError_t LaunchSample(int scalar_bytes, unsigned kmax, const EngineArgs &args,
-                         int grid, cudaStream_t stream, int *blocks_per_sm) {
+                         int grid, LaunchStream stream, int *blocks_per_sm) {
   return scalar_bytes == 8 ? LaunchSampleF64(kmax, args, grid, stream, blocks_per_sm)
                            : LaunchSampleF32(kmax, args, grid, stream, blocks_per_sm);
 }

@@ -4,7 +4,7 @@
 
 namespace thmm {
 
-cudaError_t LaunchSampleF32(unsigned kmax, const EngineArgs &args, int grid, cudaStream_t stream,
+cudaError_t LaunchSampleF32(unsigned kmax, const EngineArgs &args, int grid, LaunchStream stream,
                  int *blocks_per_sm) {
   return LaunchLogTyped<SampleEngine, float>(kmax, args, grid, stream, blocks_per_sm);
 }

@@ -5,7 +5,7 @@
 namespace thmm {
 
 cudaError_t LaunchWide(unsigned kmax, int part, const EngineArgs &args, int grid,
-                       cudaStream_t stream, int *blocks_per_sm) {
+                       LaunchStream stream, int *blocks_per_sm) {
   switch (kmax) {
   case 64:
     return part == kLinearReverse

@@ -5,7 +5,7 @@ namespace thmm {
 namespace {
 
 template <int KP, int kKind>
-cudaError_t LaunchWideKind(const PhaseArgs &args, cudaStream_t stream, int *blocks_per_sm) {
+cudaError_t LaunchWideKind(const PhaseArgs &args, LaunchStream stream, int *blocks_per_sm) {
   constexpr bool kTensor = kKind == kPhaseCompress || kKind == kPhaseCompressReverse;
   using L = wide::PhaseLayout<KP>;
   auto kernel = wide::WidePhaseKernel<KP, kKind>;
@@ -41,12 +41,11 @@ cudaError_t LaunchWideKind(const PhaseArgs &args, cudaStream_t stream, int *bloc
   const std::uint64_t slots =
       static_cast<std::uint64_t>(sms) * static_cast<std::uint64_t>(per_sm > 0 ? per_sm : 1);
   const unsigned grid = static_cast<unsigned>(args.count < slots ? args.count : slots);
-  kernel<<<grid, L::kThreads, smem, stream>>>(args);
-  return cudaGetLastError();
+  return LaunchOn(stream, kernel, grid, L::kThreads, smem, args);
 }
 
 template <int KP>
-cudaError_t LaunchWideTyped(int kind, const PhaseArgs &args, cudaStream_t stream,
+cudaError_t LaunchWideTyped(int kind, const PhaseArgs &args, LaunchStream stream,
                             int *blocks_per_sm) {
   switch (kind) {
   case kPhaseGather:
@@ -70,7 +69,7 @@ cudaError_t LaunchWideTyped(int kind, const PhaseArgs &args, cudaStream_t stream
 
 } // namespace
 
-cudaError_t LaunchWidePhase(int kind, const PhaseArgs &args, cudaStream_t stream,
+cudaError_t LaunchWidePhase(int kind, const PhaseArgs &args, LaunchStream stream,
                             int *blocks_per_sm) {
   if (args.states > 32 && args.states <= 64)
     return LaunchWideTyped<64>(kind, args, stream, blocks_per_sm);

@@ -6,7 +6,7 @@ namespace thmm {
 namespace {
 
 template <int KP, bool kReverse>
-cudaError_t LaunchStreamKind(const PhaseArgs &args, cudaStream_t stream, int *blocks_per_sm) {
+cudaError_t LaunchStreamKind(const PhaseArgs &args, LaunchStream stream, int *blocks_per_sm) {
   using S = wide::StreamLayout<KP, kReverse>;
   const bool exact = args.states == KP;
   auto kernel = args.bf16 ? (exact ? wide::WideStreamKernel<KP, kReverse, true, true>
@@ -34,13 +34,12 @@ cudaError_t LaunchStreamKind(const PhaseArgs &args, cudaStream_t stream, int *bl
     return status;
   const std::uint64_t slots = static_cast<std::uint64_t>(sms) * S::kResident;
   const unsigned grid = static_cast<unsigned>(args.count < slots ? args.count : slots);
-  kernel<<<grid, S::kThreads, S::kBytes, stream>>>(args);
-  return cudaGetLastError();
+  return LaunchOn(stream, kernel, grid, S::kThreads, S::kBytes, args);
 }
 
 } // namespace
 
-cudaError_t LaunchWideStream(int kind, const PhaseArgs &args, cudaStream_t stream,
+cudaError_t LaunchWideStream(int kind, const PhaseArgs &args, LaunchStream stream,
                              int *blocks_per_sm) {
   const bool reverse = kind == kPhaseCompressReverse;
   if (args.states <= 64)

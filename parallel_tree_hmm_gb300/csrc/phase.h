@@ -37,6 +37,7 @@
 #include <cuda_runtime.h>
 
 #include "engine.h"
+#include "launch.h"
 #include "program_builder.h"
 
 namespace thmm {
@@ -174,7 +175,7 @@ struct TreePhaseArgs {
 inline constexpr unsigned kTreePhaseThreads = 512;
 inline constexpr std::uint64_t kTreePhaseMaxBytes = 226 * 1024;
 cudaError_t LaunchTreePhase(int scalar_bytes, bool compute_f64, const TreePhaseArgs &args,
-                            cudaStream_t stream);
+                            LaunchStream stream);
 
 // Operation counts of one program per round and kind.
 struct ProgramRounds {
@@ -243,16 +244,16 @@ PhasePlan BuildPhasePlan(const ProgramSet &set, std::span<const PhaseInstance> i
 // operation (phase_groups.cuh); 32 < K <= 128 (FP32 only, forest
 // layout, no tail kinds) one CTA per operation (wide_phase.cuh).
 cudaError_t LaunchPhase(int scalar_bytes, bool compute_f64, int kind, const PhaseArgs &args,
-                        cudaStream_t stream, int *blocks_per_sm);
-cudaError_t LaunchWidePhase(int kind, const PhaseArgs &args, cudaStream_t stream,
+                        LaunchStream stream, int *blocks_per_sm);
+cudaError_t LaunchWidePhase(int kind, const PhaseArgs &args, LaunchStream stream,
                             int *blocks_per_sm);
 // The compress kinds of K a multiple of 4 among those (wide_stream.cuh).
-cudaError_t LaunchWideStream(int kind, const PhaseArgs &args, cudaStream_t stream,
+cudaError_t LaunchWideStream(int kind, const PhaseArgs &args, LaunchStream stream,
                              int *blocks_per_sm);
 // 4 < K <= 32: one lane group per operation (phase_groups.cuh), per padded
 // state count and arithmetic type.
 #define THMM_GROUP_PHASE_LAUNCHER(name)                                                    \
-  cudaError_t name(int scalar_bytes, int kind, const PhaseArgs &args, cudaStream_t stream, \
+  cudaError_t name(int scalar_bytes, int kind, const PhaseArgs &args, LaunchStream stream, \
                    int *blocks_per_sm);
 THMM_GROUP_PHASE_LAUNCHER(LaunchGroupPhase8F32)
 THMM_GROUP_PHASE_LAUNCHER(LaunchGroupPhase8F64)
@@ -269,10 +270,10 @@ THMM_GROUP_PHASE_LAUNCHER(LaunchGroupPhase28F32)
 // (roots), the top-down kinds (kPhaseRakeReverse, kPhaseCompressReverse) and
 // kPhaseTailForward, which runs the last rounds, the root and the top-down
 // steps of those rounds in one CTA per tree (tail items of every tree).
-cudaError_t LaunchPhaseMaximumF32(int kind, const PhaseArgs &args, cudaStream_t stream);
-cudaError_t LaunchPhaseMaximumF64(int kind, const PhaseArgs &args, cudaStream_t stream);
-cudaError_t LaunchPhaseSampleF32(int kind, const PhaseArgs &args, cudaStream_t stream);
-cudaError_t LaunchPhaseSampleF64(int kind, const PhaseArgs &args, cudaStream_t stream);
+cudaError_t LaunchPhaseMaximumF32(int kind, const PhaseArgs &args, LaunchStream stream);
+cudaError_t LaunchPhaseMaximumF64(int kind, const PhaseArgs &args, LaunchStream stream);
+cudaError_t LaunchPhaseSampleF32(int kind, const PhaseArgs &args, LaunchStream stream);
+cudaError_t LaunchPhaseSampleF64(int kind, const PhaseArgs &args, LaunchStream stream);
 
 // The phase-ordered copy of the observations: ordered[j * items + b] =
 // observations[b * per_item + order[j]] for j < count, b < items (a forest:

@@ -19,7 +19,7 @@ namespace group_phase {
 // 200 items of 999 nodes 745 -> 686.
 constexpr std::uint64_t kItemWarps = 608;
 template <typename Scalar, typename Compute, int KMAX, int kKind>
-cudaError_t LaunchKind(const PhaseArgs &args, cudaStream_t stream, int *blocks_per_sm) {
+cudaError_t LaunchKind(const PhaseArgs &args, LaunchStream stream, int *blocks_per_sm) {
   // Single precision is bound by instruction issue (53-60 % of the issue
   // slots in the large rounds), which folded bounds shorten: a marginal step
   // of 256 trees of 5,000 nodes at K = 20 2,202 -> 2,141 us, 500 items on a
@@ -58,9 +58,8 @@ cudaError_t LaunchKind(const PhaseArgs &args, cudaStream_t stream, int *blocks_p
     if (args.batch && args.input_paths && args.items >= 32 && warps >= kItemWarps &&
         (kKind == kPhaseGather || args.states == KMAX)) {
       constexpr unsigned per_block = kItemPhaseThreads / 32;
-      by_item<<<static_cast<unsigned>((warps + per_block - 1) / per_block), kItemPhaseThreads, 0,
-                stream>>>(args);
-      return cudaGetLastError();
+      return LaunchOn(stream, by_item, static_cast<unsigned>((warps + per_block - 1) / per_block),
+                      kItemPhaseThreads, 0, args);
     }
   }
   // One lane group per operation (finish: instance) and item.
@@ -68,12 +67,11 @@ cudaError_t LaunchKind(const PhaseArgs &args, cudaStream_t stream, int *blocks_p
   const std::uint64_t grid = (threads + kGroupPhaseThreads - 1) / kGroupPhaseThreads;
   if (grid > 0x7fffffffull)
     return cudaErrorInvalidConfiguration;
-  kernel<<<static_cast<unsigned>(grid), kGroupPhaseThreads, smem, stream>>>(args);
-  return cudaGetLastError();
+  return LaunchOn(stream, kernel, static_cast<unsigned>(grid), kGroupPhaseThreads, smem, args);
 }
 
 template <typename Scalar, typename Compute, int KMAX>
-cudaError_t LaunchTyped(int kind, const PhaseArgs &args, cudaStream_t stream,
+cudaError_t LaunchTyped(int kind, const PhaseArgs &args, LaunchStream stream,
                         int *blocks_per_sm) {
   switch (kind) {
   case kPhaseGather:
@@ -95,7 +93,7 @@ cudaError_t LaunchTyped(int kind, const PhaseArgs &args, cudaStream_t stream,
 // Compute type fixed by the translation unit; scalar_bytes picks the
 // input/output type.
 template <typename Compute, int KMAX>
-cudaError_t Launch(int scalar_bytes, int kind, const PhaseArgs &args, cudaStream_t stream,
+cudaError_t Launch(int scalar_bytes, int kind, const PhaseArgs &args, LaunchStream stream,
                    int *blocks_per_sm) {
   return scalar_bytes == 8
              ? LaunchTyped<double, Compute, KMAX>(kind, args, stream, blocks_per_sm)

@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(kThreads, kThreads > kLogPhaseThreads      ? 1
 
 // ------------------------------------------------------------- launching
 template <typename T, int KMAX, bool kSample, int kKind>
-cudaError_t LaunchLogKind(const PhaseArgs &args, cudaStream_t stream) {
+cudaError_t LaunchLogKind(const PhaseArgs &args, LaunchStream stream) {
   constexpr bool kGroups = kKind == kPhaseGather || kKind == kPhaseCompress;
   std::uint64_t grid;
   if (kKind == kPhaseTailForward) {
@@ -683,9 +683,8 @@ cudaError_t LaunchLogKind(const PhaseArgs &args, cudaStream_t stream) {
   if constexpr (kKind == kPhaseTailForward) {
     constexpr int kWide = kLogTailThreads<T, KMAX>;
     if (grid <= kLogTailBlocks) {
-      LogPhaseKernel<T, KMAX, kSample, kKind, kWide, false>
-          <<<static_cast<unsigned>(grid), kWide, 0, stream>>>(args);
-      return cudaGetLastError();
+      return LaunchOn(stream, LogPhaseKernel<T, KMAX, kSample, kKind, kWide, false>,
+                      static_cast<unsigned>(grid), kWide, 0, args);
     }
   }
   // Folded bounds, K = 8 in single precision: MAP of the Galton-Watson forest
@@ -693,18 +692,16 @@ cudaError_t LaunchLogKind(const PhaseArgs &args, cudaStream_t stream) {
   // pipe, and K = 32 is not folded: it adds a fifth to the build for one size.
   if constexpr (kGroups && sizeof(T) == 4 && KMAX <= 20) {
     if (args.states == KMAX) {
-      LogPhaseKernel<T, KMAX, kSample, kKind, kLogPhaseThreads, true>
-          <<<static_cast<unsigned>(grid), kLogPhaseThreads, 0, stream>>>(args);
-      return cudaGetLastError();
+      return LaunchOn(stream, LogPhaseKernel<T, KMAX, kSample, kKind, kLogPhaseThreads, true>,
+                      static_cast<unsigned>(grid), kLogPhaseThreads, 0, args);
     }
   }
-  LogPhaseKernel<T, KMAX, kSample, kKind, kLogPhaseThreads, false>
-      <<<static_cast<unsigned>(grid), kLogPhaseThreads, 0, stream>>>(args);
-  return cudaGetLastError();
+  return LaunchOn(stream, LogPhaseKernel<T, KMAX, kSample, kKind, kLogPhaseThreads, false>,
+                  static_cast<unsigned>(grid), kLogPhaseThreads, 0, args);
 }
 
 template <typename T, int KMAX, bool kSample>
-cudaError_t LaunchLogStates(int kind, const PhaseArgs &args, cudaStream_t stream) {
+cudaError_t LaunchLogStates(int kind, const PhaseArgs &args, LaunchStream stream) {
   switch (kind) {
   case kPhaseGather:
     return LaunchLogKind<T, KMAX, kSample, kPhaseGather>(args, stream);
@@ -728,7 +725,7 @@ cudaError_t LaunchLogStates(int kind, const PhaseArgs &args, cudaStream_t stream
 // 2.6x the terms of a compression); terms past K are skipped by K, so every
 // padding gives the same bits.
 template <typename T, bool kSample>
-cudaError_t LaunchLog(int kind, const PhaseArgs &args, cudaStream_t stream) {
+cudaError_t LaunchLog(int kind, const PhaseArgs &args, LaunchStream stream) {
   if (args.states <= 4)
     return LaunchLogStates<T, 4, kSample>(kind, args, stream);
   if (args.states <= 8)

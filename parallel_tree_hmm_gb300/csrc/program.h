@@ -13,6 +13,7 @@
 
 #include "btrc/plan.h"
 #include "engine.h"
+#include "launch.h"
 #include "program_builder.h"
 
 namespace thmm {
@@ -58,22 +59,22 @@ ProgramSet BuildPrograms(std::span<const ProgramRequest> requests, bool categori
 // root marginal), 1 = adjoint sweep (marginals), launched in that order.
 cudaError_t LaunchLinearF32(bool compute_f64, unsigned kmax, int part,
                             const EngineArgs &args, int grid,
-                            cudaStream_t stream, int *blocks_per_sm);
+                            LaunchStream stream, int *blocks_per_sm);
 cudaError_t LaunchLinearF64(bool compute_f64, unsigned kmax, int part,
                             const EngineArgs &args, int grid,
-                            cudaStream_t stream, int *blocks_per_sm);
+                            LaunchStream stream, int *blocks_per_sm);
 cudaError_t LaunchMaximum(int scalar_bytes, unsigned kmax,
-                          const EngineArgs &args, int grid, cudaStream_t stream,
+                          const EngineArgs &args, int grid, LaunchStream stream,
                           int *blocks_per_sm);
 cudaError_t LaunchSample(int scalar_bytes, unsigned kmax, const EngineArgs &args,
-                         int grid, cudaStream_t stream, int *blocks_per_sm);
+                         int grid, LaunchStream stream, int *blocks_per_sm);
 
 // Per-instance launchers behind the dispatchers above, one translation unit
 // each (engine_linear_<scalar><compute>_<part>_<half>.cu for padded state
 // counts up to 16 (Small) or above (Large), engine_maximum_f*.cu,
 // engine_sample_f*.cu) so that the build compiles them in parallel.
 #define THMM_DECLARE_LAUNCHER(NAME)                                                  \
-  cudaError_t NAME(unsigned kmax, const EngineArgs &args, int grid, cudaStream_t stream, \
+  cudaError_t NAME(unsigned kmax, const EngineArgs &args, int grid, LaunchStream stream, \
                    int *blocks_per_sm);
 #define THMM_DECLARE_LINEAR(TYPES)                                                   \
   THMM_DECLARE_LAUNCHER(LaunchLinear##TYPES##ForwardSmall)                            \
@@ -93,7 +94,7 @@ THMM_DECLARE_LAUNCHER(LaunchSampleF64)
 
 // Tensor-core sum-product kernels for 32 < K <= 128 (kmax 64 or 128, FP32).
 cudaError_t LaunchWide(unsigned kmax, int part, const EngineArgs &args, int grid,
-                       cudaStream_t stream, int *blocks_per_sm);
+                       LaunchStream stream, int *blocks_per_sm);
 // One warp whose bounded mbarrier wait cannot complete and gives up after
 // `budget` cycles, setting kErrorTensorTimeout in *error.
 cudaError_t LaunchWaitTimeoutCheck(std::uint32_t *error, long long budget,

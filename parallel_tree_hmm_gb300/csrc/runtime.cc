@@ -37,6 +37,7 @@
 
 #include "btrc/plan.h"
 #include "engine.h"
+#include "launch.h"
 #include "phase.h"
 #include "program.h"
 
@@ -176,17 +177,18 @@ struct Workspace {
   float tuned_ms = 0.0f;
 
   // Instantiated CUDA graphs of the device step, per operation and batch (at
-  // most kMaxGraphs, the oldest given up first).
+  // most kMaxGraphs; EnqueueStep).
   struct Graph {
     int operation;
     std::size_t batch;
     cudaGraphExec_t exec;
     std::uint64_t launches;
+    std::uint64_t last_use;
   };
-  static constexpr std::size_t kMaxGraphs = 16;
+  static constexpr std::size_t kMaxGraphs = 256;
   std::vector<Graph> graphs;
-  // Consecutive prepared calls of one operation and batch, launched one by
-  // one before their graph is built (EnqueuePrepared).
+  std::uint64_t graph_uses = 0;
+  // Consecutive steps of one operation and batch.
   int repeated_operation = -1;
   std::size_t repeated_batch = 0;
   int repeats = 0;
@@ -769,7 +771,8 @@ struct Workspace {
   // Launches the kernels of `operation` over the queue set in `args`, with
   // work counters at counters[0..1] (forward) and counters[4..5] (adjoint);
   // the counters must be zero. Returns the number of kernel launches.
-  int LaunchTeams(int operation, EngineArgs args, std::uint32_t *counters) {
+  int LaunchTeams(int operation, EngineArgs args, std::uint32_t *counters,
+                  const LaunchStream &to) {
     const unsigned kmax = PaddedStates(states);
     args.queue = counters;
     const int kind = operation == THMM_OP_MAXIMUM ? 1
@@ -789,14 +792,14 @@ struct Workspace {
     cudaError_t status;
     int count = 1;
     if (kind == 1) {
-      status = LaunchMaximum(scalar, kmax, args, grid_for(1), stream, nullptr);
+      status = LaunchMaximum(scalar, kmax, args, grid_for(1), to, nullptr);
     } else if (kind == 2) {
-      status = LaunchSample(scalar, kmax, args, grid_for(2), stream, nullptr);
+      status = LaunchSample(scalar, kmax, args, grid_for(2), to, nullptr);
     } else {
       const auto linear = [&](int part, int grid) {
         return scalar == 8
-                   ? LaunchLinearF64(compute_f64, kmax, part, args, grid, stream, nullptr)
-                   : LaunchLinearF32(compute_f64, kmax, part, args, grid, stream, nullptr);
+                   ? LaunchLinearF64(compute_f64, kmax, part, args, grid, to, nullptr)
+                   : LaunchLinearF32(compute_f64, kmax, part, args, grid, to, nullptr);
       };
       status = linear(0, grid_for(0));
       if (status == cudaSuccess && args.reverse) {
@@ -953,7 +956,7 @@ struct Workspace {
   // Launches MAP or sampling over instances [a, b): gather and compress
   // phases of the grid-wide rounds, the tail (or the roots), then the
   // top-down phases in reverse round order. Returns the number of launches.
-  int LaunchLogPhases(int operation, std::uint32_t a, std::uint32_t b) {
+  int LaunchLogPhases(int operation, std::uint32_t a, std::uint32_t b, const LaunchStream &to) {
     const PhaseRanges &ranges = phase_batch ? PhaseRangesFor(0, 1) : PhaseRangesFor(a, b);
     PhaseArgs args = MakePhaseArgs(operation, a, b);
     const std::size_t K = states, S = ScalarBytes();
@@ -981,7 +984,7 @@ struct Workspace {
           operation == THMM_OP_MAXIMUM
               ? (scalar == 8 ? LaunchPhaseMaximumF64 : LaunchPhaseMaximumF32)
               : (scalar == 8 ? LaunchPhaseSampleF64 : LaunchPhaseSampleF32);
-      Check(launcher(kind, args, stream), "tree-HMM accelerator kernel launch");
+      Check(launcher(kind, args, to), "tree-HMM accelerator kernel launch");
       ++count;
     };
     for (std::uint32_t r = 0; r < log_rounds; ++r) {
@@ -1030,9 +1033,9 @@ struct Workspace {
   // gather and compress phases round by round, the finish phase, then (for
   // marginals) the adjoint phases in reverse round order. Returns the number
   // of kernel launches.
-  int LaunchPhases(int operation, std::uint32_t a, std::uint32_t b) {
+  int LaunchPhases(int operation, std::uint32_t a, std::uint32_t b, const LaunchStream &to) {
     if (IsLogDomain(operation))
-      return LaunchLogPhases(operation, a, b);
+      return LaunchLogPhases(operation, a, b, to);
     if (const auto layout = TreeLayout(operation, b - a)) {
       TreePhaseArgs tree{};
       tree.at = *layout;
@@ -1050,7 +1053,7 @@ struct Workspace {
       tree.observations = observations.as<std::uint8_t>();
       tree.observed_nodes = tree_observed.as<std::uint32_t>();
       tree.observed = static_cast<std::uint32_t>(observations_per_item);
-      Check(LaunchTreePhase(scalar, compute_f64, tree, stream),
+      Check(LaunchTreePhase(scalar, compute_f64, tree, to),
             "tree-HMM accelerator kernel launch");
       return 1;
     }
@@ -1078,7 +1081,7 @@ struct Workspace {
         return;
       args.offset = static_cast<std::uint32_t>(range.first);
       args.count = static_cast<std::uint32_t>(range.second - range.first);
-      Check(LaunchPhase(scalar, compute_f64, kind, args, stream, nullptr),
+      Check(LaunchPhase(scalar, compute_f64, kind, args, to, nullptr),
             "tree-HMM accelerator kernel launch");
       ++count;
     };
@@ -1108,8 +1111,9 @@ struct Workspace {
     return count;
   }
 
-  // One device step over all instances of the batch, on the workspace stream.
-  void EnqueueDevice(int operation, std::size_t batch) {
+  // One device step over all instances of the batch, on the workspace stream or
+  // into a graph.
+  void EnqueueDevice(int operation, std::size_t batch, const LaunchStream &to) {
     EngineArgs args = MakeArgs(operation);
     args.big_items = team_order.as<std::uint32_t>();
     args.small_items = team_order.as<std::uint32_t>() + big_count;
@@ -1121,11 +1125,12 @@ struct Workspace {
       args.small_count = items_big ? 0u : static_cast<std::uint32_t>(batch);
     }
     if (UsesControl(operation))
-      Check(cudaMemsetAsync(control.ptr, 0, 32, stream), "cudaMemsetAsync");
+      Check(ClearOn(to, control.ptr, 8), "cudaMemsetAsync");
     const auto items = static_cast<std::uint32_t>(forest ? capacity : batch);
     launches = static_cast<std::uint64_t>(
-        UsePhases(operation) ? LaunchPhases(operation, 0, items)
-                             : LaunchTeams(operation, args, control.as<std::uint32_t>()));
+        UsePhases(operation)
+            ? LaunchPhases(operation, 0, items, to)
+            : LaunchTeams(operation, args, control.as<std::uint32_t>(), to));
   }
 
   // Splits the largest-first queue at `threshold` nodes (CTA teams above).
@@ -1142,66 +1147,73 @@ struct Workspace {
     DropGraphs();
   }
 
-  // Device-only step replayed from a CUDA graph captured on first use (the
-  // memset of the work counters plus the kernel launches of EnqueueDevice).
-  void EnqueueGraph(int operation, std::size_t batch) {
-    for (const Graph &graph : graphs)
-      if (graph.operation == operation && graph.batch == batch) {
-        Check(cudaGraphLaunch(graph.exec, stream), "cudaGraphLaunch");
-        launches = graph.launches;
-        return;
-      }
-    if (graphs.size() >= kMaxGraphs) {
-      // Its last replay may still run.
-      Check(cudaStreamSynchronize(stream), "graph replay");
-      Check(cudaGraphExecDestroy(graphs.front().exec), "cudaGraphExecDestroy");
-      graphs.erase(graphs.begin());
-    }
-    cudaGraph_t graph = nullptr;
-    Check(cudaStreamBeginCapture(stream, cudaStreamCaptureModeRelaxed),
-          "cudaStreamBeginCapture");
-    try {
-      EnqueueDevice(operation, batch);
-    } catch (...) {
-      static_cast<void>(cudaStreamEndCapture(stream, &graph));
-      if (graph != nullptr)
-        static_cast<void>(cudaGraphDestroy(graph));
-      throw;
-    }
-    Check(cudaStreamEndCapture(stream, &graph), "cudaStreamEndCapture");
+  // The graph of the device step (the memset of the work counters, where a kernel
+  // uses them, and the launches of EnqueueDevice), built from these calls; null
+  // if it cannot be built.
+  Graph *BuildGraph(int operation, std::size_t batch) {
+    GraphChain chain;
     cudaGraphExec_t exec = nullptr;
-    const cudaError_t status = cudaGraphInstantiate(&exec, graph, 0);
-    static_cast<void>(cudaGraphDestroy(graph));
-    Check(status, "cudaGraphInstantiate");
-    graphs.push_back({operation, batch, exec, launches});
-    Check(cudaGraphLaunch(exec, stream), "cudaGraphLaunch");
+    cudaError_t status = cudaGraphCreate(&chain.graph, 0);
+    if (status == cudaSuccess) {
+      try {
+        EnqueueDevice(operation, batch, LaunchStream(&chain));
+        status = cudaGraphInstantiate(&exec, chain.graph, 0);
+      } catch (const std::runtime_error &) {
+        status = cudaErrorUnknown;
+      }
+    }
+    if (status != cudaSuccess) {
+      static_cast<void>(cudaGetLastError());
+      return nullptr;
+    }
+    if (graphs.size() >= kMaxGraphs) {
+      const auto oldest = std::min_element(
+          graphs.begin(), graphs.end(),
+          [](const Graph &x, const Graph &y) { return x.last_use < y.last_use; });
+      static_cast<void>(cudaStreamSynchronize(stream)); // its last replay may still run
+      static_cast<void>(cudaGraphExecDestroy(oldest->exec));
+      graphs.erase(oldest);
+    }
+    graphs.push_back({operation, batch, exec, launches, 0});
+    return &graphs.back();
   }
 
-  // The device step of a prepared call. Launching a chain of 20 to 100 small
-  // kernels one by one costs the host 2 to 3 us each, replaying its graph 10
-  // to 20 us in all (64 items of 999 nodes, K = 4, 29 launches: 219 -> 204 us a
-  // call; MAP of 48 trees, K = 8: 296 -> 290 us; fewer launches than
-  // kGraphLaunches: no gain, 85.6 against 87.4 us). Building the graph costs as
-  // much as some ten calls save, so it is built when an operation has been
-  // called kGraphAfter times in a row on one batch size.
+  // The device step of a call on the workspace stream: the replay of its graph,
+  // or its launches one by one. Launching a chain of 20 to 100 small kernels one
+  // by one costs the host 2 to 3 us each, replaying its graph 10 to 20 us in all
+  // (64 items of 999 nodes, K = 4, 29 launches: 219 -> 204 us a prepared call;
+  // MAP of 48 trees, K = 8: 296 -> 290 us; fewer launches than kGraphLaunches: no
+  // gain, 85.6 against 87.4 us). Building the graph costs as much as some ten
+  // calls save, so a prepared call builds it when an operation has been called
+  // kGraphAfter times in a row on one batch size, and so does thmm_enqueue
+  // (`enqueued`, which otherwise builds it at once) when kMaxGraphs are kept: a
+  // caller that goes round more of them has its first ones replayed and the
+  // others launched, with none built on each call.
   static constexpr int kGraphAfter = 8;
   static constexpr std::uint64_t kGraphLaunches = 8;
-  void EnqueuePrepared(int operation, std::size_t batch) {
+  void EnqueueStep(int operation, std::size_t batch, bool enqueued) {
     if (operation != repeated_operation || batch != repeated_batch) {
       repeated_operation = operation;
       repeated_batch = batch;
       repeats = 0;
     }
-    // A graph's own launch takes longer than a few kernels'.
-    bool replay = repeats >= kGraphAfter && launches >= kGraphLaunches;
-    for (const Graph &graph : graphs)
-      replay = replay || (graph.operation == operation && graph.batch == batch);
-    if (replay) {
-      EnqueueGraph(operation, batch);
-    } else {
-      ++repeats;
-      EnqueueDevice(operation, batch);
+    Graph *graph = nullptr;
+    for (Graph &kept : graphs)
+      if (kept.operation == operation && kept.batch == batch)
+        graph = &kept;
+    if (graph == nullptr) {
+      const bool repeated = repeats++ >= kGraphAfter;
+      if (enqueued ? repeated || graphs.size() < kMaxGraphs
+                   : repeated && launches >= kGraphLaunches) // of the last call
+        graph = BuildGraph(operation, batch);
     }
+    if (graph == nullptr) {
+      EnqueueDevice(operation, batch, stream);
+      return;
+    }
+    Check(cudaGraphLaunch(graph->exec, stream), "cudaGraphLaunch");
+    launches = graph->launches;
+    graph->last_use = ++graph_uses;
   }
 
   static int KernelSlot(int operation) {
@@ -1211,10 +1223,10 @@ struct Workspace {
   // Mean device time of `repeats` steps of `operation` on the resident
   // inputs, after one untimed step.
   float TimeSteps(int operation, int repeats) {
-    EnqueueDevice(operation, last_batch);
+    EnqueueDevice(operation, last_batch, stream);
     Check(cudaEventRecord(events[0], stream), "cudaEventRecord");
     for (int r = 0; r < repeats; ++r)
-      EnqueueDevice(operation, last_batch);
+      EnqueueDevice(operation, last_batch, stream);
     Check(cudaEventRecord(events[1], stream), "cudaEventRecord");
     Check(cudaEventSynchronize(events[1]), "autotune step");
     float ms = 0.0f;
@@ -1356,7 +1368,7 @@ struct Workspace {
       OrderObservations(stream);
     Check(cudaEventRecord(events[1], stream), "cudaEventRecord");
     Check(cudaEventRecord(events[2], stream), "cudaEventRecord");
-    EnqueuePrepared(operation, batch);
+    EnqueueStep(operation, batch, false);
     Check(cudaEventRecord(events[3], stream), "cudaEventRecord");
     Check(cudaEventRecord(events[4], stream), "cudaEventRecord");
     const std::size_t S = ScalarBytes();
@@ -1513,8 +1525,8 @@ struct Workspace {
       args.small_count = stripe.small;
       count += static_cast<std::uint64_t>(
           UsePhases(operation)
-              ? LaunchPhases(operation, stripe.first, stripe.last)
-              : LaunchTeams(operation, args, control.as<std::uint32_t>() + 8 + 8 * c));
+              ? LaunchPhases(operation, stripe.first, stripe.last, stream)
+              : LaunchTeams(operation, args, control.as<std::uint32_t>() + 8 + 8 * c, stream));
       Check(cudaEventRecord(computed[c], stream), "cudaEventRecord");
     }
     Check(cudaEventRecord(t[3], stream), "cudaEventRecord");
@@ -2207,7 +2219,7 @@ thmm_status thmm_enqueue(thmm_workspace *workspace, int operation,
         (operation == THMM_OP_MARGINALS && !ws.marginals))
       throw std::invalid_argument("operation was not reserved");
     thmm::Check(cudaSetDevice(ws.device), "cudaSetDevice");
-    ws.EnqueueGraph(operation, ws.last_batch);
+    ws.EnqueueStep(operation, ws.last_batch, true);
     if (nodes_out != nullptr)
       *nodes_out = ws.NodesFor(ws.last_batch);
   });

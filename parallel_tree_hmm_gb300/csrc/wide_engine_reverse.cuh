@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kThreads, Layout<KP>::kCtasPerSm) WideKernel(E
 }
 
 template <int KP, int kPart>
-cudaError_t LaunchWidePart(const EngineArgs &args, int grid, cudaStream_t stream,
+cudaError_t LaunchWidePart(const EngineArgs &args, int grid, LaunchStream stream,
                            int *blocks_per_sm) {
   auto kernel = WideKernel<KP, kPart>;
   const cudaError_t status = cudaFuncSetAttribute(
@@ -232,8 +232,7 @@ cudaError_t LaunchWidePart(const EngineArgs &args, int grid, cudaStream_t stream
   if (blocks_per_sm != nullptr)
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, kernel, kThreads,
                                                          Layout<KP>::kSmemBytes);
-  kernel<<<grid, kThreads, Layout<KP>::kSmemBytes, stream>>>(args);
-  return cudaGetLastError();
+  return LaunchOn(stream, kernel, grid, kThreads, Layout<KP>::kSmemBytes, args);
 }
 
 } // namespace wide
