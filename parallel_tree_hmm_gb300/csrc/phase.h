@@ -51,7 +51,13 @@ enum PhaseKind : int {
   kPhaseCompressReverse = 4, // adjoint of the round's compressions
   kPhaseTailForward = 5,     // rounds >= the tail round, one warp or block per tree
   kPhaseTailReverse = 6,     // their adjoint, one warp or block per tree
+  kPhaseWideGather = 7,      // MAP and sampling: gathers of more than kWideGather rakes
 };
+
+// Fan-in above which a MAP or sampling gather of a grid-wide round gets a block
+// of its own (kPhaseWideGather): a lane group takes its rakes one after the
+// other.
+inline constexpr std::uint32_t kWideGather = 16;
 
 // The last rounds of a forest hold few operations (rounds 5 and later of the
 // uneven K=4 forest hold 0.4 % of them) but one launch each, and a launch
@@ -118,6 +124,7 @@ struct PhaseArgs {
   // MAP and sampling kinds (phase_log.cuh) only; their values are in the
   // input precision.
   const uint2 *ends;         // [compression] parent and child node
+  const std::uint32_t *wide; // [wide gather] its gather
   void *branches;            // [rake][K] partial sums of wide gathers
   std::uint8_t *rake_choices; // [rake][K]
   std::uint8_t *comp_choices; // [compression][K][K]
@@ -193,6 +200,8 @@ struct PhasePlan {
   std::vector<Uint4> rakes, gathers, compress;
   std::vector<Uint2> roots;
   std::vector<Uint2> ends; // [compression] parent and child node
+  // Gathers of more than kWideGather rakes, ascending (MAP and sampling; runtime.cc).
+  std::vector<std::uint32_t> wide;
   // Whether every tree's exponent sum stays in int32 (the sum-product kinds).
   bool exponents_fit = false;
   // First operation of each round in the global arrays ([rounds + 1]).

@@ -12,6 +12,13 @@
 // merge once per trailing one bit of k; at the end, merge the remaining
 // partial sums from the newest to the oldest.
 //
+// The rakes of a gather are independent up to those sums. A group takes a few of
+// them one after the other; more than kWideGather of a grid-wide round get a block
+// of their own. A tail's block, which is short of operations and not of threads,
+// forms all messages of a round before the sums. One star at K = 4, MAP, a group
+// -> a block: 100 leaves 287 -> 52 us a call, 10,000 leaves 23.7 -> 0.15 ms (the
+// per-tree engine 74 and 420 us).
+//
 // What bounds them. A factor enters through a logarithm of some 45
 // instructions, and sampling adds an exponential per term, so at K = 8 the
 // kernels are bound by instruction issue and not by DRAM (a 256-byte edge
@@ -303,24 +310,77 @@ template <typename T, int KMAX, bool kSample, bool kExact> struct LogPhaseOps {
     return r < K ? *BranchAt(rake, r) : T(0);
   }
 
-  // Rakes, branch combinations and absorption of gather i.
-  __device__ __forceinline__ void Gather(std::uint32_t i) const {
-    const uint4 op = a.gathers[i];
+  // Rake `rake` alone: its message into the branch's scratch vector.
+  __device__ __forceinline__ void Rake(std::uint32_t rake) const {
+    const uint4 op = a.rakes[rake];
+    T leaf[KMAX];
+    NodeVector(op.y, op.z, false, leaf);
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+      const unsigned r = lane + q * G;
+      if (r < K)
+        *BranchAt(rake, r) = Message(rake, op, r, leaf);
+    }
+  }
+
+  // The node value that gather `op` adds its branches to, element r.
+  __device__ __forceinline__ T Previous(const uint4 &op, unsigned r) const {
+    const std::uint32_t node = op.x & kMask;
+    return (op.x & kFlag) ? PotentialLog(InputElement(node, op.y, (op.w & kRootBit) != 0, r))
+                          : static_cast<const T *>(a.nodes)[Store(node) * K + r];
+  }
+
+  // Branch combinations and absorption of gather `op`, whose messages lie in the
+  // branches' scratch, by the whole block of kThreads threads.
+  template <int kThreads> __device__ __forceinline__ void CombineByBlock(const uint4 &op) const {
+    const std::uint32_t count = op.w & kCountMask;
+    for (std::uint32_t s = 1; s < count; s *= 2) {
+      const std::size_t pairs = (static_cast<std::size_t>(count) + s - 1) / (2 * s);
+      for (std::size_t e = threadIdx.x; e < pairs * K; e += kThreads) {
+        const auto b = op.z + static_cast<std::uint32_t>(e / K) * 2 * s;
+        const unsigned r = static_cast<unsigned>(e % K);
+        *BranchAt(b, r) = *BranchAt(b, r) + *BranchAt(b + s, r);
+      }
+      __syncthreads();
+    }
+    for (unsigned r = threadIdx.x; r < K; r += kThreads)
+      static_cast<T *>(a.nodes)[Store(op.x & kMask) * K + r] = Previous(op, r) + *BranchAt(op.z, r);
+  }
+
+  // Gather `op` by the whole block: a rake per group at a time.
+  template <int kThreads> __device__ __forceinline__ void GatherByBlock(const uint4 &op) const {
+    const std::uint32_t count = op.w & kCountMask;
+    for (std::uint32_t k = threadIdx.x / G; k < count; k += kThreads / G)
+      Rake(op.z + k);
+    __syncthreads();
+    CombineByBlock<kThreads>(op);
+  }
+
+  // Rakes (kReady: their messages lie in the branches' scratch), branch
+  // combinations and absorption of gather `op` by one group.
+  template <bool kReady> __device__ __forceinline__ void Gather(const uint4 &op) const {
     const std::uint32_t node = op.x & kMask;
     const std::uint32_t count = op.w & kCountMask;
     // Binary counter of partial sums: the low levels in registers, the others
     // (fan-in of 32 and more) in the scratch of the gather's own branches,
-    // which has an entry per rake and so one per level.
+    // which has an entry per rake and so one per level (that rake's message has
+    // been added by then).
     T partial[kLevels][ROWS];
     for (std::uint32_t k = 0; k < count; ++k) {
-      const uint4 rake = a.rakes[op.z + k];
-      T leaf[KMAX];
-      NodeVector(rake.y, rake.z, false, leaf);
       T value[ROWS];
+      if constexpr (kReady) {
 #pragma unroll
-      for (int q = 0; q < ROWS; ++q) {
-        const unsigned r = lane + q * G;
-        value[q] = r < K ? Message(op.z + k, rake, r, leaf) : T(0);
+        for (int q = 0; q < ROWS; ++q)
+          value[q] = Branch(op.z + k, lane + q * G);
+      } else {
+        const uint4 rake = a.rakes[op.z + k];
+        T leaf[KMAX];
+        NodeVector(rake.y, rake.z, false, leaf);
+#pragma unroll
+        for (int q = 0; q < ROWS; ++q) {
+          const unsigned r = lane + q * G;
+          value[q] = r < K ? Message(op.z + k, rake, r, leaf) : T(0);
+        }
       }
       bool carry = true;
 #pragma unroll
@@ -373,13 +433,8 @@ template <typename T, int KMAX, bool kSample, bool kExact> struct LogPhaseOps {
 #pragma unroll
     for (int q = 0; q < ROWS; ++q) {
       const unsigned r = lane + q * G;
-      if (r < K) {
-        const T previous =
-            (op.x & kFlag)
-                ? PotentialLog(InputElement(node, op.y, (op.w & kRootBit) != 0, r))
-                : dst[r];
-        dst[r] = previous + sum[q];
-      }
+      if (r < K)
+        dst[r] = Previous(op, r) + sum[q];
     }
   }
 
@@ -596,6 +651,10 @@ inline constexpr int kLogTailThreads = sizeof(T) == 4 && KMAX <= 8    ? 512
                                                                       : kLogPhaseThreads;
 constexpr std::uint64_t kLogTailBlocks = 152; // SMs
 
+// Fan-in above which a tail's block forms a gather's sums together; its messages
+// lie in scratch already.
+constexpr std::uint32_t kWideCombine = 32;
+
 template <typename T, int KMAX, bool kSample, int kKind, int kThreads, bool kExact>
 __global__ void __launch_bounds__(kThreads, kThreads > kLogPhaseThreads      ? 1
                                             : KMAX <= 8 && sizeof(T) == 4 ? 4
@@ -613,9 +672,26 @@ __global__ void __launch_bounds__(kThreads, kThreads > kLogPhaseThreads      ? 1
     const unsigned group = threadIdx.x / G;
     for (std::uint32_t e = 0; e < tree.z; ++e) {
       const uint4 round = args.tail_rounds[tree.y + e];
-      for (std::uint32_t i = group; i < round.y; i += kThreads / G)
-        ops.Gather(round.x + i);
+      const uint2 rakes = args.tail_rakes[tree.y + e];
+      for (std::uint32_t i = group; i < rakes.y; i += kThreads / G)
+        ops.Rake(rakes.x + i);
       __syncthreads();
+      bool wide = false;
+      for (std::uint32_t i = group; i < round.y; i += kThreads / G) {
+        const uint4 op = args.gathers[round.x + i];
+        if ((op.w & kCountMask) > kWideCombine)
+          wide = true;
+        else
+          ops.template Gather<true>(op);
+      }
+      if (__syncthreads_or(wide)) {
+        for (std::uint32_t i = 0; i < round.y; ++i) {
+          const uint4 op = args.gathers[round.x + i];
+          if ((op.w & kCountMask) > kWideCombine)
+            ops.template CombineByBlock<kThreads>(op);
+        }
+        __syncthreads();
+      }
       if (round.w != 0) {
         for (std::uint32_t i = group; i < round.w; i += kThreads / G)
           ops.Compress(round.z + i);
@@ -637,6 +713,10 @@ __global__ void __launch_bounds__(kThreads, kThreads > kLogPhaseThreads      ? 1
         ops.ExpandRake(rakes.x + i);
       __syncthreads();
     }
+  } else if constexpr (kKind == kPhaseWideGather) {
+    const std::uint32_t op = args.batch ? blockIdx.x / args.items : blockIdx.x;
+    const Ops ops(args, args.batch ? args.first_item + blockIdx.x % args.items : 0u, tile);
+    ops.template GatherByBlock<kThreads>(args.gathers[args.wide[args.offset + op]]);
   } else {
     constexpr bool kGroups = kKind == kPhaseGather || kKind == kPhaseCompress;
     const std::uint32_t t =
@@ -651,9 +731,11 @@ __global__ void __launch_bounds__(kThreads, kThreads > kLogPhaseThreads      ? 1
       item = args.first_item + t % args.items;
     }
     const Ops ops(args, item, tile);
-    if constexpr (kKind == kPhaseGather)
-      ops.Gather(args.offset + op);
-    else if constexpr (kKind == kPhaseCompress)
+    if constexpr (kKind == kPhaseGather) {
+      const uint4 gather = args.gathers[args.offset + op];
+      if ((gather.w & kCountMask) <= kWideGather)
+        ops.template Gather<false>(gather);
+    } else if constexpr (kKind == kPhaseCompress)
       ops.Compress(args.offset + op);
     else if constexpr (kKind == kPhaseFinish)
       ops.Root(args.offset + op, args.batch ? item : args.offset + op);
@@ -671,6 +753,8 @@ cudaError_t LaunchLogKind(const PhaseArgs &args, LaunchStream stream) {
   std::uint64_t grid;
   if (kKind == kPhaseTailForward) {
     grid = args.batch ? args.items : args.count;
+  } else if (kKind == kPhaseWideGather) {
+    grid = static_cast<std::uint64_t>(args.count) * args.items;
   } else {
     const std::uint64_t threads = static_cast<std::uint64_t>(args.count) * args.items *
                                   (kGroups ? GroupLanes<KMAX>() : 1);
@@ -715,6 +799,8 @@ cudaError_t LaunchLogStates(int kind, const PhaseArgs &args, LaunchStream stream
     return LaunchLogKind<T, KMAX, kSample, kPhaseCompressReverse>(args, stream);
   case kPhaseTailForward:
     return LaunchLogKind<T, KMAX, kSample, kPhaseTailForward>(args, stream);
+  case kPhaseWideGather:
+    return LaunchLogKind<T, KMAX, kSample, kPhaseWideGather>(args, stream);
   default:
     return cudaErrorInvalidValue;
   }

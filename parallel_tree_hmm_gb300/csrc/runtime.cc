@@ -234,7 +234,7 @@ struct Workspace {
   // every tree; none of the tail records exist when every round is grid-wide.
   std::uint32_t log_rounds = 0;
   bool log_tail = false;
-  DeviceBuffer phase_ends, log_tail_items, log_tail_rounds, log_tail_rakes;
+  DeviceBuffer phase_ends, phase_wide, log_tail_items, log_tail_rounds, log_tail_rakes;
   // A whole tree per block (TreePhaseKernel): records of its rounds.
   DeviceBuffer tree_rounds, tree_rakes, tree_observed;
   // Phase-ordered copy of the observations (PhasePlan::observation_order),
@@ -297,6 +297,7 @@ struct Workspace {
           &compress_ends, &gathers, &team_order, &stripe_order, &control, &node_in,
           &phase_rakes, &phase_gathers, &phase_compress, &phase_roots, &node_exp,
           &comp_exp, &tail_items, &tail_rounds, &tail_rakes, &phase_ends,
+          &phase_wide,
           &tree_rounds, &tree_rakes, &tree_observed, &log_tail_items, &log_tail_rounds, &log_tail_rakes, &phase_observations,
           &observation_order, &edge_in,
           &observations, &root_potential, &emission, &uniforms, &values,
@@ -531,6 +532,10 @@ struct Workspace {
         }
         if (maximum || sampling) {
           phase_ends.Upload(phase.ends, stream);
+          for (std::size_t g = 0; g < phase.gathers.size(); ++g)
+            if ((phase.gathers[g].w & kCountMask) > kWideGather)
+              phase.wide.push_back(static_cast<std::uint32_t>(g));
+          phase_wide.Upload(phase.wide, stream);
           SetLogRounds();
         }
         node_exp.Allocate(total_nodes * sizeof(int));
@@ -967,6 +972,7 @@ struct Workspace {
     args.branches = work + total_nodes * K * S;
     args.comps = work + (total_nodes + rake_total) * K * S;
     args.ends = phase_ends.as<uint2>();
+    args.wide = phase_wide.as<std::uint32_t>();
     args.rake_choices = bytes.as<std::uint8_t>();
     args.comp_choices = bytes.as<std::uint8_t>() + rake_total * K;
     args.states_out = states_out.as<std::uint32_t>();
@@ -987,8 +993,15 @@ struct Workspace {
       Check(launcher(kind, args, to), "tree-HMM accelerator kernel launch");
       ++count;
     };
+    const auto wide_from = [&](std::uint64_t gather) {
+      return static_cast<std::uint64_t>(
+          std::lower_bound(phase.wide.begin(), phase.wide.end(), gather) - phase.wide.begin());
+    };
     for (std::uint32_t r = 0; r < log_rounds; ++r) {
       launch(kPhaseGather, ranges.gather[r]);
+      if (!phase.wide.empty())
+        launch(kPhaseWideGather,
+               {wide_from(ranges.gather[r].first), wide_from(ranges.gather[r].second)});
       launch(kPhaseCompress, ranges.compress[r]);
     }
     launch(log_tail ? kPhaseTailForward : kPhaseFinish,
