@@ -3,8 +3,9 @@
 
 namespace thmm {
 
-cudaError_t LaunchPhaseMaximumF64(int kind, const PhaseArgs &args, LaunchStream stream) {
-  return LaunchLog<double, false>(kind, args, stream);
+cudaError_t LaunchPhaseMaximumF64(int kind, const PhaseArgs &args, LaunchStream stream,
+                                  int *blocks_per_sm) {
+  return LaunchLog<double, false>(kind, args, stream, blocks_per_sm);
 }
 
 } // namespace thmm

@@ -3,8 +3,9 @@
 
 namespace thmm {
 
-cudaError_t LaunchPhaseSampleF32(int kind, const PhaseArgs &args, LaunchStream stream) {
-  return LaunchLog<float, true>(kind, args, stream);
+cudaError_t LaunchPhaseSampleF32(int kind, const PhaseArgs &args, LaunchStream stream,
+                                  int *blocks_per_sm) {
+  return LaunchLog<float, true>(kind, args, stream, blocks_per_sm);
 }
 
 } // namespace thmm

@@ -3,8 +3,9 @@
 
 namespace thmm {
 
-cudaError_t LaunchPhaseSampleF64(int kind, const PhaseArgs &args, LaunchStream stream) {
-  return LaunchLog<double, true>(kind, args, stream);
+cudaError_t LaunchPhaseSampleF64(int kind, const PhaseArgs &args, LaunchStream stream,
+                                  int *blocks_per_sm) {
+  return LaunchLog<double, true>(kind, args, stream, blocks_per_sm);
 }
 
 } // namespace thmm

@@ -112,6 +112,17 @@ std::uint32_t PhasePlan::AutoTailRound(std::uint64_t ops) const {
   return rounds;
 }
 
+std::uint32_t PhasePlan::TreeTailRound(std::uint64_t ops) const {
+  std::uint32_t first = 0;
+  for (const ProgramRounds &c : program_rounds) {
+    std::uint32_t r = c.rounds;
+    while (r > first && c.gathers[r - 1] + std::uint64_t{c.compressions[r - 1]} <= ops)
+      --r;
+    first = std::max(first, r);
+  }
+  return first;
+}
+
 PhasePlan BuildPhasePlan(const ProgramSet &set, std::span<const PhaseInstance> instances,
                          std::uint64_t total_nodes, std::uint64_t total_edges_out,
                          unsigned threads) {

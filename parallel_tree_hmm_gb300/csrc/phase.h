@@ -230,6 +230,8 @@ struct PhasePlan {
   // Default tail round: the first round with fewer than `ops` gathers and
   // compressions over all instances.
   std::uint32_t AutoTailRound(std::uint64_t ops) const;
+  // The first round from which no tree has more than `ops` gathers and compressions.
+  std::uint32_t TreeTailRound(std::uint64_t ops) const;
 };
 
 struct PhaseInstance {
@@ -279,10 +281,14 @@ THMM_GROUP_PHASE_LAUNCHER(LaunchGroupPhase28F32)
 // (roots), the top-down kinds (kPhaseRakeReverse, kPhaseCompressReverse) and
 // kPhaseTailForward, which runs the last rounds, the root and the top-down
 // steps of those rounds in one CTA per tree (tail items of every tree).
-cudaError_t LaunchPhaseMaximumF32(int kind, const PhaseArgs &args, LaunchStream stream);
-cudaError_t LaunchPhaseMaximumF64(int kind, const PhaseArgs &args, LaunchStream stream);
-cudaError_t LaunchPhaseSampleF32(int kind, const PhaseArgs &args, LaunchStream stream);
-cudaError_t LaunchPhaseSampleF64(int kind, const PhaseArgs &args, LaunchStream stream);
+cudaError_t LaunchPhaseMaximumF32(int kind, const PhaseArgs &args, LaunchStream stream,
+                                  int *blocks_per_sm);
+cudaError_t LaunchPhaseMaximumF64(int kind, const PhaseArgs &args, LaunchStream stream,
+                                  int *blocks_per_sm);
+cudaError_t LaunchPhaseSampleF32(int kind, const PhaseArgs &args, LaunchStream stream,
+                                 int *blocks_per_sm);
+cudaError_t LaunchPhaseSampleF64(int kind, const PhaseArgs &args, LaunchStream stream,
+                                 int *blocks_per_sm);
 
 // The phase-ordered copy of the observations: ordered[j * items + b] =
 // observations[b * per_item + order[j]] for j < count, b < items (a forest:

@@ -658,6 +658,7 @@ constexpr std::uint32_t kWideCombine = 32;
 template <typename T, int KMAX, bool kSample, int kKind, int kThreads, bool kExact>
 __global__ void __launch_bounds__(kThreads, kThreads > kLogPhaseThreads      ? 1
                                             : KMAX <= 8 && sizeof(T) == 4 ? 4
+                                            : KMAX <= 4                   ? 3
                                                                           : 2)
     LogPhaseKernel(PhaseArgs args) {
   using Ops = LogPhaseOps<T, KMAX, kSample, kExact>;
@@ -748,8 +749,12 @@ __global__ void __launch_bounds__(kThreads, kThreads > kLogPhaseThreads      ? 1
 
 // ------------------------------------------------------------- launching
 template <typename T, int KMAX, bool kSample, int kKind>
-cudaError_t LaunchLogKind(const PhaseArgs &args, LaunchStream stream) {
+cudaError_t LaunchLogKind(const PhaseArgs &args, LaunchStream stream, int *blocks_per_sm) {
   constexpr bool kGroups = kKind == kPhaseGather || kKind == kPhaseCompress;
+  if (blocks_per_sm != nullptr)
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        blocks_per_sm, LogPhaseKernel<T, KMAX, kSample, kKind, kLogPhaseThreads, false>,
+        kLogPhaseThreads, 0);
   std::uint64_t grid;
   if (kKind == kPhaseTailForward) {
     grid = args.batch ? args.items : args.count;
@@ -785,22 +790,22 @@ cudaError_t LaunchLogKind(const PhaseArgs &args, LaunchStream stream) {
 }
 
 template <typename T, int KMAX, bool kSample>
-cudaError_t LaunchLogStates(int kind, const PhaseArgs &args, LaunchStream stream) {
+cudaError_t LaunchLogStates(int kind, const PhaseArgs &args, LaunchStream stream, int *blocks_per_sm) {
   switch (kind) {
   case kPhaseGather:
-    return LaunchLogKind<T, KMAX, kSample, kPhaseGather>(args, stream);
+    return LaunchLogKind<T, KMAX, kSample, kPhaseGather>(args, stream, blocks_per_sm);
   case kPhaseCompress:
-    return LaunchLogKind<T, KMAX, kSample, kPhaseCompress>(args, stream);
+    return LaunchLogKind<T, KMAX, kSample, kPhaseCompress>(args, stream, blocks_per_sm);
   case kPhaseFinish:
-    return LaunchLogKind<T, KMAX, kSample, kPhaseFinish>(args, stream);
+    return LaunchLogKind<T, KMAX, kSample, kPhaseFinish>(args, stream, blocks_per_sm);
   case kPhaseRakeReverse:
-    return LaunchLogKind<T, KMAX, kSample, kPhaseRakeReverse>(args, stream);
+    return LaunchLogKind<T, KMAX, kSample, kPhaseRakeReverse>(args, stream, blocks_per_sm);
   case kPhaseCompressReverse:
-    return LaunchLogKind<T, KMAX, kSample, kPhaseCompressReverse>(args, stream);
+    return LaunchLogKind<T, KMAX, kSample, kPhaseCompressReverse>(args, stream, blocks_per_sm);
   case kPhaseTailForward:
-    return LaunchLogKind<T, KMAX, kSample, kPhaseTailForward>(args, stream);
+    return LaunchLogKind<T, KMAX, kSample, kPhaseTailForward>(args, stream, blocks_per_sm);
   case kPhaseWideGather:
-    return LaunchLogKind<T, KMAX, kSample, kPhaseWideGather>(args, stream);
+    return LaunchLogKind<T, KMAX, kSample, kPhaseWideGather>(args, stream, blocks_per_sm);
   default:
     return cudaErrorInvalidValue;
   }
@@ -811,18 +816,18 @@ cudaError_t LaunchLogStates(int kind, const PhaseArgs &args, LaunchStream stream
 // 2.6x the terms of a compression); terms past K are skipped by K, so every
 // padding gives the same bits.
 template <typename T, bool kSample>
-cudaError_t LaunchLog(int kind, const PhaseArgs &args, LaunchStream stream) {
+cudaError_t LaunchLog(int kind, const PhaseArgs &args, LaunchStream stream, int *blocks_per_sm) {
   if (args.states <= 4)
-    return LaunchLogStates<T, 4, kSample>(kind, args, stream);
+    return LaunchLogStates<T, 4, kSample>(kind, args, stream, blocks_per_sm);
   if (args.states <= 8)
-    return LaunchLogStates<T, 8, kSample>(kind, args, stream);
+    return LaunchLogStates<T, 8, kSample>(kind, args, stream, blocks_per_sm);
   if (args.states <= 16)
-    return LaunchLogStates<T, 16, kSample>(kind, args, stream);
+    return LaunchLogStates<T, 16, kSample>(kind, args, stream, blocks_per_sm);
   if constexpr (sizeof(T) == 4) {
     if (args.states <= 20)
-      return LaunchLogStates<T, 20, kSample>(kind, args, stream);
+      return LaunchLogStates<T, 20, kSample>(kind, args, stream, blocks_per_sm);
   }
-  return args.states <= 32 ? LaunchLogStates<T, 32, kSample>(kind, args, stream)
+  return args.states <= 32 ? LaunchLogStates<T, 32, kSample>(kind, args, stream, blocks_per_sm)
                            : cudaErrorInvalidValue;
 }
 

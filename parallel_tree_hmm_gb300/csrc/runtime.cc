@@ -230,10 +230,11 @@ struct Workspace {
   std::uint32_t phase_rounds = 0;
   DeviceBuffer tail_items, tail_rounds, tail_rakes;
   std::vector<std::uint32_t> tail_instances;
-  // MAP and sampling (phase_log.cuh): rounds run grid-wide, then the tail of
-  // every tree; none of the tail records exist when every round is grid-wide.
+  // MAP and sampling (phase_log.cuh): rounds run grid-wide before the tail of
+  // every tree, and the tail CTAs that the chip holds (MAP, sampling; 0: no tail
+  // records).
   std::uint32_t log_rounds = 0;
-  bool log_tail = false;
+  std::uint64_t log_tail_blocks[2] = {0, 0};
   DeviceBuffer phase_ends, phase_wide, log_tail_items, log_tail_rounds, log_tail_rakes;
   // A whole tree per block (TreePhaseKernel): records of its rounds.
   DeviceBuffer tree_rounds, tree_rakes, tree_observed;
@@ -289,7 +290,7 @@ struct Workspace {
     phase_rounds = 0;
     tail_instances.clear();
     log_rounds = 0;
-    log_tail = false;
+    log_tail_blocks[0] = log_tail_blocks[1] = 0;
     observation_reads = 0;
     phase_batch = false;
     for (DeviceBuffer *buffer :
@@ -884,28 +885,55 @@ struct Workspace {
            (IsLogDomain(operation) ? phase.enabled : LinearPhases());
   }
 
-  // Grid-wide rounds of MAP and sampling: up to the first round whose
-  // operations, shared out over the trees, are at most four passes of a CTA
-  // (512 threads' worth; 64 operations at 8 states). From there a grid-wide
-  // launch would do less than its own launch costs, and one CTA per tree runs
-  // the remaining rounds, the root and their top-down steps in one launch. At one
-  // (four, sixteen) passes: MAP of 48 trees of up to 6,000 nodes, K = 8, 273
-  // (257, 314) us, sampling of 320 trees of up to 50,000 nodes 1,943 (1,948,
-  // 1,984). A forest of more than 2^20 trees stays grid-wide (its tail records).
+  // Tails of MAP and sampling (one CTA per tree runs the last rounds, the root and
+  // their top-down steps in one launch), for calls whose trees fill the chip once
+  // at most: beyond that a tree would wait for the others' whole chains, and every
+  // round runs grid-wide (LogTail). Tails -> every round grid-wide, sampling at
+  // K = 4: 400 items of 15 nodes 96 -> 96 us, 2,048 210 -> 103, 16,384 1,117 ->
+  // 145.
+  // They start at the first round whose operations, shared out over the trees, are
+  // at most four passes of a CTA (512 threads' worth; 64 operations at 8 states),
+  // and the largest tree's at most four times that: a grid-wide launch would do less
+  // than its own launch costs. At one (four, sixteen) passes: MAP of 48 trees of up
+  // to 6,000 nodes, K = 8, 273 (257, 314) us, sampling of 320 trees of up to 50,000
+  // nodes 1,943 (1,948, 1,984). With the largest tree held to four passes as well:
+  // those 48 trees 274 us; with it not held: one tree of 50,000 nodes and 500 of 20
+  // 7,027 us, its CTA working alone.
   void SetLogRounds() {
     const std::uint64_t lanes = states <= 4 ? 1 : states <= 8 ? 8 : states <= 16 ? 16 : 32;
     const std::uint64_t trees = phase.instance_program.size(); // 1 in the batch layout
-    log_rounds = phase.AutoTailRound(trees * (512 / lanes) + 1);
-    log_tail = trees <= (1u << 20);
-    if (!log_tail) {
-      log_rounds = phase.rounds;
+    log_rounds = std::max(phase.AutoTailRound(trees * (512 / lanes) + 1),
+                          phase.TreeTailRound(4 * (512 / lanes)));
+    log_tail_blocks[0] = log_tail_blocks[1] = 0;
+    if (trees > (1u << 20)) // no tail records
       return;
+    PhaseArgs probe{};
+    probe.states = static_cast<std::uint32_t>(states);
+    for (const int operation : {THMM_OP_MAXIMUM, THMM_OP_SAMPLE}) {
+      if (!(operation == THMM_OP_MAXIMUM ? maximum : sampling))
+        continue;
+      int blocks = 0;
+      Check(LogLauncher(operation)(kPhaseTailForward, probe, nullptr, &blocks),
+            "occupancy query");
+      log_tail_blocks[operation == THMM_OP_SAMPLE] =
+          static_cast<std::uint64_t>(blocks) * static_cast<std::uint64_t>(sms);
     }
     const PhasePlan::Tail tail = phase.BuildTail(log_rounds, true);
     log_tail_items.Upload(tail.items, stream);
     log_tail_rounds.Upload(tail.rounds, stream);
     log_tail_rakes.Upload(tail.rakes, stream);
     Check(cudaStreamSynchronize(stream), "tail record upload");
+  }
+  auto LogLauncher(int operation) const
+      -> cudaError_t (*)(int, const PhaseArgs &, LaunchStream, int *) {
+    return operation == THMM_OP_MAXIMUM
+               ? (scalar == 8 ? LaunchPhaseMaximumF64 : LaunchPhaseMaximumF32)
+               : (scalar == 8 ? LaunchPhaseSampleF64 : LaunchPhaseSampleF32);
+  }
+  // Whether a launch of `operation` over `trees` trees (batch layout: items) has a
+  // tail.
+  bool LogTail(int operation, std::uint64_t trees) const {
+    return trees <= log_tail_blocks[operation == THMM_OP_SAMPLE];
   }
 
   const PhaseRanges &PhaseRangesFor(std::uint32_t a, std::uint32_t b) {
@@ -986,28 +1014,27 @@ struct Workspace {
         return;
       args.offset = static_cast<std::uint32_t>(range.first);
       args.count = static_cast<std::uint32_t>(range.second - range.first);
-      const auto launcher =
-          operation == THMM_OP_MAXIMUM
-              ? (scalar == 8 ? LaunchPhaseMaximumF64 : LaunchPhaseMaximumF32)
-              : (scalar == 8 ? LaunchPhaseSampleF64 : LaunchPhaseSampleF32);
-      Check(launcher(kind, args, to), "tree-HMM accelerator kernel launch");
+      Check(LogLauncher(operation)(kind, args, to, nullptr),
+            "tree-HMM accelerator kernel launch");
       ++count;
     };
     const auto wide_from = [&](std::uint64_t gather) {
       return static_cast<std::uint64_t>(
           std::lower_bound(phase.wide.begin(), phase.wide.end(), gather) - phase.wide.begin());
     };
-    for (std::uint32_t r = 0; r < log_rounds; ++r) {
+    const bool tail = LogTail(operation, b - a);
+    const std::uint32_t grid_rounds = tail ? log_rounds : phase.rounds;
+    for (std::uint32_t r = 0; r < grid_rounds; ++r) {
       launch(kPhaseGather, ranges.gather[r]);
       if (!phase.wide.empty())
         launch(kPhaseWideGather,
                {wide_from(ranges.gather[r].first), wide_from(ranges.gather[r].second)});
       launch(kPhaseCompress, ranges.compress[r]);
     }
-    launch(log_tail ? kPhaseTailForward : kPhaseFinish,
+    launch(tail ? kPhaseTailForward : kPhaseFinish,
            phase_batch ? std::pair<std::uint64_t, std::uint64_t>{0, 1}
                        : std::pair<std::uint64_t, std::uint64_t>{a, b});
-    for (std::uint32_t r = log_rounds; r-- > 0;) {
+    for (std::uint32_t r = grid_rounds; r-- > 0;) {
       launch(kPhaseCompressReverse, ranges.compress[r]);
       launch(kPhaseRakeReverse, ranges.rake[r]);
     }
