@@ -52,6 +52,8 @@ enum PhaseKind : int {
   kPhaseTailForward = 5,     // rounds >= the tail round, one warp or block per tree
   kPhaseTailReverse = 6,     // their adjoint, one warp or block per tree
   kPhaseWideGather = 7,      // MAP and sampling: gathers of more than kWideGather rakes
+  kPhaseRake = 8,            // MAP and sampling: a round's rakes apart from their sums
+  kPhaseReadyGather = 9,     // ... and the sums (the wide gathers': kPhaseWideGather)
 };
 
 // Fan-in above which a MAP or sampling gather of a grid-wide round gets a block
@@ -125,6 +127,7 @@ struct PhaseArgs {
   // input precision.
   const uint2 *ends;         // [compression] parent and child node
   const std::uint32_t *wide; // [wide gather] its gather
+  std::uint32_t ready;       // the messages of the wide gathers lie in scratch
   void *branches;            // [rake][K] partial sums of wide gathers
   std::uint8_t *rake_choices; // [rake][K]
   std::uint8_t *comp_choices; // [compression][K][K]
@@ -200,8 +203,9 @@ struct PhasePlan {
   std::vector<Uint4> rakes, gathers, compress;
   std::vector<Uint2> roots;
   std::vector<Uint2> ends; // [compression] parent and child node
-  // Gathers of more than kWideGather rakes, ascending (MAP and sampling; runtime.cc).
-  std::vector<std::uint32_t> wide;
+  // Gathers of more than kWideGather rakes, ascending, and each round's largest
+  // fan-in (MAP and sampling; runtime.cc).
+  std::vector<std::uint32_t> wide, fan_in;
   // Whether every tree's exponent sum stays in int32 (the sum-product kinds).
   bool exponents_fit = false;
   // First operation of each round in the global arrays ([rounds + 1]).

@@ -347,12 +347,15 @@ template <typename T, int KMAX, bool kSample, bool kExact> struct LogPhaseOps {
       static_cast<T *>(a.nodes)[Store(op.x & kMask) * K + r] = Previous(op, r) + *BranchAt(op.z, r);
   }
 
-  // Gather `op` by the whole block: a rake per group at a time.
+  // Gather `op` by the whole block: a rake per group at a time, unless the
+  // messages are ready.
   template <int kThreads> __device__ __forceinline__ void GatherByBlock(const uint4 &op) const {
     const std::uint32_t count = op.w & kCountMask;
-    for (std::uint32_t k = threadIdx.x / G; k < count; k += kThreads / G)
-      Rake(op.z + k);
-    __syncthreads();
+    if (a.ready == 0) {
+      for (std::uint32_t k = threadIdx.x / G; k < count; k += kThreads / G)
+        Rake(op.z + k);
+      __syncthreads();
+    }
     CombineByBlock<kThreads>(op);
   }
 
@@ -651,6 +654,11 @@ inline constexpr int kLogTailThreads = sizeof(T) == 4 && KMAX <= 8    ? 512
                                                                       : kLogPhaseThreads;
 constexpr std::uint64_t kLogTailBlocks = 152; // SMs
 
+// Kinds that run a lane group per operation.
+template <int kKind>
+inline constexpr bool kLogGroups = kKind == kPhaseGather || kKind == kPhaseCompress ||
+                                   kKind == kPhaseRake || kKind == kPhaseReadyGather;
+
 // Fan-in above which a tail's block forms a gather's sums together; its messages
 // lie in scratch already.
 constexpr std::uint32_t kWideCombine = 32;
@@ -719,7 +727,7 @@ __global__ void __launch_bounds__(kThreads, kThreads > kLogPhaseThreads      ? 1
     const Ops ops(args, args.batch ? args.first_item + blockIdx.x % args.items : 0u, tile);
     ops.template GatherByBlock<kThreads>(args.gathers[args.wide[args.offset + op]]);
   } else {
-    constexpr bool kGroups = kKind == kPhaseGather || kKind == kPhaseCompress;
+    constexpr bool kGroups = kLogGroups<kKind>;
     const std::uint32_t t =
         kGroups ? static_cast<std::uint32_t>(
                       (static_cast<std::uint64_t>(blockIdx.x) * kThreads + threadIdx.x) / G)
@@ -732,11 +740,13 @@ __global__ void __launch_bounds__(kThreads, kThreads > kLogPhaseThreads      ? 1
       item = args.first_item + t % args.items;
     }
     const Ops ops(args, item, tile);
-    if constexpr (kKind == kPhaseGather) {
+    if constexpr (kKind == kPhaseGather || kKind == kPhaseReadyGather) {
       const uint4 gather = args.gathers[args.offset + op];
       if ((gather.w & kCountMask) <= kWideGather)
-        ops.template Gather<false>(gather);
-    } else if constexpr (kKind == kPhaseCompress)
+        ops.template Gather<kKind == kPhaseReadyGather>(gather);
+    } else if constexpr (kKind == kPhaseRake)
+      ops.Rake(args.offset + op);
+    else if constexpr (kKind == kPhaseCompress)
       ops.Compress(args.offset + op);
     else if constexpr (kKind == kPhaseFinish)
       ops.Root(args.offset + op, args.batch ? item : args.offset + op);
@@ -750,7 +760,7 @@ __global__ void __launch_bounds__(kThreads, kThreads > kLogPhaseThreads      ? 1
 // ------------------------------------------------------------- launching
 template <typename T, int KMAX, bool kSample, int kKind>
 cudaError_t LaunchLogKind(const PhaseArgs &args, LaunchStream stream, int *blocks_per_sm) {
-  constexpr bool kGroups = kKind == kPhaseGather || kKind == kPhaseCompress;
+  constexpr bool kGroups = kLogGroups<kKind>;
   if (blocks_per_sm != nullptr)
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         blocks_per_sm, LogPhaseKernel<T, KMAX, kSample, kKind, kLogPhaseThreads, false>,
@@ -779,7 +789,8 @@ cudaError_t LaunchLogKind(const PhaseArgs &args, LaunchStream stream, int *block
   // Folded bounds, K = 8 in single precision: MAP of the Galton-Watson forest
   // 1,296 -> 1,222 us, sampling 2,069 -> 1,950 us. Double is bound by its
   // pipe, and K = 32 is not folded: it adds a fifth to the build for one size.
-  if constexpr (kGroups && sizeof(T) == 4 && KMAX <= 20) {
+  if constexpr ((kKind == kPhaseGather || kKind == kPhaseCompress) && sizeof(T) == 4 &&
+                KMAX <= 20) {
     if (args.states == KMAX) {
       return LaunchOn(stream, LogPhaseKernel<T, KMAX, kSample, kKind, kLogPhaseThreads, true>,
                       static_cast<unsigned>(grid), kLogPhaseThreads, 0, args);
@@ -806,6 +817,10 @@ cudaError_t LaunchLogStates(int kind, const PhaseArgs &args, LaunchStream stream
     return LaunchLogKind<T, KMAX, kSample, kPhaseTailForward>(args, stream, blocks_per_sm);
   case kPhaseWideGather:
     return LaunchLogKind<T, KMAX, kSample, kPhaseWideGather>(args, stream, blocks_per_sm);
+  case kPhaseRake:
+    return LaunchLogKind<T, KMAX, kSample, kPhaseRake>(args, stream, blocks_per_sm);
+  case kPhaseReadyGather:
+    return LaunchLogKind<T, KMAX, kSample, kPhaseReadyGather>(args, stream, blocks_per_sm);
   default:
     return cudaErrorInvalidValue;
   }

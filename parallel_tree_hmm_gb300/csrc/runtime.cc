@@ -533,9 +533,16 @@ struct Workspace {
         }
         if (maximum || sampling) {
           phase_ends.Upload(phase.ends, stream);
-          for (std::size_t g = 0; g < phase.gathers.size(); ++g)
-            if ((phase.gathers[g].w & kCountMask) > kWideGather)
-              phase.wide.push_back(static_cast<std::uint32_t>(g));
+          for (std::uint32_t r = 0; r < phase.rounds; ++r) {
+            std::uint32_t most = 0;
+            for (std::uint64_t g = phase.gather_base[r]; g < phase.gather_base[r + 1]; ++g) {
+              const std::uint32_t fan_in = phase.gathers[g].w & kCountMask;
+              most = std::max(most, fan_in);
+              if (fan_in > kWideGather)
+                phase.wide.push_back(static_cast<std::uint32_t>(g));
+            }
+            phase.fan_in.push_back(most);
+          }
           phase_wide.Upload(phase.wide, stream);
           SetLogRounds();
         }
@@ -924,6 +931,19 @@ struct Workspace {
     log_tail_rakes.Upload(tail.rakes, stream);
     Check(cudaStreamSynchronize(stream), "tail record upload");
   }
+  // Whether the rakes of round r are launched apart from the sums. A group takes a
+  // gather's rakes one after the other, at K = 4 some 2 us each in single precision
+  // and 30 in double, and a round of few gathers waits for the widest of them: up to
+  // 1,024 threads an SM, 128 in double, whose pipe is full then. Together -> apart,
+  // MAP of 2,048 stars of 14 leaves, K = 4, double 450 -> 136 us. Where the gathers
+  // fill the chip the messages' way through memory costs more than it saves (1,200
+  // items of 3 nodes, K = 20, double 174 -> 232).
+  bool SplitRound(std::uint32_t r, std::uint64_t gathers) const {
+    const std::uint64_t lanes = states <= 4 ? 1 : states <= 8 ? 8 : states <= 16 ? 16 : 32;
+    const std::uint64_t threads = gathers * lanes, chip = static_cast<std::uint64_t>(sms);
+    return scalar == 8 ? phase.fan_in[r] > 1 && threads <= 128 * chip
+                       : phase.fan_in[r] > 4 && threads <= 1024 * chip;
+  }
   auto LogLauncher(int operation) const
       -> cudaError_t (*)(int, const PhaseArgs &, LaunchStream, int *) {
     return operation == THMM_OP_MAXIMUM
@@ -1025,7 +1045,11 @@ struct Workspace {
     const bool tail = LogTail(operation, b - a);
     const std::uint32_t grid_rounds = tail ? log_rounds : phase.rounds;
     for (std::uint32_t r = 0; r < grid_rounds; ++r) {
-      launch(kPhaseGather, ranges.gather[r]);
+      const std::uint64_t gathers = ranges.gather[r].second - ranges.gather[r].first;
+      args.ready = SplitRound(r, gathers * args.items);
+      if (args.ready)
+        launch(kPhaseRake, ranges.rake[r]);
+      launch(args.ready ? kPhaseReadyGather : kPhaseGather, ranges.gather[r]);
       if (!phase.wide.empty())
         launch(kPhaseWideGather,
                {wide_from(ranges.gather[r].first), wide_from(ranges.gather[r].second)});
