@@ -900,17 +900,19 @@ struct Workspace {
   // 145.
   // They start at the first round whose operations, shared out over the trees, are
   // at most four passes of a CTA (512 threads' worth; 64 operations at 8 states),
-  // and the largest tree's at most four times that: a grid-wide launch would do less
-  // than its own launch costs. At one (four, sixteen) passes: MAP of 48 trees of up
-  // to 6,000 nodes, K = 8, 273 (257, 314) us, sampling of 320 trees of up to 50,000
-  // nodes 1,943 (1,948, 1,984). With the largest tree held to four passes as well:
-  // those 48 trees 274 us; with it not held: one tree of 50,000 nodes and 500 of 20
-  // 7,027 us, its CTA working alone.
+  // and so are the largest tree's (four times as many where the CTAs have 512 or 256
+  // threads): a grid-wide launch would do less than its own launch costs. At one
+  // (four, sixteen) passes: MAP of 48 trees of up to 6,000 nodes, K = 8, 273 (257,
+  // 314) us, sampling of 320 trees of up to 50,000 nodes 1,943 (1,948, 1,984). With
+  // those 48 trees' largest held to a quarter: 274 us; four of 20,000 nodes and 300
+  // of 50, K = 4, CTAs of 128 threads, with the largest held to four times as many
+  // 266 us, without 243; one of 50,000 and 500 of 20, K = 8, not held 7,027, held 256.
   void SetLogRounds() {
     const std::uint64_t lanes = states <= 4 ? 1 : states <= 8 ? 8 : states <= 16 ? 16 : 32;
     const std::uint64_t trees = phase.instance_program.size(); // 1 in the batch layout
+    const bool wide = trees <= static_cast<std::uint64_t>(sms) && scalar == 4 && states <= 20;
     log_rounds = std::max(phase.AutoTailRound(trees * (512 / lanes) + 1),
-                          phase.TreeTailRound(4 * (512 / lanes)));
+                          phase.TreeTailRound((wide ? 4 : 1) * (512 / lanes)));
     log_tail_blocks[0] = log_tail_blocks[1] = 0;
     if (trees > (1u << 20)) // no tail records
       return;
