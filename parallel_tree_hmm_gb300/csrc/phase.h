@@ -128,6 +128,7 @@ struct PhaseArgs {
   const uint2 *ends;         // [compression] parent and child node
   const std::uint32_t *wide; // [wide gather] its gather
   std::uint32_t ready;       // the messages of the wide gathers lie in scratch
+  std::uint32_t narrow;      // tail blocks of one warp (K <= 4)
   void *branches;            // [rake][K] partial sums of wide gathers
   std::uint8_t *rake_choices; // [rake][K]
   std::uint8_t *comp_choices; // [compression][K][K]

@@ -665,6 +665,7 @@ constexpr std::uint32_t kWideCombine = 32;
 
 template <typename T, int KMAX, bool kSample, int kKind, int kThreads, bool kExact>
 __global__ void __launch_bounds__(kThreads, kThreads > kLogPhaseThreads      ? 1
+                                            : kThreads < kLogPhaseThreads ? 12
                                             : KMAX <= 8 && sizeof(T) == 4 ? 4
                                             : KMAX <= 4                   ? 3
                                                                           : 2)
@@ -761,6 +762,12 @@ __global__ void __launch_bounds__(kThreads, kThreads > kLogPhaseThreads      ? 1
 template <typename T, int KMAX, bool kSample, int kKind>
 cudaError_t LaunchLogKind(const PhaseArgs &args, LaunchStream stream, int *blocks_per_sm) {
   constexpr bool kGroups = kLogGroups<kKind>;
+  constexpr bool kNarrow = kKind == kPhaseTailForward && KMAX == 4 && sizeof(T) == 4;
+  if constexpr (kNarrow) {
+    if (blocks_per_sm != nullptr && args.narrow)
+      return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+          blocks_per_sm, LogPhaseKernel<T, KMAX, kSample, kKind, 32, false>, 32, 0);
+  }
   if (blocks_per_sm != nullptr)
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         blocks_per_sm, LogPhaseKernel<T, KMAX, kSample, kKind, kLogPhaseThreads, false>,
@@ -779,6 +786,11 @@ cudaError_t LaunchLogKind(const PhaseArgs &args, LaunchStream stream, int *block
     return cudaSuccess;
   if (grid > 0x7fffffffull)
     return cudaErrorInvalidConfiguration;
+  if constexpr (kNarrow) {
+    if (args.narrow)
+      return LaunchOn(stream, LogPhaseKernel<T, KMAX, kSample, kKind, 32, false>,
+                      static_cast<unsigned>(grid), 32, 0, args);
+  }
   if constexpr (kKind == kPhaseTailForward) {
     constexpr int kWide = kLogTailThreads<T, KMAX>;
     if (grid <= kLogTailBlocks) {

@@ -235,6 +235,7 @@ struct Workspace {
   // records).
   std::uint32_t log_rounds = 0;
   std::uint64_t log_tail_blocks[2] = {0, 0};
+  std::uint64_t log_narrow_blocks[2] = {0, 0}; // of one warp (0: not for these trees)
   DeviceBuffer phase_ends, phase_wide, log_tail_items, log_tail_rounds, log_tail_rakes;
   // A whole tree per block (TreePhaseKernel): records of its rounds.
   DeviceBuffer tree_rounds, tree_rakes, tree_observed;
@@ -291,6 +292,7 @@ struct Workspace {
     tail_instances.clear();
     log_rounds = 0;
     log_tail_blocks[0] = log_tail_blocks[1] = 0;
+    log_narrow_blocks[0] = log_narrow_blocks[1] = 0;
     observation_reads = 0;
     phase_batch = false;
     for (DeviceBuffer *buffer :
@@ -914,6 +916,7 @@ struct Workspace {
     log_rounds = std::max(phase.AutoTailRound(trees * (512 / lanes) + 1),
                           phase.TreeTailRound((wide ? 4 : 1) * (512 / lanes)));
     log_tail_blocks[0] = log_tail_blocks[1] = 0;
+    log_narrow_blocks[0] = log_narrow_blocks[1] = 0;
     if (trees > (1u << 20)) // no tail records
       return;
     PhaseArgs probe{};
@@ -921,11 +924,15 @@ struct Workspace {
     for (const int operation : {THMM_OP_MAXIMUM, THMM_OP_SAMPLE}) {
       if (!(operation == THMM_OP_MAXIMUM ? maximum : sampling))
         continue;
-      int blocks = 0;
-      Check(LogLauncher(operation)(kPhaseTailForward, probe, nullptr, &blocks),
-            "occupancy query");
-      log_tail_blocks[operation == THMM_OP_SAMPLE] =
-          static_cast<std::uint64_t>(blocks) * static_cast<std::uint64_t>(sms);
+      for (probe.narrow = 0; probe.narrow < 2; ++probe.narrow) {
+        if (probe.narrow && (scalar == 8 || states > 4 || sorted_nodes.front() > 256))
+          break;
+        int blocks = 0;
+        Check(LogLauncher(operation)(kPhaseTailForward, probe, nullptr, &blocks),
+              "occupancy query");
+        (probe.narrow ? log_narrow_blocks : log_tail_blocks)[operation == THMM_OP_SAMPLE] =
+            static_cast<std::uint64_t>(blocks) * static_cast<std::uint64_t>(sms);
+      }
     }
     const PhasePlan::Tail tail = phase.BuildTail(log_rounds, true);
     log_tail_items.Upload(tail.items, stream);
@@ -953,9 +960,15 @@ struct Workspace {
                : (scalar == 8 ? LaunchPhaseSampleF64 : LaunchPhaseSampleF32);
   }
   // Whether a launch of `operation` over `trees` trees (batch layout: items) has a
-  // tail.
-  bool LogTail(int operation, std::uint64_t trees) const {
-    return trees <= log_tail_blocks[operation == THMM_OP_SAMPLE];
+  // tail. More trees than CTAs of four warps have one of a warp each in single
+  // precision up to 4 states and 256 nodes, where a round's operations are a few
+  // passes of a warp and cost less than the round's launches: MAP at K = 2, 2,048
+  // items of 63 (255) nodes 114 -> 86 (154 -> 142) us; in double, whose pipe a few
+  // lanes of a warp keep busy, sampling at K = 4, 1,200 items of 15 447 -> 666.
+  bool LogTail(int operation, std::uint64_t trees, std::uint32_t &narrow) const {
+    const int slot = operation == THMM_OP_SAMPLE;
+    narrow = trees > log_tail_blocks[slot];
+    return trees <= (narrow ? log_narrow_blocks : log_tail_blocks)[slot];
   }
 
   const PhaseRanges &PhaseRangesFor(std::uint32_t a, std::uint32_t b) {
@@ -1044,7 +1057,7 @@ struct Workspace {
       return static_cast<std::uint64_t>(
           std::lower_bound(phase.wide.begin(), phase.wide.end(), gather) - phase.wide.begin());
     };
-    const bool tail = LogTail(operation, b - a);
+    const bool tail = LogTail(operation, b - a, args.narrow);
     const std::uint32_t grid_rounds = tail ? log_rounds : phase.rounds;
     for (std::uint32_t r = 0; r < grid_rounds; ++r) {
       const std::uint64_t gathers = ranges.gather[r].second - ranges.gather[r].first;
