@@ -1081,16 +1081,20 @@ struct Workspace {
   }
 
   // Whether `items` items of a batch workspace run a whole tree per block, and
-  // the shared memory of a block: the tree fits, the blocks are at most three
-  // waves of the chip, and either a tree's rounds are one pass of the block (512
-  // nodes) or there are 32 items and more. Measured, a launch per round and kind
-  // -> a block per item, marginals at K = 4: 32 to 152 items of 999 nodes 96 to
-  // 111 -> 27 us, 608 (two waves) 121 -> 96, 1,216 (four) 164 -> 188; 399 nodes,
-  // 1,216 items (under three waves) 100 -> 76, 2,432 125 -> 146; 99 nodes, 1,216
-  // items (two) 66 -> 51, 2,432 (four) 72 -> 100. A few larger trees would gain
-  // as well (8 items of 999 nodes, 98 -> 27), but the one launch per round and
-  // kind of such a batch is what thmm_workspace_launches has reported, and is
-  // kept.
+  // the shared memory of a block: the tree fits, either its rounds are one pass of
+  // the block (512 nodes) or there are 32 items and more, and the blocks, each a
+  // chain of its own, are few enough that their waves cost less than the launches
+  // they save, which are few for a tree of two or three rounds. A block's chain is
+  // longer in FP64, where at most three blocks an SM gain (two up to two rounds);
+  // in FP32 eight do (four up to three rounds), of large trees three waves. Measured,
+  // a launch per round and kind -> a block per item, marginals at K = 4, FP32: 32 to
+  // 152 items of 999 nodes 96 to 111 -> 27 us; 61 nodes, 152 (1,216, 1,824) items
+  // -41 (-9, +7) %, 3 nodes, 608 (760, 1,824) items -1 (+12, +35) %; FP64: 61 nodes,
+  // 456 (608, 1,824) items -22 (-9, +78) %, 3 nodes, 304 (456) items +1 (+13) %;
+  // log Z: the same lines within a few per cent, but one round is no gain (3 nodes,
+  // 32 items 47 -> 50 us). A few larger trees would gain as well (8 items of 999
+  // nodes, 98 -> 27), but the one launch per round and kind of such a batch is what
+  // thmm_workspace_launches has reported, and is kept.
   std::optional<TreePhaseLayout> TreeLayout(int operation, std::uint64_t items) const {
     if (!phase_batch || states > 4 || (nodes_per_item > 512 && items < 32))
       return std::nullopt;
@@ -1103,7 +1107,10 @@ struct Workspace {
       return std::nullopt;
     const std::uint64_t resident =
         std::min<std::uint64_t>(2048 / kTreePhaseThreads, 228 * 1024 / (at.bytes + 2048));
-    if (items > 3 * resident * static_cast<std::uint64_t>(sms))
+    const std::uint64_t per_sm =
+        compute_f64 ? (phase.rounds > 2 ? 3 : 2) : (phase.rounds > 3 ? 8 : 4);
+    if (phase.rounds < (operation == THMM_OP_MARGINALS ? 1u : 2u) ||
+        items > std::min(3 * resident, per_sm) * static_cast<std::uint64_t>(sms))
       return std::nullopt;
     return at;
   }
