@@ -102,14 +102,15 @@ __device__ __forceinline__ void Store4(D *p, const T (&in)[4]) {
   }
 }
 
-// Asynchronous global -> shared copies of 16 (4, 8) bytes.
+// Asynchronous global -> shared copies of 4, 8 or 16 bytes, through L1: in the
+// batch layout every group of an SM reads the same few matrices, and past L1 (.cg)
+// all SMs queue for the same lines of L2. The one gather launch of 8,192 items of 3
+// nodes at K = 8: 51.6 -> 5.5 us.
 template <int kBytes> __device__ __forceinline__ void CopyAsync(void *dst, const void *src) {
-  const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-  if constexpr (kBytes == 16)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at), "l"(src) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(at), "l"(src), "n"(kBytes)
-                 : "memory");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                   static_cast<unsigned>(__cvta_generic_to_shared(dst))),
+               "l"(src), "n"(kBytes)
+               : "memory");
 }
 __device__ __forceinline__ void CopyCommit() {
   asm volatile("cp.async.commit_group;" ::: "memory");
