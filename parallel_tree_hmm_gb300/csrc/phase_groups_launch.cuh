@@ -62,8 +62,9 @@ cudaError_t LaunchKind(const PhaseArgs &args, LaunchStream stream, int *blocks_p
                       kItemPhaseThreads, 0, args);
     }
   }
-  // One lane group per operation (finish: instance) and item.
-  const std::uint64_t threads = static_cast<std::uint64_t>(args.count) * args.items * lanes;
+  // One lane group per operation (finish: instance, or a thread) and item.
+  const std::uint64_t threads = static_cast<std::uint64_t>(args.count) * args.items *
+                                (kKind == kPhaseFinish && !args.reverse ? 1u : lanes);
   const std::uint64_t grid = (threads + kGroupPhaseThreads - 1) / kGroupPhaseThreads;
   if (grid > 0x7fffffffull)
     return cudaErrorInvalidConfiguration;
