@@ -26,7 +26,7 @@ cudaError_t LaunchKind(const PhaseArgs &args, LaunchStream stream, int *blocks_p
     return cudaErrorInvalidValue; // no tail in the shared-topology layout
   }
   // One thread per operation, or one warp or block per tree for the tails.
-  const bool block_tail = kTail && args.count < kTailBlockTrees;
+  const bool block_tail = kTail && args.count <= kTailBlockTrees<Compute, kKind>;
   auto kernel = block_tail ? PhaseKernel<Scalar, Compute, kKind, kTail ? kPhaseThreads : 1>
                            : PhaseKernel<Scalar, Compute, kKind, kTail ? 32 : 1>;
   if (blocks_per_sm != nullptr)

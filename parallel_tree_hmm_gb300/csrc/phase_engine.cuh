@@ -557,11 +557,18 @@ struct PhaseOps {
 // Tail rounds of one tree per team of kTeam threads (kPhaseTailForward /
 // kPhaseTailReverse): a warp or a block, whose threads take the operations of
 // a step in turn, with a barrier (which also orders their global-memory
-// accesses) between steps. With many trees a warp each fills the chip; below
+// accesses) between steps. With many trees a warp each fills the chip; up to
 // kTailBlockTrees a block each does, and a step of a large tree takes a
-// quarter of the passes. Measured, warps -> blocks: marginals of 512 trees in
-// double precision 551 -> 465 us, of 4,096 trees (K = 4) 1,739 -> 1,795 us.
-constexpr std::uint32_t kTailBlockTrees = 1024;
+// quarter of the passes. The line is what the chip (152 SMs) holds of the kind's
+// blocks at its registers (58 to 66, reverse 80 to 92; FP64 100 to 104 and 140);
+// beyond it some blocks wait for the others' whole chains. Warps -> blocks:
+// marginals of 304 (456, 608) trees of 999 nodes, K = 4, FP64 -10 (-6, +4) %, of
+// 456 (760, 1,000) of 127 nodes, K = 2, FP32 +4 (0, +7) %, of 608 (760) of 999 -7
+// (0) %; of 4,096 trees, K = 4, 1,739 -> 1,795 us.
+template <typename Compute, int kKind>
+inline constexpr std::uint32_t kTailBlockTrees =
+    152 * (kKind == kPhaseTailForward ? (sizeof(Compute) == 4 ? 7 : 4)
+                                      : (sizeof(Compute) == 4 ? 5 : 3));
 
 // Starts moving `count` 16-byte records from `p` into L2 (a hint).
 __device__ __forceinline__ void PrefetchRecords(const void *p, std::uint32_t count) {
