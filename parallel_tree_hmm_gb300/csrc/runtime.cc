@@ -878,9 +878,10 @@ struct Workspace {
     return false;
   }
 
-  // Whether `operation` runs kernels with work counters or an error word.
-  bool UsesControl(int operation) const {
-    return !UsePhases(operation) || states > 32 || operation == THMM_OP_SAMPLE;
+  // Whether `operation` over `items` items runs kernels with work counters or an
+  // error word.
+  bool UsesControl(int operation, std::size_t items) const {
+    return !UsePhases(operation, items) || states > 32 || operation == THMM_OP_SAMPLE;
   }
   static bool IsLogDomain(int operation) {
     return operation == THMM_OP_MAXIMUM || operation == THMM_OP_SAMPLE;
@@ -889,9 +890,23 @@ struct Workspace {
   bool LinearPhases() const {
     return phase.enabled && phase.exponents_fit;
   }
-  bool UsePhases(int operation) const {
+  bool UsePhases(int operation, std::size_t items) const {
     return schedule == THMM_SCHEDULE_PHASES &&
-           (IsLogDomain(operation) ? phase.enabled : LinearPhases());
+           (IsLogDomain(operation) ? phase.enabled : LinearPhases()) &&
+           !OneLaunch(operation, items);
+  }
+  // Log Z alone of a small tree's items, 5 to 8 states in the batch API: its few
+  // rounds cost more as launches than in one launch of the per-tree engine, whose
+  // warps take an item each. Per-tree engine -> rounds, single precision, us a call:
+  // K = 6, 128 items, 31 nodes 65 -> 78, 61 nodes 81 -> 75; 31 nodes, 1,024 items 70
+  // -> 85, at K = 5 4,096 items 16 % less by rounds; K = 12, 31 nodes, 128 items 18 %
+  // less. A star's one round is a chain either way (K = 5, 399 leaves, 128 items 326
+  // -> 378). Marginals, with more work a launch, gain or lose little (K = 5, one item
+  // of 9 nodes 76 -> 82, of 31 99 -> 104, of 127 23 % less).
+  bool OneLaunch(int operation, std::size_t items) const {
+    return phase_batch && states > 4 && states <= 8 && !IsLogDomain(operation) &&
+           operation != THMM_OP_MARGINALS && items <= 2048 &&
+           (nodes_per_item <= 48 || phase.rounds == 1);
   }
 
   // Tails of MAP and sampling (one CTA per tree runs the last rounds, the root and
@@ -1210,11 +1225,11 @@ struct Workspace {
       args.big_count = items_big ? static_cast<std::uint32_t>(batch) : 0u;
       args.small_count = items_big ? 0u : static_cast<std::uint32_t>(batch);
     }
-    if (UsesControl(operation))
+    if (UsesControl(operation, batch))
       Check(ClearOn(to, control.ptr, 8), "cudaMemsetAsync");
     const auto items = static_cast<std::uint32_t>(forest ? capacity : batch);
     launches = static_cast<std::uint64_t>(
-        UsePhases(operation)
+        UsePhases(operation, batch)
             ? LaunchPhases(operation, 0, items, to)
             : LaunchTeams(operation, args, control.as<std::uint32_t>(), to));
   }
@@ -1465,7 +1480,7 @@ struct Workspace {
               "cudaMemcpyAsync result download");
     };
     download(h_values, values, items * S);
-    if (UsesControl(operation))
+    if (UsesControl(operation, batch))
       download(h_control, control, 16);
     if (operation == THMM_OP_MARGINALS) {
       download(h_node_out, node_out, NodesFor(batch) * states * S);
@@ -1485,7 +1500,7 @@ struct Workspace {
     outcome.timings.upload_ms = upload_ms;
     outcome.timings.kernel_ms = kernel_ms;
     outcome.timings.download_ms = download_ms;
-    outcome.error = UsesControl(operation) ? h_control.as<std::uint32_t>()[2] : 0u;
+    outcome.error = UsesControl(operation, batch) ? h_control.as<std::uint32_t>()[2] : 0u;
     if (outcome.error & kErrorTensorTimeout)
       throw std::runtime_error("tree-HMM accelerator tensor-core wait timed out");
     outcome.timings.wall_ms =
@@ -1610,7 +1625,7 @@ struct Workspace {
       args.small_items = stripe_order.as<std::uint32_t>() + stripe.first + stripe.big;
       args.small_count = stripe.small;
       count += static_cast<std::uint64_t>(
-          UsePhases(operation)
+          UsePhases(operation, batch)
               ? LaunchPhases(operation, stripe.first, stripe.last, stream)
               : LaunchTeams(operation, args, control.as<std::uint32_t>() + 8 + 8 * c, stream));
       Check(cudaEventRecord(computed[c], stream), "cudaEventRecord");
