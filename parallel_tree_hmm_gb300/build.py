@@ -58,6 +58,9 @@ SOURCES = [
     "engine_wide_phase.cu",
     "engine_wide_stream.cu",
     "engine_phase_groups_32_f64.cu",
+    "engine_phase_groups_28_f64.cu",
+    "engine_phase_groups_24_f64.cu",
+    "engine_phase_groups_20_f64.cu",
     "engine_phase_groups_32_f32.cu",
     "engine_phase_groups_28_f32.cu",
     "engine_phase_groups_24_f32.cu",

@@ -105,15 +105,20 @@ cudaError_t LaunchPhase(int scalar_bytes, bool compute_f64, int kind, const Phas
       return compute_f64
                  ? LaunchGroupPhase16F64(scalar_bytes, kind, args, stream, blocks_per_sm)
                  : LaunchGroupPhase16F32(scalar_bytes, kind, args, stream, blocks_per_sm);
-    if (compute_f64)
-      return LaunchGroupPhase32F64(scalar_bytes, kind, args, stream, blocks_per_sm);
     if (args.states <= 20)
-      return LaunchGroupPhase20F32(scalar_bytes, kind, args, stream, blocks_per_sm);
+      return compute_f64
+                 ? LaunchGroupPhase20F64(scalar_bytes, kind, args, stream, blocks_per_sm)
+                 : LaunchGroupPhase20F32(scalar_bytes, kind, args, stream, blocks_per_sm);
     if (args.states <= 24)
-      return LaunchGroupPhase24F32(scalar_bytes, kind, args, stream, blocks_per_sm);
+      return compute_f64
+                 ? LaunchGroupPhase24F64(scalar_bytes, kind, args, stream, blocks_per_sm)
+                 : LaunchGroupPhase24F32(scalar_bytes, kind, args, stream, blocks_per_sm);
     if (args.states <= 28)
-      return LaunchGroupPhase28F32(scalar_bytes, kind, args, stream, blocks_per_sm);
-    return LaunchGroupPhase32F32(scalar_bytes, kind, args, stream, blocks_per_sm);
+      return compute_f64
+                 ? LaunchGroupPhase28F64(scalar_bytes, kind, args, stream, blocks_per_sm)
+                 : LaunchGroupPhase28F32(scalar_bytes, kind, args, stream, blocks_per_sm);
+    return compute_f64 ? LaunchGroupPhase32F64(scalar_bytes, kind, args, stream, blocks_per_sm)
+                       : LaunchGroupPhase32F32(scalar_bytes, kind, args, stream, blocks_per_sm);
   }
   if (scalar_bytes == 8)
     return compute_f64 ? LaunchTyped<double, double>(kind, args, stream, blocks_per_sm)

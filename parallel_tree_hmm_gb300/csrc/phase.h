@@ -278,8 +278,11 @@ THMM_GROUP_PHASE_LAUNCHER(LaunchGroupPhase16F64)
 THMM_GROUP_PHASE_LAUNCHER(LaunchGroupPhase32F32)
 THMM_GROUP_PHASE_LAUNCHER(LaunchGroupPhase32F64)
 THMM_GROUP_PHASE_LAUNCHER(LaunchGroupPhase20F32)
+THMM_GROUP_PHASE_LAUNCHER(LaunchGroupPhase20F64)
 THMM_GROUP_PHASE_LAUNCHER(LaunchGroupPhase24F32)
+THMM_GROUP_PHASE_LAUNCHER(LaunchGroupPhase24F64)
 THMM_GROUP_PHASE_LAUNCHER(LaunchGroupPhase28F32)
+THMM_GROUP_PHASE_LAUNCHER(LaunchGroupPhase28F64)
 #undef THMM_GROUP_PHASE_LAUNCHER
 
 // MAP and sampling (K <= 32, phase_log.cuh): the forward kinds, kPhaseFinish
