@@ -102,15 +102,16 @@ __device__ __forceinline__ void Store4(D *p, const T (&in)[4]) {
   }
 }
 
-// Asynchronous global -> shared copies of 4, 8 or 16 bytes, through L1: in the
-// batch layout every group of an SM reads the same few matrices, and past L1 (.cg)
-// all SMs queue for the same lines of L2. The one gather launch of 8,192 items of 3
-// nodes at K = 8: 51.6 -> 5.5 us.
-template <int kBytes> __device__ __forceinline__ void CopyAsync(void *dst, const void *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
-                   static_cast<unsigned>(__cvta_generic_to_shared(dst))),
-               "l"(src), "n"(kBytes)
-               : "memory");
+// Asynchronous global -> shared copies of 4, 8 or 16 bytes; of 16 past L1 unless
+// the source is shared.
+template <int kBytes, bool kShared = false>
+__device__ __forceinline__ void CopyAsync(void *dst, const void *src) {
+  const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+  if constexpr (kBytes == 16 && !kShared)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(at), "l"(src), "n"(kBytes)
+                 : "memory");
 }
 __device__ __forceinline__ void CopyCommit() {
   asm volatile("cp.async.commit_group;" ::: "memory");
@@ -119,8 +120,13 @@ template <int kPending> __device__ __forceinline__ void CopyWait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
 }
 
-// kExact: K == KMAX, so that the compiler folds the bounds and the strides.
-template <typename Scalar, typename Compute, int KMAX, bool kExact> struct GroupPhaseOps {
+// Variants. In single precision K == KMAX has one for each layout, so that the
+// compiler folds the bounds and the strides, and the general one has K < KMAX; in
+// double the general one is the only one.
+enum GroupForm : int { kGeneralForm = 0, kForestForm = 1, kBatchForm = 2 };
+
+template <typename Scalar, typename Compute, int KMAX, int kForm> struct GroupPhaseOps {
+  static constexpr bool kExact = kForm != kGeneralForm;
   using Tile = GroupTile<KMAX>;
   static constexpr int G = Tile::G, CQ = Tile::CQ, TR = Tile::TR, RG = Tile::RG, P = Tile::P;
   const PhaseArgs &a;
@@ -141,6 +147,10 @@ template <typename Scalar, typename Compute, int KMAX, bool kExact> struct Group
         mask(G == 32 ? kFull : ((1u << (G & 31)) - 1u) << (threadIdx.x % 32 / G * G)),
         ti(lane / CQ), tj(lane % CQ), smem(group_smem) {}
 
+  // K == KMAX: rows of whole 16-byte quads.
+  __device__ __forceinline__ bool Whole() const {
+    return kExact || (sizeof(Compute) == 8 && K == KMAX);
+  }
   __device__ __forceinline__ std::size_t Store(std::uint32_t object) const {
     return object * stride + item;
   }
@@ -207,39 +217,46 @@ template <typename Scalar, typename Compute, int KMAX, bool kExact> struct Group
   // Zero padding of a matrix buffer whose K is below KMAX (the copies write
   // rows and columns below K only).
   __device__ __forceinline__ void ClearPadding(Compute *m) const {
-    if (K != KMAX)
+    if (!Whole())
       for (unsigned i = lane; i < Tile::kMatrix; i += G)
         m[i] = Compute(0);
   }
   // Starts copying a K x K matrix into `m` (pitch P); complete after
   // CopyCommit, CopyWait and a group barrier.
-  template <typename T> __device__ __forceinline__ void StageFrom(const T *src, Compute *m) const {
-    if (K == KMAX) { // rows of whole 16-byte quads
-      constexpr int kQuads = KMAX * CQ;
+  template <bool kShared, typename T>
+  __device__ __forceinline__ void StageWhole(const T *src, Compute *m) const {
+    constexpr int kQuads = KMAX * CQ;
 #pragma unroll
-      for (int first = 0; first < kQuads; first += G) {
-        const unsigned q = first + lane;
-        if (kQuads % G == 0 || q < kQuads) {
-          Compute *dst = m + (q / CQ) * P + 4 * (q % CQ);
-          if constexpr (sizeof(T) == sizeof(Compute)) {
+    for (int first = 0; first < kQuads; first += G) {
+      const unsigned q = first + lane;
+      if (kQuads % G == 0 || q < kQuads) {
+        Compute *dst = m + (q / CQ) * P + 4 * (q % CQ);
+        if constexpr (sizeof(T) == sizeof(Compute)) {
 #pragma unroll
-            for (unsigned part = 0; part < sizeof(T) / 4; ++part)
-              CopyAsync<16>(dst + part * 2, src + 4 * q + part * 2);
-          } else {
-            T in[4];
-            Load4(src + 4 * q, in);
-            const Compute out[4] = {static_cast<Compute>(in[0]), static_cast<Compute>(in[1]),
-                                    static_cast<Compute>(in[2]), static_cast<Compute>(in[3])};
-            Store4(dst, out);
-          }
+          for (unsigned part = 0; part < sizeof(T) / 4; ++part)
+            CopyAsync<16, kShared>(dst + part * 2, src + 4 * q + part * 2);
+        } else {
+          T in[4];
+          Load4(src + 4 * q, in);
+          const Compute out[4] = {static_cast<Compute>(in[0]), static_cast<Compute>(in[1]),
+                                  static_cast<Compute>(in[2]), static_cast<Compute>(in[3])};
+          Store4(dst, out);
         }
       }
-    } else {
-      // Four elements at a time, each place found by itself: a gather's rakes are
-      // a chain, and a division and dependent places were a fifth of its link (128
-      // items of a star of 399 leaves, K = 5, 425 -> 378 us a call).
-#pragma unroll 4
-      for (unsigned i = lane; i < KK; i += G) {
+    }
+  }
+  // The same for K < KMAX, element by element. Each place is found by itself and
+  // eight are under way at a time: a gather's rakes are a chain, and a division,
+  // dependent places and (for inputs of another width) one load after the other were
+  // a quarter of its link (log Z of a star of 998 leaves, K = 7, 922 -> 700 us a call,
+  // with double inputs 1,772 -> 1,335).
+  template <typename T>
+  __device__ __forceinline__ void StagePadded(const T *src, Compute *m) const {
+    constexpr int kSteps = (KMAX * KMAX + G - 1) / G;
+#pragma unroll 8
+    for (int step = 0; step < kSteps; ++step) {
+      const unsigned i = lane + step * G;
+      if (i < KK) {
         Compute *dst = m + i + (i * inverse >> 16) * (P - K); // row r at r * P
         if constexpr (sizeof(T) == sizeof(Compute))
           CopyAsync<sizeof(T)>(dst, src + i);
@@ -248,17 +265,33 @@ template <typename Scalar, typename Compute, int KMAX, bool kExact> struct Group
       }
     }
   }
-  __device__ __forceinline__ void Stage(std::uint32_t ref, Compute *m) const {
-    if (ref & kFlag)
-      StageFrom(static_cast<const Compute *>(CompAt(ref & kMask)), m);
+  template <bool kShared, typename T>
+  __device__ __forceinline__ void StageFrom(const T *src, Compute *m) const {
+    if (Whole())
+      StageWhole<kShared>(src, m);
     else
-      StageFrom(EdgeAt(ref), m);
+      StagePadded(src, m);
+  }
+  // An edge of the batch layout comes through L1: every group of an SM reads the
+  // same few, and past L1 all SMs queue for the same lines of L2 (the one gather
+  // launch of 8,192 items of 3 nodes at K = 8 51.6 -> 5.3 us). A forest's edges are
+  // read once, and L1 only delays them (256 trees of 5,000 nodes, K = 20, 2,123 ->
+  // 2,159 us).
+  __device__ __forceinline__ void Stage(std::uint32_t ref, Compute *m) const {
+    // Edges of another width are converted, through registers.
+    constexpr bool kSame = sizeof(Scalar) == sizeof(Compute);
+    if (ref & kFlag)
+      StageFrom<false>(static_cast<const Compute *>(CompAt(ref & kMask)), m);
+    else if (kSame && (kForm == kBatchForm || (kForm == kGeneralForm && Whole() && a.batch != 0)))
+      StageFrom<true>(EdgeAt(ref), m);
+    else
+      StageFrom<false>(EdgeAt(ref), m);
   }
   // Writes the K x K matrix in `m` out, transformed element by element
   // (value, row, column).
   template <bool kStreaming, typename T, class Map>
   __device__ __forceinline__ void Drain(const Compute *m, T *dst, Map map) const {
-    if (K == KMAX) {
+    if (Whole()) {
       constexpr int kQuads = KMAX * CQ;
 #pragma unroll
       for (int first = 0; first < kQuads; first += G) {
@@ -474,7 +507,7 @@ template <typename Scalar, typename Compute, int KMAX, bool kExact> struct Group
 #pragma unroll
           for (int c = 0; c < 4; ++c)
             out[q][c] = ScalePow2(out[q][c], -s);
-          if (K == KMAX) {
+          if (Whole()) {
             Store4(dst + r * KMAX + 4 * tj, out[q]);
           } else {
 #pragma unroll
@@ -587,7 +620,7 @@ template <typename Scalar, typename Compute, int KMAX, bool kExact> struct Group
 #pragma unroll
     for (int q = 0; q < TR; ++q) {
       const unsigned r = ti + q * RG;
-      if (K == KMAX && ti < RG && (RG * TR == KMAX || r < K)) {
+      if (Whole() && ti < RG && (RG * TR == KMAX || r < K)) {
         Load4(output_adjoint + r * KMAX + 4 * tj, adjoint[q]);
       } else {
 #pragma unroll
@@ -749,11 +782,11 @@ template <int KMAX, bool kWide> constexpr int GroupPhaseMinBlocks(int kind) {
 
 // One kind of one round: lane group g of the grid runs operation offset + g /
 // items of item first_item + g % items (finish: the root record).
-template <typename Scalar, typename Compute, int KMAX, int kKind, bool kExact>
+template <typename Scalar, typename Compute, int KMAX, int kKind, int kForm>
 __global__ void __launch_bounds__(kGroupPhaseThreads,
                                   GroupPhaseMinBlocks<KMAX, sizeof(Compute) == 8>(kKind))
     GroupPhaseKernel(PhaseArgs args) {
-  using Ops = GroupPhaseOps<Scalar, Compute, KMAX, kExact>;
+  using Ops = GroupPhaseOps<Scalar, Compute, KMAX, kForm>;
   constexpr int G = Ops::G;
   constexpr int kElements = kGroupPhaseElements<KMAX, kKind>;
   extern __shared__ __align__(16) unsigned char group_smem[];

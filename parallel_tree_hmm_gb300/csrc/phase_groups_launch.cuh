@@ -24,10 +24,11 @@ cudaError_t LaunchKind(const PhaseArgs &args, LaunchStream stream, int *blocks_p
   // slots in the large rounds), which folded bounds shorten: a marginal step
   // of 256 trees of 5,000 nodes at K = 20 2,202 -> 2,141 us, 500 items on a
   // 399-node tree 386 -> 377 us. Double is bound by its pipe and keeps one variant.
-  auto kernel = GroupPhaseKernel<Scalar, Compute, KMAX, kKind, false>;
+  auto kernel = GroupPhaseKernel<Scalar, Compute, KMAX, kKind, kGeneralForm>;
   if constexpr (sizeof(Compute) == 4) {
     if (args.states == KMAX)
-      kernel = GroupPhaseKernel<Scalar, Compute, KMAX, kKind, true>;
+      kernel = args.batch ? GroupPhaseKernel<Scalar, Compute, KMAX, kKind, kBatchForm>
+                          : GroupPhaseKernel<Scalar, Compute, KMAX, kKind, kForestForm>;
   }
   constexpr unsigned lanes = GroupLanes<KMAX>();
   constexpr unsigned smem = kGroupPhaseThreads / lanes * kGroupPhaseElements<KMAX, kKind> *

@@ -129,7 +129,7 @@ template <typename Scalar, int KMAX, bool kExact> struct ItemPhaseOps {
         const unsigned q = at + lane;
         if (kQuads % 32 == 0 || q < kQuads) {
           if constexpr (sizeof(Scalar) == 4) {
-            CopyAsync<16>(dst + 4 * q, src + 4 * q);
+            CopyAsync<16, true>(dst + 4 * q, src + 4 * q);
           } else {
             Scalar in[4];
             Load4(src + 4 * q, in);
