@@ -384,7 +384,8 @@ thmm_status thmm_device_inputs_ready(thmm_workspace *workspace, size_t batch);
  * THMM_SCHEDULE_PHASES runs each round of every tree in one grid-wide launch
  * per operation kind (the default where available: forests at every state
  * count and the batch API up to 32 states; the batch API above 32 states
- * always uses THMM_SCHEDULE_TEAMS). Under THMM_SCHEDULE_PHASES the first
+ * always uses THMM_SCHEDULE_TEAMS, and so does log Z alone of few small items at
+ * 5 to 8 states). Under THMM_SCHEDULE_PHASES the first
  * `phase_rounds` rounds run as grid-wide launches and the remaining rounds of
  * each tree in one warp or block per tree, for the sum-product calls of a
  * forest up to 4 states (0: chosen from the operation counts; at least the

@@ -29,9 +29,9 @@
 // per-tree engines took the right factor's K^2 logarithms once per lane.
 // K <= 4 has one thread per operation and K^2 <= 16 logarithms of its own.
 // Measured on one GB300, per-tree engines -> these kernels: MAP of 320
-// Galton-Watson trees (8.2 M nodes, K = 8) 7.57 -> 1.58 ms, sampling of the
-// same trees 11.4 -> 2.9 ms, a host-to-host MAP call on 48 uneven trees
-// (76 k nodes, K = 8) 2.35 -> 0.32 ms.
+// Galton-Watson trees (8.2 M nodes, K = 8) 7.57 -> 1.21 ms, sampling of the
+// same trees 11.4 -> 1.94 ms, a host-to-host MAP call on 48 uneven trees
+// (76 k nodes, K = 8) 2.35 -> 0.26 ms.
 #ifndef THMM_PHASE_LOG_CUH_
 #define THMM_PHASE_LOG_CUH_
 

@@ -39,7 +39,6 @@
 #define THMM_MULF(a, b) __fmul_rn((a), (b))
 #define THMM_ADDF(a, b) __fadd_rn((a), (b))
 #define THMM_SUBF(a, b) __fsub_rn((a), (b))
-#define THMM_DIVF(a, b) __fdiv_rn((a), (b))
 #define THMM_FMA(a, b, c) __fma_rn((a), (b), (c))
 #define THMM_MUL(a, b) __dmul_rn((a), (b))
 #define THMM_ADD(a, b) __dadd_rn((a), (b))
@@ -50,7 +49,6 @@
 #define THMM_MULF(a, b) ((a) * (b))
 #define THMM_ADDF(a, b) ((a) + (b))
 #define THMM_SUBF(a, b) ((a) - (b))
-#define THMM_DIVF(a, b) ((a) / (b))
 #define THMM_FMA(a, b, c) fma((a), (b), (c))
 #define THMM_MUL(a, b) ((a) * (b))
 #define THMM_ADD(a, b) ((a) + (b))
